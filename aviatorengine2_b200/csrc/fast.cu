@@ -30,7 +30,6 @@
 // correctly rounded binary32, so t and the barycentrics are bit-identical to
 // the plain kernel's; the watertight variant (Woop, Benthin and Wald, "Watertight
 // Ray/Triangle Intersection", JCGT 2013) is selected with `quant`.
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,6 +46,7 @@
 #include "fast_trace.cuh"
 #include "fast_walk.cuh"
 #include "kernels.h"
+#include "quantise.cuh"
 #include "trace_common.cuh"
 
 namespace ae {
@@ -91,7 +91,7 @@ void quantise(float o, int e, float a, float b, uint8_t &qa, uint8_t &qb, bool &
 
 struct Collapser {
     const ae_bvh_node *bin;  // this mesh's binary nodes
-    std::vector<QNode> &out;
+    std::vector<WideNode> &out;
     bool ok = true;
     int max_stack = 0;
 
@@ -115,8 +115,8 @@ struct Collapser {
             kids.insert(kids.begin() + best, uint32_t(bin[open].left));
         }
         const uint32_t self = uint32_t(out.size());
-        out.push_back(QNode{});
-        QNode q;
+        out.push_back(WideNode{});
+        WideNode q;
         std::memset(&q, 0, sizeof(q));
         Box nb = node_box(bin[i]);
         // Conservative frame: the union of the children.
@@ -166,8 +166,8 @@ struct Collapser {
 
 // Worst-case stack entries of the kernel's loop over this tree: on each
 // node the far hit children are pushed (up to nchild - 1).
-int stack_need(const std::vector<QNode> &nodes, uint32_t root) {
-    const QNode &q = nodes[root];
+int stack_need(const std::vector<WideNode> &nodes, uint32_t root) {
+    const WideNode &q = nodes[root];
     int best = 0;
     for (int k = 0; k < q.nchild; k++) {
         if (q.child[k] & kLeafBit) continue;
@@ -324,7 +324,7 @@ struct ObjectTree {
 // mesh).  Checks, before anything reaches a device: every link stays inside
 // the tree, every leaf inside the mesh's triangles, every quantised box
 // contains its exact box, and the traversal stack bound.
-bool build_qbvh(const ae_bvh_node *bin, uint32_t n_bin, uint32_t tri_count, std::vector<QNode> &out, uint32_t &root,
+bool build_qbvh(const ae_bvh_node *bin, uint32_t n_bin, uint32_t tri_count, std::vector<WideNode> &out, uint32_t &root,
                 int &stack, std::string &err) {
     out.clear();
     stack = 0;
@@ -361,7 +361,7 @@ bool build_qbvh(const ae_bvh_node *bin, uint32_t n_bin, uint32_t tri_count, std:
     if (!col.ok) { err = "a child box cannot be quantised conservatively"; return false; }
     // Final structural check of what the kernel will follow.
     for (size_t i = 0; i < out.size(); i++) {
-        const QNode &q = out[i];
+        const WideNode &q = out[i];
         if (q.nchild < 2 || q.nchild > 4) { err = "node child count"; return false; }
         for (int k = 0; k < q.nchild; k++) {
             const uint32_t r = q.child[k];
@@ -430,35 +430,6 @@ __global__ void k_object_boxes(const uint4 *__restrict__ meta, const FastInst *_
     }
 }
 
-// Smallest power-of-two scale whose 255 steps from `org` reach `top`
-// (the host collapser's frame rule); false when none fits the exponent range.
-__device__ bool frame_exponent(float org, float top, int &e) {
-    const float extent = top - org;
-    e = -126;
-    if (extent > 0.0f) {
-        e = int(ceil(log2(double(extent) / 255.0)));
-        while (ldexp(255.0, e) < double(extent)) e++;
-        e = max(e, -126);
-    }
-    while (e <= 127 && fmaf(255.0f, ldexpf(1.0f, e), org) < top) e++;
-    return e <= 127;
-}
-
-// Child interval [a, b] quantised outward in the frame (org, 2^e): the
-// decoded bounds org + q 2^e (fmaf) contain it.
-__device__ bool quantise_outward(float org, int e, float a, float b, uint8_t &qa, uint8_t &qb) {
-    const float sc = ldexpf(1.0f, e);
-    double la = floor((double(a) - double(org)) / double(sc)), lb = ceil((double(b) - double(org)) / double(sc));
-    la = fmin(fmax(la, 0.0), 255.0);
-    lb = fmin(fmax(lb, 0.0), 255.0);
-    int ia = int(la), ib = int(lb);
-    while (ia > 0 && fmaf(float(ia), sc, org) > a) ia--;
-    while (ib < 255 && fmaf(float(ib), sc, org) < b) ib++;
-    qa = uint8_t(ia);
-    qb = uint8_t(ib);
-    return fmaf(float(ia), sc, org) <= a && fmaf(float(ib), sc, org) >= b;
-}
-
 // One level of the instance tree's bottom-up refresh (levels deepest first):
 // a node's float box is the union of its children's (objects' boxes for leaf
 // children), and its children are re-quantised in the node's new frame.  A
@@ -471,45 +442,20 @@ __global__ void k_instance_tree_level(QNode *__restrict__ nodes, float *__restri
     if (k >= count) return;
     const int32_t ni = level[k];
     QNode q = nodes[ni];
-    float cb[4][6];
+    const int n = int(q.scale >> 24);
+    float cb[4][6], u[6];
     bool cv[4];
-    float u[6] = {3.402823466e38f, 3.402823466e38f, 3.402823466e38f, -3.402823466e38f, -3.402823466e38f,
-                  -3.402823466e38f};
-    bool any = false;
     for (int c = 0; c < 4; c++) {
         cv[c] = false;
-        if (c >= q.nchild) continue;
+        if (c >= n) continue;
         const uint32_t ref = q.child[c];
         const float *x = (ref & kLeafBit) ? obj_box + 6 * size_t(leaf_first(ref)) : nbox + 6 * size_t(ref);
         bool ok = true;
         for (int a = 0; a < 6; a++) { cb[c][a] = x[a]; ok = ok && isfinite(x[a]); }
         for (int a = 0; a < 3; a++) ok = ok && cb[c][a] <= cb[c][3 + a];
         cv[c] = ok;
-        if (!ok) continue;
-        any = true;
-        for (int a = 0; a < 3; a++) { u[a] = fminf(u[a], cb[c][a]); u[3 + a] = fmaxf(u[3 + a], cb[c][3 + a]); }
     }
-    bool good = true;
-    int ex[3] = {0, 0, 0};
-    if (any) {
-        q.ox = u[0]; q.oy = u[1]; q.oz = u[2];
-        for (int a = 0; a < 3; a++) good = frame_exponent(u[a], u[3 + a], ex[a]) && good;
-    } else {
-        q.ox = q.oy = q.oz = 0.0f;
-        u[0] = u[1] = u[2] = __int_as_float(0x7f800000);
-        u[3] = u[4] = u[5] = -__int_as_float(0x7f800000);
-    }
-    q.ex = int8_t(good ? ex[0] : 0); q.ey = int8_t(good ? ex[1] : 0); q.ez = int8_t(good ? ex[2] : 0);
-    const float org[3] = {q.ox, q.oy, q.oz};
-    for (int c = 0; c < 4; c++) {
-        if (cv[c] && any && good) {
-            for (int a = 0; a < 3; a++)
-                good = quantise_outward(org[a], ex[a], cb[c][a], cb[c][3 + a], q.lo[a][c], q.hi[a][c]) && good;
-        } else {
-            for (int a = 0; a < 3; a++) { q.lo[a][c] = 255; q.hi[a][c] = 0; }
-        }
-    }
-    if (!good) atomicExch(bad, 1u);
+    if (!quantise_node(q, n, cb, cv, u)) atomicExch(bad, 1u);
     nodes[ni] = q;
     float *o = nbox + 6 * size_t(ni);
     for (int a = 0; a < 6; a++) o[a] = u[a];
@@ -548,7 +494,7 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
     for (uint32_t s = 0; s < n; s++) T.idx[s] = s;
     T.nodes.reserve(2 * size_t(n));
     T.build(0, n, 0);
-    std::vector<QNode> out;
+    std::vector<WideNode> out;
     uint32_t root;
     if (T.nodes[0].count > 0) {
         root = leaf_ref(uint32_t(T.nodes[0].left), 1);
@@ -579,8 +525,17 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
         F.obj_box.reserve(size_t(n) * 6) || F.static_box.reserve(size_t(n) * 6) || F.tflag.reserve(1))
         return c->fail(AE_ERR_OOM, "instance tree");
     int rc;
+    // Links and child counts; the refresh writes frames and planes.
+    std::vector<QNode> dev(out.size(), QNode{});
+    for (size_t i = 0; i < out.size(); i++) {
+        dev[i].scale = uint32_t(out[i].nchild) << 24;
+        for (int k = 0; k < 4; k++) {
+            dev[i].plane[k] = make_uint2(0u, kPlaneUnused);
+            dev[i].child[k] = out[i].child[k];
+        }
+    }
     if (!out.empty() &&
-        ((rc = c->cuda(cudaMemcpyAsync(F.tnodes.ptr, out.data(), out.size() * sizeof(QNode), cudaMemcpyHostToDevice,
+        ((rc = c->cuda(cudaMemcpyAsync(F.tnodes.ptr, dev.data(), dev.size() * sizeof(QNode), cudaMemcpyHostToDevice,
                                        c->stream), "upload instance tree")) ||
          (rc = c->cuda(cudaMemcpyAsync(F.tlevels.ptr, order.data(), order.size() * sizeof(int32_t),
                                        cudaMemcpyHostToDevice, c->stream), "upload instance tree levels"))))
@@ -639,8 +594,7 @@ int prepare_fast(Ctx *c) {
         // New geometry arrays: every mesh is converted again (the device
         // buffers are reused).
         F.mesh_roots.clear();
-        F.host_nodes.clear();
-        F.host_tris.clear();
+        F.n_tris = 0;
         F.mesh_sub.clear();
         F.host_sub.clear();
         F.max_stack = 0;
@@ -654,34 +608,11 @@ int prepare_fast(Ctx *c) {
         const ae_instance &m = c->host_instances[i];
         const auto key = std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase);
         if (F.mesh_roots.count(key)) continue;
-        // Triangle records of this mesh in slot order.
-        const uint32_t tri_base = uint32_t(F.host_tris.size() / 12);
-        F.host_tris.resize(F.host_tris.size() + size_t(m.triangleCount) * 12);
-        float *dst = F.host_tris.data() + size_t(tri_base) * 12;
-        for (uint32_t t = 0; t < m.triangleCount; t++) {
-            for (int v = 0; v < 3; v++) {
-                const ae_vertex &vx = c->host_vertices[m.vertexBase + c->host_indices[m.indexBase + 3 * t + v]];
-                dst[12 * t + 3 * v + 0] = vx.px;
-                dst[12 * t + 3 * v + 1] = vx.py;
-                dst[12 * t + 3 * v + 2] = vx.pz;
-            }
-            dst[12 * t + 9] = dst[12 * t + 10] = dst[12 * t + 11] = 0.0f;
-        }
-        uint32_t root;
-        std::vector<QNode> local;
-        int need = 0;
-        std::string err;
-        if (!build_qbvh(c->host_blas.data() + m.blasBase, uint32_t(c->n_blas - m.blasBase), m.triangleCount, local,
-                        root, need, err))
-            return c->fail(AE_ERR_LAYOUT, "4-wide BVH of instance %u: %s", i, err.c_str());
-        const uint32_t before = uint32_t(F.host_nodes.size());
-        for (QNode &q : local)
-            for (int k = 0; k < q.nchild; k++)
-                if (!(q.child[k] & kLeafBit)) q.child[k] += before;
-        if (!(root & kLeafBit)) root += before;
-        F.host_nodes.insert(F.host_nodes.end(), local.begin(), local.end());
-        F.max_stack = std::max(F.max_stack, need);
-        F.mesh_roots[key] = std::make_pair(root, tri_base);
+        // The root reference is filled in by the build; triangle records are
+        // numbered in the order in which the meshes are met.
+        if (m.triangleCount > 0xffffffffu - F.n_tris) return c->fail(AE_ERR_LAYOUT, "more than 2^32 triangles");
+        F.mesh_roots[key] = std::make_pair(0u, F.n_tris);
+        F.n_tris += m.triangleCount;
         FastScene::MeshSub ms;
         ms.first = uint32_t(F.host_sub.size() / 6);
         ms.count = mesh_sub_boxes(c->host_blas.data() + m.blasBase, F.host_sub);
@@ -690,21 +621,10 @@ int prepare_fast(Ctx *c) {
         F.mesh_sub[key] = ms;
         F.geometry_dirty = true;
     }
-    if (F.max_stack + 1 > kFastStack)
-        return c->fail(AE_ERR_LAYOUT, "4-wide BVH needs %d stack entries (> %d)", F.max_stack + 1, kFastStack);
     int rc;
     if (F.geometry_dirty) {
         rebuilt = true;
-        F.n_nodes = uint32_t(F.host_nodes.size());
-        F.n_tris = uint32_t(F.host_tris.size() / 12);
-        if (F.nodes.reserve(std::max<size_t>(F.n_nodes, 1)) || F.tris.reserve(std::max<size_t>(size_t(F.n_tris) * 3, 1)))
-            return c->fail(AE_ERR_OOM, "fast scene buffers");
-        if (F.n_nodes && (rc = c->cuda(cudaMemcpyAsync(F.nodes.ptr, F.host_nodes.data(), F.n_nodes * sizeof(QNode),
-                                                       cudaMemcpyHostToDevice, c->stream), "upload nodes")))
-            return rc;
-        if ((rc = c->cuda(cudaMemcpyAsync(F.tris.ptr, F.host_tris.data(), F.host_tris.size() * sizeof(float),
-                                          cudaMemcpyHostToDevice, c->stream), "upload triangles")))
-            return rc;
+        if ((rc = build_mesh_structures(c, F))) return rc;
         if (F.sub_boxes.reserve(std::max<size_t>(F.host_sub.size(), 1))) return c->fail(AE_ERR_OOM, "mesh sub-boxes");
         if (!F.host_sub.empty() &&
             (rc = c->cuda(cudaMemcpyAsync(F.sub_boxes.ptr, F.host_sub.data(), F.host_sub.size() * sizeof(float),
@@ -766,45 +686,6 @@ int prepare_fast(Ctx *c) {
     if (F.has_volumes)
         return c->fail(AE_ERR_STATE, "participating media consume RNG in the reference's visit order; use the plain kernel");
     c->fast_ready = true;
-    return AE_OK;
-}
-
-// The precision form's shading records: per triangle, in the optimised
-// BVH's slot order, the three vertex normals and UVs rounded to FP16
-// (round to nearest even), 32 bytes (layout in wf_common.cuh).
-int prepare_precision(Ctx *c) {
-    int rc = prepare_fast(c);
-    if (rc) return rc;
-    FastScene &F = *c->fast;
-    if (F.shade16_tris == F.n_tris && F.shade16.ptr) return AE_OK;
-    std::vector<uint16_t> h(size_t(std::max(F.n_tris, 1u)) * 16, 0);
-    auto half_bits = [](float x) {
-        const __half v = __float2half_rn(x);
-        uint16_t b;
-        std::memcpy(&b, &v, 2);
-        return b;
-    };
-    for (const auto &kv : F.mesh_roots) {
-        const uint32_t vbase = std::get<0>(kv.first), ibase = std::get<1>(kv.first), tris = std::get<2>(kv.first);
-        const uint32_t tri_base = kv.second.second;
-        for (uint32_t t = 0; t < tris; t++) {
-            uint16_t *r = h.data() + (size_t(tri_base) + t) * 16;
-            for (int v = 0; v < 3; v++) {
-                const ae_vertex &vx = c->host_vertices[vbase + c->host_indices[ibase + 3 * t + v]];
-                r[3 * v + 0] = half_bits(vx.nx);
-                r[3 * v + 1] = half_bits(vx.ny);
-                r[3 * v + 2] = half_bits(vx.nz);
-                r[9 + 2 * v] = half_bits(vx.u);
-                r[10 + 2 * v] = half_bits(vx.v);
-            }
-        }
-    }
-    if (F.shade16.reserve(size_t(std::max(F.n_tris, 1u)) * 2)) return c->fail(AE_ERR_OOM, "FP16 shading records");
-    if ((rc = c->cuda(cudaMemcpyAsync(F.shade16.ptr, h.data(), h.size() * 2, cudaMemcpyHostToDevice, c->stream),
-                      "upload FP16 shading records")))
-        return rc;
-    if ((rc = c->cuda(cudaStreamSynchronize(c->stream), "FP16 shading records"))) return rc;
-    F.shade16_tris = F.n_tris;
     return AE_OK;
 }
 
@@ -1039,7 +920,7 @@ cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
 extern "C" int ae_build_wide_bvh(const ae_bvh_node *blas, uint32_t n_nodes, uint32_t tri_count, void *out_nodes,
                                  uint32_t capacity, uint32_t *out_count, uint32_t *out_root, int32_t *out_stack) {
     if (!blas || !out_count || !out_root || !out_stack) return AE_ERR_INVALID;
-    std::vector<ae::QNode> nodes;
+    std::vector<ae::WideNode> nodes;
     uint32_t root = 0;
     int stack = 0;
     std::string err;
@@ -1051,6 +932,6 @@ extern "C" int ae_build_wide_bvh(const ae_bvh_node *blas, uint32_t n_nodes, uint
     *out_root = root;
     *out_stack = stack;
     if (nodes.size() > capacity || (!out_nodes && !nodes.empty())) return AE_ERR_OVERSIZE;
-    if (!nodes.empty()) std::memcpy(out_nodes, nodes.data(), nodes.size() * sizeof(ae::QNode));
+    if (!nodes.empty()) std::memcpy(out_nodes, nodes.data(), nodes.size() * sizeof(ae::WideNode));
     return AE_OK;
 }

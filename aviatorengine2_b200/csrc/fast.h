@@ -5,6 +5,8 @@
 
 namespace ae {
 int prepare_fast(Ctx *c);
+// Nodes and triangle records of the listed meshes on the device (fast_build.cu).
+int build_mesh_structures(Ctx *c, FastScene &F);
 int prepare_precision(Ctx *c);
 void destroy_fast(Ctx *c);
 cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, bool quant, cudaStream_t st);

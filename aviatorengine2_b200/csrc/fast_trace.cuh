@@ -16,7 +16,26 @@
 
 namespace ae {
 
-struct QNode {               // 64 B
+// A 4-wide node of the walks, 64 bytes.  `scale` holds, per axis, the biased
+// binary32 exponent of 2^14 times the node's quantum 2^e (bytes 0-2), and the
+// number of children in use (byte 3).  A child's eight bytes are its
+// quantised planes {lo x, lo y, lo z, hi x, hi y, hi z} and the two bytes
+// kPlaneB6, kPlaneB7: one byte permute of the pair with a selector that the
+// ray's direction sign picks gives the bits 0x4000qq00, the float
+// 2 + q 2^-14, so a plane costs one permute and one fma, with no conversion
+// and no subtraction of a bias.  An unused slot carries 0x7fff there, which
+// makes every plane a NaN and the interval test false.
+struct QNode {
+    float ox, oy, oz;        // frame origin, below the node box minimum
+    uint32_t scale;
+    uint2 plane[4];
+    uint32_t child[4];       // interior: node index; leaf: leaf_ref(first, count)
+};
+static_assert(sizeof(QNode) == 64, "QNode must be 64 bytes");
+constexpr uint32_t kPlaneTail = 0x40000000u, kPlaneUnused = 0x7fff0000u;  // bytes 6-7 of a child's planes
+
+// The node layout that ae_build_wide_bvh hands out (include/ae_b200.h).
+struct WideNode {            // 64 B
     float ox, oy, oz;        // node box minimum
     int8_t ex, ey, ez;       // child box scale 2^e per axis
     uint8_t nchild;          // children in use (2..4)
@@ -25,7 +44,7 @@ struct QNode {               // 64 B
     uint32_t child[4];       // interior: node index; leaf: leaf_ref(first, count)
     uint32_t pad[2];
 };
-static_assert(sizeof(QNode) == 64, "QNode must be 64 bytes");
+static_assert(sizeof(WideNode) == 64, "WideNode must be 64 bytes");
 constexpr uint32_t kLeafBit = 0x80000000u;
 // A leaf reference: bit 31 set, primitive count in bits 24-30 (1..127), first
 // slot in bits 0-23.  prepare_fast refuses meshes outside those limits.
@@ -73,13 +92,11 @@ struct FastScene {
     int max_stack = 0;
     uint64_t geometry_key = ~0ull, scene_key = ~0ull;
     bool has_volumes = false;
-    // host_nodes / host_tris grew and are not on the device yet (an upload
-    // that failed is retried by the next prepare_fast)
+    // a mesh is listed (mesh_roots) whose structures are not on the device yet
+    // (a build that failed is retried by the next prepare_fast)
     bool geometry_dirty = false;
     // per distinct mesh (vertexBase, indexBase, triangleCount, blasBase)
     std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>, std::pair<uint32_t, uint32_t>> mesh_roots;
-    std::vector<QNode> host_nodes;
-    std::vector<float> host_tris;
     // Instance-level tree.  Per mesh: its local sub-boxes (host_sub, six
     // floats each) at sub_boxes[first .. first + count) and the largest
     // coordinate magnitude they reach.
@@ -179,60 +196,62 @@ AE_DEV bool tri_test_wt(f3 o, const WtRay &W, float tn, float tf, const float4 &
     return tri_wt(o, W, tn, tf, mk(r0.x, r0.y, r0.z), mk(r0.w, r1.x, r1.y), mk(r1.z, r1.w, r2.x), t, a, b);
 }
 
-// Relative widening of slab intervals in the optimised walk (entry scaled
-// down, exit scaled up; t >= tnear > 0 on the entry side).
-constexpr float kEntryShrink = 0.99999904632568359375f;  // 1 - 2^-20
-constexpr float kExitGrow = 1.00000095367431640625f;     // 1 + 2^-20
+// Relative widening of slab intervals in the optimised walks: an interval's
+// exit and the best distance are scaled up by 1 + 2^-19 before they are
+// compared with an entry.  That covers the relative rounding of the plane
+// distances (the absolute part, under 2^-8 of a quantum, is kept free by the
+// quantiser), so neither a nearer hit nor one on a box's face is pruned.
+constexpr float kExitGrow = 1.0000019073486328125f;  // 1 + 2^-19
 
-// Byte k (0..3) of w as an exact float: the byte permute builds the bits
-// 0x4B0000bb, which are 2^23 + bb, and the subtraction is exact.  Same value
-// as float(bb), without a conversion on the XU pipe.
-AE_DEV float byte_as_float(uint32_t w, int k) {
-    const uint32_t bits = __byte_perm(w, 0x4B000000u, 0x7440u | uint32_t(k));
-    return __fsub_rn(__uint_as_float(bits), 8388608.0f);
+AE_DEV float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+AE_DEV float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
-// Entry distance of the 4 quantised child boxes; an inverted slot or a miss
-// yields +inf.  Computed as q * (s/d) + (o - p)/d per slab with a relative
-// widening of 2^-20 on the exit side, which covers the rounding of this
-// formulation (the decoded boxes already contain the exact ones).
+// Entry distances of a node's four child boxes; +inf for a child that the ray
+// misses or that starts beyond the best hit.  Distances are in units of the
+// ray parameter; plane q of an axis lies at (o - p)/d + q s/d, evaluated as
+// (2 + q 2^-14) ix + bx with ix = 2^14 s/d and bx = (o - p)/d - 2 ix.
 //
-// The near and far planes of each slab are picked once per node from the sign
-// of the direction term: the rounded fma is monotone in q, so for a valid
-// child (lo <= hi) the pick gives exactly min and max of the two plane
-// distances, and the intervals are bit for bit those of the min/max form.
+// The walks are bound by issue slots with 11-13 of 32 lanes active, so the
+// count of instructions here is what a step costs: the permute builds a
+// plane's float directly, the near and far bytes are chosen by the permute's
+// selector instead of by selects, three-operand min and max fold an interval,
+// and an unused slot rejects itself.
 AE_DEV void child_hits(const QNode *nodep, f3 o, f3 inv, float tn, float tf, float tmin[4], uint32_t child[4]) {
-    const float4 *p = reinterpret_cast<const float4 *>(nodep);
-    const float4 w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2), w3 = __ldg(p + 3);
-    const uint32_t meta = __float_as_uint(w0.w);
-    const int ex = int(int8_t(meta & 0xff)), ey = int(int8_t((meta >> 8) & 0xff)), ez = int(int8_t((meta >> 16) & 0xff));
-    const float sx = __int_as_float((ex + 127) << 23), sy = __int_as_float((ey + 127) << 23),
-                sz = __int_as_float((ez + 127) << 23);
-    const float ix = sx * inv.x, iy = sy * inv.y, iz = sz * inv.z;
-    const float bx = (w0.x - o.x) * inv.x, by = (w0.y - o.y) * inv.y, bz = (w0.z - o.z) * inv.z;
-    const uint32_t lox = __float_as_uint(w1.x), loy = __float_as_uint(w1.y), loz = __float_as_uint(w1.z);
-    const uint32_t hix = __float_as_uint(w1.w), hiy = __float_as_uint(w2.x), hiz = __float_as_uint(w2.y);
-    // Near-plane and far-plane bytes per axis.
-    const uint32_t nx = ix >= 0.0f ? lox : hix, fx = ix >= 0.0f ? hix : lox;
-    const uint32_t ny = iy >= 0.0f ? loy : hiy, fy = iy >= 0.0f ? hiy : loy;
-    const uint32_t nz = iz >= 0.0f ? loz : hiz, fz = iz >= 0.0f ? hiz : loz;
-    // A slot is in use when its x range is not inverted (one byte-wise compare).
-    const uint32_t valid = __vcmpleu4(lox, hix);
-    child[0] = __float_as_uint(w2.z); child[1] = __float_as_uint(w2.w);
-    child[2] = __float_as_uint(w3.x); child[3] = __float_as_uint(w3.y);
+    const uint4 *p = reinterpret_cast<const uint4 *>(nodep);
+    const uint4 w0 = __ldg(p), pa = __ldg(p + 1), pb = __ldg(p + 2), cr = __ldg(p + 3);
+    const float ix = __uint_as_float(__byte_perm(w0.w, 0u, 0x0444u) >> 1) * inv.x;
+    const float iy = __uint_as_float(__byte_perm(w0.w, 0u, 0x1444u) >> 1) * inv.y;
+    const float iz = __uint_as_float(__byte_perm(w0.w, 0u, 0x2444u) >> 1) * inv.z;
+    const float bx = fmaf(-2.0f, ix, (__uint_as_float(w0.x) - o.x) * inv.x);
+    const float by = fmaf(-2.0f, iy, (__uint_as_float(w0.y) - o.y) * inv.y);
+    const float bz = fmaf(-2.0f, iz, (__uint_as_float(w0.z) - o.z) * inv.z);
+    // Selectors {6, q, 6, 7}: q = 0, 1, 2 for the low planes and 3, 4, 5 for
+    // the high ones; a negative direction enters through the high plane.
+    const uint32_t nx = 0x7606u ^ (uint32_t(__float_as_int(inv.x) >> 31) & 0x30u), fx = nx ^ 0x30u;
+    const uint32_t ny = 0x7616u ^ (uint32_t(__float_as_int(inv.y) >> 31) & 0x50u), fy = ny ^ 0x50u;
+    const uint32_t nz = 0x7626u ^ (uint32_t(__float_as_int(inv.z) >> 31) & 0x70u), fz = nz ^ 0x70u;
+    const float tfg = tf * kExitGrow;
+    const uint32_t lo_w[4] = {pa.x, pa.z, pb.x, pb.z}, hi_w[4] = {pa.y, pa.w, pb.y, pb.w};
+    child[0] = cr.x; child[1] = cr.y; child[2] = cr.z; child[3] = cr.w;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const float t0x = fmaf(byte_as_float(nx, k), ix, bx), t1x = fmaf(byte_as_float(fx, k), ix, bx);
-        const float t0y = fmaf(byte_as_float(ny, k), iy, by), t1y = fmaf(byte_as_float(fy, k), iy, by);
-        const float t0z = fmaf(byte_as_float(nz, k), iz, bz), t1z = fmaf(byte_as_float(fz, k), iz, bz);
-        const float lo = fmaxf(fmaxf(t0x, t0y), fmaxf(t0z, tn));
-        const float hi = fminf(fminf(t1x, t1y), t1z);
-        // Widened by 2^-20 relative on both sides: the interval computed here
-        // then contains the exact one, so neither a closer hit nor one lying
-        // on the box's face is pruned by rounding.
-        const float lo_c = lo * kEntryShrink;
-        const bool hit = ((valid >> (8 * k)) & 1u) && lo_c <= fminf(hi * kExitGrow, tf);
-        tmin[k] = hit ? lo_c : __int_as_float(0x7f800000);
+        const float t0x = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], nx)), ix, bx);
+        const float t0y = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], ny)), iy, by);
+        const float t0z = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], nz)), iz, bz);
+        const float t1x = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fx)), ix, bx);
+        const float t1y = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fy)), iy, by);
+        const float t1z = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fz)), iz, bz);
+        const float lo = fmaxf(max3(t0x, t0y, t0z), tn);
+        const float hi = min3(t1x, t1y, t1z) * kExitGrow;
+        tmin[k] = lo <= hi && lo <= tfg ? lo : __int_as_float(0x7f800000);
     }
 }
 
@@ -282,7 +301,7 @@ AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, uint
         while (sp > 0) {
             sp--;
             const uint2 e = sp < SS ? stk[sp * nthreads + tid] : spill[sp - SS];
-            if (__uint_as_float(e.y) <= best.t) {
+            if (__uint_as_float(e.y) <= best.t * kExitGrow) {
                 cur = e.x;
                 return true;
             }
@@ -354,7 +373,7 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
     auto pop = [&]() {
         while (sp > 0) {
             sp--;
-            if (tdist[sp] <= best.t) {
+            if (tdist[sp] <= best.t * kExitGrow) {
                 cur = tstack[sp];
                 return true;
             }

@@ -75,7 +75,7 @@ struct Walker {
     AE_DEV void tlas_pop(const WalkStacks<SS> &K) {
         while (tsp > 0) {
             tsp--;
-            if (K.tdist[tsp] <= best.t) {
+            if (K.tdist[tsp] <= best.t * kExitGrow) {
                 tcur = K.tstack[tsp];
                 phase = (tcur & kLeafBit) ? kWalkObject : kWalkTlas;
                 return;
@@ -90,7 +90,7 @@ struct Walker {
         while (bsp > 0) {
             bsp--;
             const uint2 e = bsp < SS ? stk[bsp * nt + tid] : K.spill[bsp - SS];
-            if (__uint_as_float(e.y) <= best.t) {
+            if (__uint_as_float(e.y) <= best.t * kExitGrow) {
                 cur = e.x;
                 return;
             }
