@@ -120,13 +120,14 @@ struct FastScene {
     uint64_t tlas_key = ~0ull, sub_key = ~0ull;
 };
 
-// Traversal stack per thread: the first kSharedStack entries in shared
-// memory, the rest (rarely reached: only along the deepest paths of the
-// largest meshes) in a per-thread local array.  prepare_fast checks that no
-// tree needs more than kFastStack entries.
-constexpr int kSharedStack = 24;
-constexpr int kLocalStack = 40;
-constexpr int kFastStack = kSharedStack + kLocalStack;
+// Traversal stack per thread, one for both trees (a mesh's entries lie above
+// the instance tree's): the first kSharedStack entries in shared memory, the
+// rest (rarely reached: only along the deepest paths of the largest meshes) in
+// a per-thread local array.  prepare_fast checks that no mesh tree needs more
+// than kFastStack entries and no instance tree more than kTlas4Stack.
+constexpr int kSharedStack = 12;
+constexpr int kFastStack = 64;
+constexpr int kWalkStack = kFastStack + kTlas4Stack;
 
 // ---------------------------------------------------------------------------
 // Device
@@ -259,9 +260,9 @@ AE_DEV void child_hits(const QNode *nodep, f3 o, f3 inv, float tn, float tf, flo
 // value of the same sign, so products stay finite (no 0 * inf).
 AE_DEV float slab_inv(float x) { return fabsf(x) > 1e-20f ? 1.0f / x : copysignf(1e20f, x); }
 
-// Sorts child_hits' four (distance, child) pairs nearest first and returns
-// how many were hit (misses carry +inf and sort last).
-AE_DEV int sort_hits(float tm[4], uint32_t ch[4]) {
+// Sorts child_hits' four (distance, child) pairs nearest first (misses carry
+// +inf and sort last); false when none was hit.
+AE_DEV bool sort_hits(float tm[4], uint32_t ch[4]) {
 #define AE_SWAP(i, j)                                            \
     if (tm[j] < tm[i]) {                                         \
         const float tt = tm[i]; tm[i] = tm[j]; tm[j] = tt;       \
@@ -269,17 +270,47 @@ AE_DEV int sort_hits(float tm[4], uint32_t ch[4]) {
     }
     AE_SWAP(0, 1) AE_SWAP(2, 3) AE_SWAP(0, 2) AE_SWAP(1, 3) AE_SWAP(1, 2)
 #undef AE_SWAP
-    int nh = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) nh += tm[k] != __int_as_float(0x7f800000) ? 1 : 0;
-    return nh;
+    return tm[0] != __int_as_float(0x7f800000);
+}
+
+// One thread's traversal stack: its column of the block's shared-memory part
+// and the entries beyond it.
+template <int SS>
+struct WalkStack {
+    uint2 spill[kWalkStack - SS];
+};
+// The bound check of the spilled part keeps every access inside the array for
+// any input (prepare_fast has checked the trees' needs).
+template <int SS>
+AE_DEV void stack_push(WalkStack<SS> &K, uint2 *stk, int &sp, int tid, int nt, uint32_t ref, float t) {
+    const uint2 e = make_uint2(ref, __float_as_uint(t));
+    if (sp < SS) stk[sp * nt + tid] = e;
+    else if (sp < kWalkStack) K.spill[sp - SS] = e;
+    else return;
+    sp++;
+}
+template <int SS>
+AE_DEV uint2 stack_at(const WalkStack<SS> &K, const uint2 *stk, int i, int tid, int nt) {
+    return i < SS ? stk[i * nt + tid] : K.spill[i - SS];
+}
+// A node's hit children but the nearest, farthest first.  Written out, so
+// that the sorted distances and references stay in registers (a loop over
+// them put both arrays in local memory: eight stores a node, the largest
+// single cost of the walks).
+template <int SS>
+AE_DEV void push_far(WalkStack<SS> &K, uint2 *stk, int &sp, int tid, int nt, const float tm[4], const uint32_t ch[4]) {
+    const float none = __int_as_float(0x7f800000);
+    if (tm[3] != none) stack_push(K, stk, sp, tid, nt, ch[3], tm[3]);
+    if (tm[2] != none) stack_push(K, stk, sp, tid, nt, ch[2], tm[2]);
+    if (tm[1] != none) stack_push(K, stk, sp, tid, nt, ch[1], tm[1]);
 }
 
 // T (optional): touch counters - wide nodes in `blas`, 48-byte triangle
-// records in `tris`.
+// records in `tris`.  The stack's first `base` entries belong to the caller.
 template <bool WT, int SS = kSharedStack>
 AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, uint64_t orank, f3 o, f3 d, float tn,
-                       Best &best, uint2 *stk, int tid, int nthreads, Touch *T = nullptr) {
+                       Best &best, WalkStack<SS> &K, uint2 *stk, const int base, int tid, int nthreads,
+                       Touch *T = nullptr) {
     // ToLocal (hybrid:534-543) exactly as the reference, so the local ray and
     // every triangle's t are bit-identical to the plain kernel's.
     f3 lo = quat_rotate(-I.qx, -I.qy, -I.qz, I.qw, o - mk(I.px, I.py, I.pz));
@@ -293,14 +324,13 @@ AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, uint
     WtRay W;
     if (WT) W = wt_setup(ld);
     const float4 *tris = V.tris + size_t(I.tri_base) * 3;
-    uint2 spill[kFastStack - SS];
-    int sp = 0;
+    int sp = base;
     uint32_t cur = I.root;
     // Next stack entry still no farther than the best hit; false when none.
     auto pop = [&]() {
-        while (sp > 0) {
+        while (sp > base) {
             sp--;
-            const uint2 e = sp < SS ? stk[sp * nthreads + tid] : spill[sp - SS];
+            const uint2 e = stack_at(K, stk, sp, tid, nthreads);
             if (__uint_as_float(e.y) <= best.t * kExitGrow) {
                 cur = e.x;
                 return true;
@@ -316,17 +346,8 @@ AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, uint
             uint32_t ch[4];
             if (T) T->blas++;
             child_hits(V.nodes + cur, lo, inv, tn, best.t, tm, ch);
-            const int nh = sort_hits(tm, ch);
-            if (nh > 0) {
-                // Far hits onto the stack (farthest deepest), continue with the
-                // nearest.  prepare_fast checked that the tree never needs more
-                // than kFastStack entries; the bound check keeps that true for
-                // any input.
-                for (int k = nh - 1; k >= 1; k--) {
-                    if (sp < SS) stk[sp * nthreads + tid] = make_uint2(ch[k], __float_as_uint(tm[k]));
-                    else if (sp < kFastStack) spill[sp - SS] = make_uint2(ch[k], __float_as_uint(tm[k]));
-                    sp = sp < kFastStack ? sp + 1 : sp;
-                }
+            if (sort_hits(tm, ch)) {
+                push_far(K, stk, sp, tid, nthreads, tm, ch);
                 cur = ch[0];
             } else if (!pop()) {
                 return;
@@ -365,16 +386,16 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
     best.object = AE_MISS; best.prim = AE_MISS; best.orank = 0; best.lrank = 0;
     if (V.troot == kEmptyTlas) return best;
     const f3 inv = mk(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
-    uint32_t tstack[kTlas4Stack];
-    float tdist[kTlas4Stack];
+    WalkStack<SS> K;
     int sp = 0;
     uint32_t cur = V.troot;
     // Next stack entry no farther than the best hit; false when none is left.
     auto pop = [&]() {
         while (sp > 0) {
             sp--;
-            if (tdist[sp] <= best.t * kExitGrow) {
-                cur = tstack[sp];
+            const uint2 e = stack_at(K, stk, sp, tid, nt);
+            if (__uint_as_float(e.y) <= best.t * kExitGrow) {
+                cur = e.x;
                 return true;
             }
         }
@@ -390,16 +411,8 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
             uint32_t ch[4];
             if (T) T->tlas++;
             child_hits(V.tnodes + cur, o, inv, tn, best.t, tm, ch);
-            const int nh = sort_hits(tm, ch);
-            if (nh > 0) {
-                // prepare_fast checked the tree against kTlas4Stack.
-                for (int k = nh - 1; k >= 1; k--) {
-                    if (sp < kTlas4Stack) {
-                        tstack[sp] = ch[k];
-                        tdist[sp] = tm[k];
-                        sp++;
-                    }
-                }
+            if (sort_hits(tm, ch)) {
+                push_far(K, stk, sp, tid, nt, tm, ch);
                 cur = ch[0];
             } else if (!pop()) {
                 live = false;
@@ -420,7 +433,7 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
             I.px = a.x; I.py = a.y; I.pz = a.z; I.scale = a.w;
             I.qx = b.x; I.qy = b.y; I.qz = b.z; I.qw = b.w;
             I.root = __float_as_uint(c.x); I.tri_base = __float_as_uint(c.y);
-            trace_mesh<WT, SS>(V, I, slot, orank, o, d, tn, best, stk, tid, nt, T);
+            trace_mesh<WT, SS>(V, I, slot, orank, o, d, tn, best, K, stk, sp, tid, nt, T);
         } else {
             DHit h;
             const ae_object *obj = S.objects + slot;

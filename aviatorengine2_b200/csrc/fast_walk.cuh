@@ -28,15 +28,10 @@ enum : uint32_t { kWalkTlas = 0, kWalkObject = 1, kWalkBlas = 2, kWalkDone = 3 }
 // wavefront frame 177 ms against 192 ms and 179 ms.
 constexpr int kWalkBlocksPerSm = 7;
 
-// The walk's per-thread local stacks: the instance-tree stack and the BLAS
-// entries beyond the shared-memory part.  Kept out of Walker so its scalar
-// state can live in registers.
+// The walk's stack beyond its shared-memory part.  Kept out of Walker so its
+// scalar state can live in registers.
 template <int SS = kSharedStack>
-struct WalkStacks {
-    uint32_t tstack[kTlas4Stack];
-    float tdist[kTlas4Stack];
-    uint2 spill[kFastStack - SS];
-};
+using WalkStacks = WalkStack<SS>;
 
 template <bool WT, int SS = kSharedStack>
 struct Walker {
@@ -45,15 +40,16 @@ struct Walker {
     float tn, time;
     Best best;
     uint32_t phase;
-    // instance tree: the current node, or the leaf (object) being entered
-    uint32_t tcur;
-    int tsp;
+    // the node or leaf to step next, of the tree that `phase` names
+    uint32_t cur;
+    // stack entries, and how many of them belong to the instance tree while a
+    // mesh is walked
+    int sp, base;
     // current mesh instance
     f3 lo, ld, linv;
     WtRay W;
-    uint32_t tri_base, cur, slot;
+    uint32_t tri_base, slot;
     uint64_t orank;
-    int bsp;
 
     // tmax below kFarStart starts the walk as if a hit at tmax were already
     // found: every hit nearer than tmax is still found, with the same tie
@@ -65,37 +61,27 @@ struct Walker {
         time = time_;
         best.t = tmax; best.alpha = 0.0f; best.beta = 0.0f;
         best.object = AE_MISS; best.prim = AE_MISS; best.orank = 0; best.lrank = 0;
-        tsp = 0;
+        sp = 0;
+        base = 0;
         tinv = mk(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
-        tcur = V.troot;
-        phase = (tcur & kLeafBit) ? (leaf_count(tcur) ? kWalkObject : kWalkDone) : kWalkTlas;
+        cur = V.troot;
+        phase = (cur & kLeafBit) ? (leaf_count(cur) ? kWalkObject : kWalkDone) : kWalkTlas;
     }
 
-    // Next instance-tree stack entry no farther than the best hit, or done.
-    AE_DEV void tlas_pop(const WalkStacks<SS> &K) {
-        while (tsp > 0) {
-            tsp--;
-            if (K.tdist[tsp] <= best.t * kExitGrow) {
-                tcur = K.tstack[tsp];
-                phase = (tcur & kLeafBit) ? kWalkObject : kWalkTlas;
+    // Next stack entry no farther than the best hit, or done; an entry below
+    // `base` leads back from the mesh to the instance tree.
+    AE_DEV void pop(const WalkStack<SS> &K, const uint2 *stk, int tid, int nt) {
+        const float far = best.t * kExitGrow;
+        while (sp > 0) {
+            sp--;
+            const uint2 e = stack_at(K, stk, sp, tid, nt);
+            if (__uint_as_float(e.y) <= far) {
+                cur = e.x;
+                if (phase != kWalkBlas || sp < base) phase = (cur & kLeafBit) ? kWalkObject : kWalkTlas;
                 return;
             }
         }
         phase = kWalkDone;
-    }
-
-    // Next BLAS stack entry no farther than the best hit, or back to the
-    // instance tree.
-    AE_DEV void blas_pop(const WalkStacks<SS> &K, const uint2 *stk, int tid, int nt) {
-        while (bsp > 0) {
-            bsp--;
-            const uint2 e = bsp < SS ? stk[bsp * nt + tid] : K.spill[bsp - SS];
-            if (__uint_as_float(e.y) <= best.t * kExitGrow) {
-                cur = e.x;
-                return;
-            }
-        }
-        tlas_pop(K);
     }
 
     // The walk's phase group for warp-level step scheduling: 0 interior node
@@ -106,7 +92,7 @@ struct Walker {
     }
 
     // One step; returns true once the ray is finished (best is final).
-    AE_DEV bool step(const DevScene &S, const FastView &V, WalkStacks<SS> &K, uint2 *stk, int tid, int nt) {
+    AE_DEV bool step(const DevScene &S, const FastView &V, WalkStack<SS> &K, uint2 *stk, int tid, int nt) {
         if (phase == kWalkBlas && (cur & kLeafBit)) {
             const uint32_t first = leaf_first(cur), cnt = leaf_count(cur);
             const float4 *tris = V.tris + size_t(tri_base) * 3;
@@ -123,11 +109,11 @@ struct Walker {
                     best.orank = orank; best.lrank = ~first;
                 }
             }
-            blas_pop(K, stk, tid, nt);
+            pop(K, stk, tid, nt);
             return phase == kWalkDone;
         }
         if (phase == kWalkObject) {
-            slot = leaf_first(tcur);
+            slot = leaf_first(cur);
             const uint4 m = __ldg(V.meta + slot);
             orank = object_rank(m, slot);
             const uint32_t shape = m.x & 0xff;
@@ -146,7 +132,7 @@ struct Walker {
                 if (WT) W = wt_setup(ld);
                 tri_base = __float_as_uint(c.y);
                 cur = __float_as_uint(c.x);
-                bsp = 0;
+                base = sp;
                 phase = kWalkBlas;
                 return false;
             }
@@ -161,7 +147,7 @@ struct Walker {
                 best.t = h.t; best.alpha = h.alpha; best.beta = h.beta;
                 best.object = slot; best.prim = AE_MISS; best.orank = orank; best.lrank = 0;
             }
-            tlas_pop(K);
+            pop(K, stk, tid, nt);
             return phase == kWalkDone;
         }
         if (phase == kWalkDone) return true;
@@ -171,31 +157,14 @@ struct Walker {
         const bool top = phase == kWalkTlas;
         float tm[4];
         uint32_t ch[4];
-        child_hits(top ? V.tnodes + tcur : V.nodes + cur, top ? o : lo, top ? tinv : linv, tn, best.t, tm, ch);
-        const int nh = sort_hits(tm, ch);
-        if (nh > 0) {
-            if (top) {
-                for (int k = nh - 1; k >= 1; k--) {
-                    if (tsp < kTlas4Stack) {
-                        K.tstack[tsp] = ch[k];
-                        K.tdist[tsp] = tm[k];
-                        tsp++;
-                    }
-                }
-                tcur = ch[0];
-                phase = (tcur & kLeafBit) ? kWalkObject : kWalkTlas;
-            } else {
-                for (int k = nh - 1; k >= 1; k--) {
-                    if (bsp < SS) stk[bsp * nt + tid] = make_uint2(ch[k], __float_as_uint(tm[k]));
-                    else if (bsp < kFastStack) K.spill[bsp - SS] = make_uint2(ch[k], __float_as_uint(tm[k]));
-                    bsp = bsp < kFastStack ? bsp + 1 : bsp;
-                }
-                cur = ch[0];
-            }
+        child_hits((top ? V.tnodes : V.nodes) + cur, top ? o : lo, top ? tinv : linv, tn, best.t, tm, ch);
+        if (sort_hits(tm, ch)) {
+            push_far(K, stk, sp, tid, nt, tm, ch);
+            cur = ch[0];
+            if (top && (cur & kLeafBit)) phase = kWalkObject;
             return false;
         }
-        if (top) tlas_pop(K);
-        else blas_pop(K, stk, tid, nt);
+        pop(K, stk, tid, nt);
         return phase == kWalkDone;
     }
 };
