@@ -390,7 +390,8 @@ bool build_qbvh(const ae_bvh_node *bin, uint32_t n_bin, uint32_t tri_count, std:
 // kernels' ToLocal and triangle arithmetic for rays that start within the
 // scene's coordinate range (the margin is 2^-14 of it).
 __global__ void k_object_boxes(const uint4 *__restrict__ meta, const FastInst *__restrict__ inst,
-                               const float *__restrict__ sub, const float *__restrict__ static_box, uint32_t n,
+                               const float *__restrict__ sub, const uint2 *__restrict__ sub_refs,
+                               const float *__restrict__ static_box, uint32_t n,
                                float margin, float *__restrict__ out) {
     const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (slot >= n) return;  // whole warps
@@ -400,7 +401,8 @@ __global__ void k_object_boxes(const uint4 *__restrict__ meta, const FastInst *_
         const FastInst I = inst[m.y];
         const double s = (I.scale != 0.0f && I.scale != 1.0f) ? double(I.scale) : 1.0;
         const double qx = I.qx, qy = I.qy, qz = I.qz, qw = I.qw;
-        const uint32_t first = I.pad[0], cnt = I.pad[1];
+        const uint2 sr = sub_refs[I.sub];
+        const uint32_t first = sr.x, cnt = sr.y;
         for (uint32_t j = lane; j < cnt * 8u; j += 32) {
             const float *x = sub + 6 * size_t(first + j / 8);
             const uint32_t k = j & 7u;
@@ -571,7 +573,7 @@ static int refresh_instance_tree(Ctx *c, FastScene &F) {
     const uint32_t n = c->n_objects;
     int rc;
     if ((rc = c->cuda(cudaMemsetAsync(F.tflag.ptr, 0, sizeof(uint32_t), c->stream), "instance tree flag"))) return rc;
-    k_object_boxes<<<(n * 32 + 255) / 256, 256, 0, c->stream>>>(F.obj_meta.ptr, F.inst.ptr, F.sub_boxes.ptr,
+    k_object_boxes<<<(n * 32 + 255) / 256, 256, 0, c->stream>>>(F.obj_meta.ptr, F.inst.ptr, F.sub_boxes.ptr, F.sub_refs.ptr,
                                                                  F.static_box.ptr, n, margin, F.obj_box.ptr);
     for (size_t l = 0; l + 1 < F.tlevel_start.size(); l++) {
         const int32_t cnt = F.tlevel_start[l + 1] - F.tlevel_start[l];
@@ -614,6 +616,7 @@ int prepare_fast(Ctx *c) {
         F.mesh_roots[key] = std::make_pair(0u, F.n_tris);
         F.n_tris += m.triangleCount;
         FastScene::MeshSub ms;
+        ms.index = uint32_t(F.mesh_sub.size());
         ms.first = uint32_t(F.host_sub.size() / 6);
         ms.count = mesh_sub_boxes(c->host_blas.data() + m.blasBase, F.host_sub);
         ms.radius = 0.0f;
@@ -630,6 +633,13 @@ int prepare_fast(Ctx *c) {
             (rc = c->cuda(cudaMemcpyAsync(F.sub_boxes.ptr, F.host_sub.data(), F.host_sub.size() * sizeof(float),
                                           cudaMemcpyHostToDevice, c->stream), "upload mesh sub-boxes")))
             return rc;
+        std::vector<uint2> sub_refs(std::max<size_t>(F.mesh_sub.size(), 1), make_uint2(0u, 0u));
+        for (const auto &kv : F.mesh_sub) sub_refs[kv.second.index] = make_uint2(kv.second.first, kv.second.count);
+        if (F.sub_refs.reserve(sub_refs.size())) return c->fail(AE_ERR_OOM, "mesh sub-boxes");
+        if ((rc = c->cuda(cudaMemcpyAsync(F.sub_refs.ptr, sub_refs.data(), sub_refs.size() * sizeof(uint2),
+                                          cudaMemcpyHostToDevice, c->stream), "upload mesh sub-boxes")) ||
+            (rc = c->cuda(cudaStreamSynchronize(c->stream), "mesh sub-boxes")))
+            return rc;
         F.geometry_dirty = false;
     }
     // Scene-derived part: instances and object metadata, per upload.
@@ -644,8 +654,8 @@ int prepare_fast(Ctx *c) {
             f.root = rt.first;
             f.tri_base = rt.second;
             const FastScene::MeshSub &ms = F.mesh_sub.at(std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase));
-            f.pad[0] = ms.first;
-            f.pad[1] = ms.count;
+            f.inv_scale = m.scale != 0.0f && m.scale != 1.0f ? 1.0f / m.scale : 1.0f;
+            f.sub = ms.index;
         }
         // Each object's rank comes from the reference TLAS leaf that holds it.
         std::vector<uint32_t> leaf_first_of(std::max<uint32_t>(c->n_objects, 1), 0u);

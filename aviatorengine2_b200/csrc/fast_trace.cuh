@@ -59,7 +59,8 @@ struct FastInst {            // 48 B
     float qx, qy, qz, qw;
     uint32_t root;           // QNode index of the mesh root, or a leaf ref
     uint32_t tri_base;       // first triangle record of the mesh
-    uint32_t pad[2];
+    float inv_scale;         // 1 / scale as ToLocal divides, 1 for a rigid instance
+    uint32_t sub;            // the mesh's entry in FastScene::sub_refs
 };
 static_assert(sizeof(FastInst) == 48, "FastInst must be 48 bytes");
 
@@ -101,12 +102,13 @@ struct FastScene {
     // floats each) at sub_boxes[first .. first + count) and the largest
     // coordinate magnitude they reach.
     struct MeshSub {
-        uint32_t first, count;
+        uint32_t first, count, index;
         float radius;
     };
     std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>, MeshSub> mesh_sub;
     std::vector<float> host_sub;
     DevBuf<float> sub_boxes;
+    DevBuf<uint2> sub_refs;       // per mesh: its first sub-box and their number
     DevBuf<QNode> tnodes;         // the tree's nodes (boxes rewritten on every refresh)
     DevBuf<float> tbox;           // float box per tree node (6 floats)
     DevBuf<float> obj_box;        // conservative world box per object (6 floats)
@@ -148,25 +150,27 @@ inline FastView fast_view(const FastScene &F, const FastInst *inst = nullptr, co
                     F.troot};
 }
 
-// Rank of an object's candidates (see Best): ~first slot of the reference
-// TLAS leaf holding the object, then the slot.
-AE_DEV uint64_t object_rank(const uint4 &meta, uint32_t slot) { return (uint64_t(~meta.z) << 32) | slot; }
-
-// Best candidate so far with its visit rank (see the file comment).  A
-// candidate ranks by (object rank, leaf rank, slot): object rank is
-// (~first slot of its TLAS leaf) << 32 | object slot, leaf rank is ~first slot
-// of its BLAS leaf; larger means visited later by the reference's walk.
+// Best candidate so far.  Equal distances rank by (object rank, leaf rank,
+// slot), larger meaning visited later by the reference's walk (see the file
+// comment): an object's rank is ~first slot of the reference TLAS leaf holding
+// it (the metadata's z word), then its slot; the leaf rank is ~first slot of
+// the BLAS leaf.  Object ranks are read when two distances are equal, which is
+// rare, and not carried along.
 struct Best {
     float t, alpha, beta;
     uint32_t object, prim;
-    uint64_t orank;
     uint32_t lrank;
 };
+AE_DEV bool later_object(const FastView &V, uint32_t object, uint32_t than) {
+    if (than == AE_MISS) return true;
+    const uint32_t a = __ldg(&V.meta[object].z), b = __ldg(&V.meta[than].z);
+    return a != b ? a < b : object > than;
+}
 // Given a hit at t <= best.t (the tests reject t > far), keep it if nearer or
 // equally near and later in the reference's visit order.
-AE_DEV bool takes(const Best &b, float t, uint64_t orank, uint32_t lrank, uint32_t slot) {
+AE_DEV bool takes(const FastView &V, const Best &b, float t, uint32_t object, uint32_t lrank, uint32_t slot) {
     if (t < b.t) return true;
-    if (orank != b.orank) return orank > b.orank;
+    if (object != b.object) return later_object(V, object, b.object);
     if (lrank != b.lrank) return lrank > b.lrank;
     return slot > b.prim;
 }
@@ -184,10 +188,23 @@ AE_DEV bool tri_test_ref(f3 o, f3 d, float tn, float tf, const float4 &r0, const
     if (AE_FABS(den) < 1e-12f) return false;
     t = AE_DIV(AE_SUB(dot(n, p0), dot(n, o)), den);
     if (t < tn || t > tf) return false;
-    const f3 w = n / nn;
     const f3 pl = o + d * t - p0;
-    a = dot(w, cross(pl, e2));
-    b = dot(w, cross(e1, pl));
+    const f3 ca = cross(pl, e2), cb = cross(e1, pl);
+    // Most candidates lie outside by far more than rounding: those are turned
+    // away without the reference's three divisions.  a = (n / nn) . ca and
+    // its terms' roundings stay within 2^-21 of sum |n_i ca_i| / nn (and of
+    // the smallest binary32 values, which the last term covers), so a sum
+    // below -2^-20 of that has a < 0; the same for b, and for a + b > 1.
+    const float ma = fmaf(fabsf(n.x), fabsf(ca.x), fmaf(fabsf(n.y), fabsf(ca.y), fabsf(n.z * ca.z)));
+    const float mb = fmaf(fabsf(n.x), fabsf(cb.x), fmaf(fabsf(n.y), fabsf(cb.y), fabsf(n.z * cb.z)));
+    const float sa = fmaf(n.x, ca.x, fmaf(n.y, ca.y, n.z * ca.z)), sb = fmaf(n.x, cb.x, fmaf(n.y, cb.y, n.z * cb.z));
+    constexpr float kRel = 9.5367431640625e-07f;  // 2^-20
+    const float tiny = nn * 1e-30f;
+    if (fmaf(ma, kRel, sa) + tiny < 0.0f || fmaf(mb, kRel, sb) + tiny < 0.0f) return false;
+    if (fmaf(ma + mb, -kRel, sa + sb) > fmaf(nn, kRel, nn) + tiny) return false;
+    const f3 w = n / nn;
+    a = dot(w, ca);
+    b = dot(w, cb);
     return !(a < 0.0f || b < 0.0f || AE_ADD(a, b) > 1.0f);
 }
 
@@ -257,8 +274,15 @@ AE_DEV void child_hits(const QNode *nodep, f3 o, f3 inv, float tn, float tf, flo
 }
 
 // Safe reciprocal for slab tests: a zero component becomes a huge finite
-// value of the same sign, so products stay finite (no 0 * inf).
-AE_DEV float slab_inv(float x) { return fabsf(x) > 1e-20f ? 1.0f / x : copysignf(1e20f, x); }
+// value of the same sign, so products stay finite (no 0 * inf).  The hardware
+// reciprocal (within 1 ulp) scales an axis's plane distances by at most 2^-23,
+// inside the intervals' widening; a correctly rounded quotient cost about ten
+// instructions an axis.
+AE_DEV float slab_inv(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fabsf(x) > 1e-20f ? r : copysignf(1e20f, x);
+}
 
 // Sorts child_hits' four (distance, child) pairs nearest first (misses carry
 // +inf and sort last); false when none was hit.
@@ -308,18 +332,16 @@ AE_DEV void push_far(WalkStack<SS> &K, uint2 *stk, int &sp, int tid, int nt, con
 // T (optional): touch counters - wide nodes in `blas`, 48-byte triangle
 // records in `tris`.  The stack's first `base` entries belong to the caller.
 template <bool WT, int SS = kSharedStack>
-AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, uint64_t orank, f3 o, f3 d, float tn,
+AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, f3 o, f3 d, float tn,
                        Best &best, WalkStack<SS> &K, uint2 *stk, const int base, int tid, int nthreads,
                        Touch *T = nullptr) {
     // ToLocal (hybrid:534-543) exactly as the reference, so the local ray and
     // every triangle's t are bit-identical to the plain kernel's.
     f3 lo = quat_rotate(-I.qx, -I.qy, -I.qz, I.qw, o - mk(I.px, I.py, I.pz));
     f3 ld = quat_rotate(-I.qx, -I.qy, -I.qz, I.qw, d);
-    if (I.scale != 0.0f && I.scale != 1.0f) {
-        const float inv = AE_DIV(1.0f, I.scale);
-        lo = lo * inv;
-        ld = ld * inv;
-    }
+    // Multiplying by exactly 1 changes nothing, so rigid instances need no branch.
+    lo = lo * I.inv_scale;
+    ld = ld * I.inv_scale;
     const f3 inv = mk(slab_inv(ld.x), slab_inv(ld.y), slab_inv(ld.z));
     WtRay W;
     if (WT) W = wt_setup(ld);
@@ -362,10 +384,10 @@ AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, uint
             float t, a, b;
             const bool h = WT ? tri_test_wt(lo, W, tn, best.t, r0, r1, r2, t, a, b)
                               : tri_test_ref(lo, ld, tn, best.t, r0, r1, r2, t, a, b);
-            if (h && takes(best, t, orank, ~first, s)) {
+            if (h && takes(V, best, t, slot, ~first, s)) {
                 best.t = t; best.alpha = a; best.beta = b;
                 best.object = slot; best.prim = s;
-                best.orank = orank; best.lrank = ~first;
+                best.lrank = ~first;
             }
         }
         if (!pop()) return;
@@ -383,7 +405,7 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
                          int nt, Touch *T = nullptr) {
     Best best;
     best.t = kFarStart; best.alpha = 0.0f; best.beta = 0.0f;
-    best.object = AE_MISS; best.prim = AE_MISS; best.orank = 0; best.lrank = 0;
+    best.object = AE_MISS; best.prim = AE_MISS; best.lrank = 0;
     if (V.troot == kEmptyTlas) return best;
     const f3 inv = mk(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
     WalkStack<SS> K;
@@ -422,7 +444,6 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
         if (!live) break;
         const uint32_t slot = leaf_first(cur);
         const uint4 m = __ldg(V.meta + slot);
-        const uint64_t orank = object_rank(m, slot);
         const uint32_t shape = m.x & 0xff;
         if (T) T->objects++;
         if (shape == AE_SHAPE_MESH) {
@@ -433,7 +454,8 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
             I.px = a.x; I.py = a.y; I.pz = a.z; I.scale = a.w;
             I.qx = b.x; I.qy = b.y; I.qz = b.z; I.qw = b.w;
             I.root = __float_as_uint(c.x); I.tri_base = __float_as_uint(c.y);
-            trace_mesh<WT, SS>(V, I, slot, orank, o, d, tn, best, K, stk, sp, tid, nt, T);
+            I.inv_scale = c.z;
+            trace_mesh<WT, SS>(V, I, slot, o, d, tn, best, K, stk, sp, tid, nt, T);
         } else {
             DHit h;
             const ae_object *obj = S.objects + slot;
@@ -442,9 +464,9 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
             else if (shape == AE_SHAPE_QUAD) hit = hit_planar_ref(obj, false, o, d, tn, best.t, h);
             else if (shape == AE_SHAPE_TRIANGLE) hit = hit_planar_ref(obj, true, o, d, tn, best.t, h);
             else hit = hit_box_ref(obj, o, d, tn, best.t, h);
-            if (hit && takes(best, h.t, orank, 0u, 0u)) {
+            if (hit && takes(V, best, h.t, slot, 0u, 0u)) {
                 best.t = h.t; best.alpha = h.alpha; best.beta = h.beta;
-                best.object = slot; best.prim = AE_MISS; best.orank = orank; best.lrank = 0;
+                best.object = slot; best.prim = AE_MISS; best.lrank = 0;
             }
         }
         if (!pop()) break;

@@ -49,7 +49,6 @@ struct Walker {
     f3 lo, ld, linv;
     WtRay W;
     uint32_t tri_base, slot;
-    uint64_t orank;
 
     // tmax below kFarStart starts the walk as if a hit at tmax were already
     // found: every hit nearer than tmax is still found, with the same tie
@@ -60,7 +59,7 @@ struct Walker {
         tn = tn_;
         time = time_;
         best.t = tmax; best.alpha = 0.0f; best.beta = 0.0f;
-        best.object = AE_MISS; best.prim = AE_MISS; best.orank = 0; best.lrank = 0;
+        best.object = AE_MISS; best.prim = AE_MISS; best.lrank = 0;
         sp = 0;
         base = 0;
         tinv = mk(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
@@ -103,10 +102,10 @@ struct Walker {
                 float t, a, b;
                 const bool h = WT ? tri_test_wt(lo, W, tn, best.t, r0, r1, r2, t, a, b)
                                   : tri_test_ref(lo, ld, tn, best.t, r0, r1, r2, t, a, b);
-                if (h && takes(best, t, orank, ~first, s)) {
+                if (h && takes(V, best, t, slot, ~first, s)) {
                     best.t = t; best.alpha = a; best.beta = b;
                     best.object = slot; best.prim = s;
-                    best.orank = orank; best.lrank = ~first;
+                    best.lrank = ~first;
                 }
             }
             pop(K, stk, tid, nt);
@@ -115,7 +114,6 @@ struct Walker {
         if (phase == kWalkObject) {
             slot = leaf_first(cur);
             const uint4 m = __ldg(V.meta + slot);
-            orank = object_rank(m, slot);
             const uint32_t shape = m.x & 0xff;
             if (shape == AE_SHAPE_MESH) {
                 // ToLocal (hybrid:534-543), as trace_mesh.
@@ -123,11 +121,8 @@ struct Walker {
                 const float4 a = __ldg(ip), b = __ldg(ip + 1), c = __ldg(ip + 2);
                 lo = quat_rotate(-b.x, -b.y, -b.z, b.w, o - mk(a.x, a.y, a.z));
                 ld = quat_rotate(-b.x, -b.y, -b.z, b.w, d);
-                if (a.w != 0.0f && a.w != 1.0f) {
-                    const float inv = AE_DIV(1.0f, a.w);
-                    lo = lo * inv;
-                    ld = ld * inv;
-                }
+                lo = lo * c.z;
+                ld = ld * c.z;
                 linv = mk(slab_inv(ld.x), slab_inv(ld.y), slab_inv(ld.z));
                 if (WT) W = wt_setup(ld);
                 tri_base = __float_as_uint(c.y);
@@ -143,9 +138,9 @@ struct Walker {
             else if (shape == AE_SHAPE_QUAD) hit = hit_planar_ref(obj, false, o, d, tn, best.t, h);
             else if (shape == AE_SHAPE_TRIANGLE) hit = hit_planar_ref(obj, true, o, d, tn, best.t, h);
             else hit = hit_box_ref(obj, o, d, tn, best.t, h);
-            if (hit && takes(best, h.t, orank, 0u, 0u)) {
+            if (hit && takes(V, best, h.t, slot, 0u, 0u)) {
                 best.t = h.t; best.alpha = h.alpha; best.beta = h.beta;
-                best.object = slot; best.prim = AE_MISS; best.orank = orank; best.lrank = 0;
+                best.object = slot; best.prim = AE_MISS; best.lrank = 0;
             }
             pop(K, stk, tid, nt);
             return phase == kWalkDone;
