@@ -710,10 +710,10 @@ void destroy_fast(Ctx *c) {
 // 6 resident blocks left the latency-bound walk short of warps.
 template <bool WT>
 __global__ void __launch_bounds__(128, 8) k_closest_fast(DevScene S, FastView V, const ae_ray *__restrict__ rays,
-                                                      uint32_t n, ae_hit *__restrict__ hits) {
+                                                      uint32_t n, uint32_t lanes, ae_hit *__restrict__ hits) {
     extern __shared__ uint2 stk[];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const uint32_t lane = threadIdx.x & 31u, i = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * lanes + lane;
+    if (lane >= lanes || i >= n) return;
     const float4 *rp = reinterpret_cast<const float4 *>(rays + i);
     const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
     const Best best = closest_fast<WT>(S, V, mk(r0.x, r0.y, r0.z), mk(r1.x, r1.y, r1.z), r0.w, r1.w, stk,
@@ -775,11 +775,12 @@ __global__ void __launch_bounds__(128, kWalkBlocksPerSm) k_closest_walk(DevScene
                                                                      ae_hit *__restrict__ hits, uint32_t *next) {
     extern __shared__ uint2 stk[];
     if (!DYN) {
-        const uint32_t stride = gridDim.x * blockDim.x;
-        uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+        const uint32_t warps = gridDim.x * (blockDim.x / 32), lanes = spread_lanes(n, warps);
+        const uint32_t stride = warps * lanes;
+        uint32_t k = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * lanes + (threadIdx.x & 31u);
         Walker<false> w;
         WalkStacks<> K;
-        bool active = k < n;
+        bool active = (threadIdx.x & 31u) < lanes && k < n;
         if (active) {
             const ae_ray r = rays[k];
             w.start(V, mk(r.ox, r.oy, r.oz), mk(r.dx, r.dy, r.dz), r.tnear, r.time);
@@ -879,7 +880,7 @@ cudaError_t launch_closest_walk(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         per_sm = std::max(per_sm, 1);
     }
-    const uint32_t grid = std::min<uint32_t>(uint32_t(per_sm) * uint32_t(sms), (n + threads - 1) / threads);
+    const uint32_t grid = std::min<uint32_t>(uint32_t(per_sm) * uint32_t(sms), (n + 3) / 4);  // at least a ray a warp
     if (n < kWalkDynamicMin) {
         k_closest_walk<false><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, hits, nullptr);
         return cudaGetLastError();
@@ -915,12 +916,22 @@ cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
     FastView V = fast_view(F);
     const int threads = 128;
     const size_t smem = size_t(kSharedStack) * threads * sizeof(uint2);
+    // Fewer rays than the GPU holds at once: fewer of them in each warp.
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        sms = std::max(sms, 1);
+    }
+    const uint32_t per_block = threads / 32, lanes = spread_lanes(n, uint32_t(sms) * 8u * per_block);
+    const uint32_t grid = uint32_t((uint64_t(n) + per_block * lanes - 1) / (per_block * lanes));
     if (quant) {
         cudaFuncSetAttribute(k_closest_fast<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        k_closest_fast<true><<<(n + threads - 1) / threads, threads, smem, st>>>(c->scene(), V, rays, n, hits);
+        k_closest_fast<true><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, lanes, hits);
     } else {
         cudaFuncSetAttribute(k_closest_fast<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        k_closest_fast<false><<<(n + threads - 1) / threads, threads, smem, st>>>(c->scene(), V, rays, n, hits);
+        k_closest_fast<false><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, lanes, hits);
     }
     return cudaGetLastError();
 }

@@ -207,13 +207,15 @@ template <bool DYN>
 __global__ void __launch_bounds__(128, kWalkBlocksPerSm) k_sv_extend_walk(SvView W, int q, uint32_t run) {
     extern __shared__ uint2 stk[];
     const uint32_t count = W.cnt[q];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t warps = gridDim.x * (blockDim.x / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
+    const uint32_t stride = warps * lanes;
+    uint32_t k = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * lanes + lane;
+    run = min(run, lanes);
     Walker<false> w;
     WalkStacks<> K;
     const SceneRec *R = nullptr;
-    bool active = !DYN && k < count;
-    bool need = DYN, exhausted = false;
+    bool active = !DYN && lane < lanes && k < count;
+    bool need = DYN && lane < lanes, exhausted = false;
     uint32_t cbase = 0, cend = 0;
     auto begin = [&]() {
         const ae_ray r = W.qray[q][k];
@@ -296,16 +298,18 @@ __global__ void __launch_bounds__(THREADS, kWalkBlocksPerSm * 128 / THREADS) k_s
     // sample's scene (its slot's) is read through the scene table.
     extern __shared__ uint2 stk[];
     const uint32_t count = W.cnt[SV_SH];
-    const uint32_t stride = gridDim.x * THREADS;
-    uint32_t k = blockIdx.x * THREADS + threadIdx.x;
+    const uint32_t warps = gridDim.x * (THREADS / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
+    const uint32_t stride = warps * lanes;
+    uint32_t k = (blockIdx.x * (THREADS / 32) + threadIdx.x / 32) * lanes + lane;
+    run = min(run, lanes);
     Walker<false> w;
     WalkStacks<> K;
     const SceneRec *R = nullptr;
     uint32_t e = 0;
     f3 so, sd, lp;
     int step = 0;
-    bool active = !DYN && k < count;
-    bool need = DYN, exhausted = false;
+    bool active = !DYN && lane < lanes && k < count;
+    bool need = DYN && lane < lanes, exhausted = false;
     uint32_t cbase = 0, cend = 0;
     auto begin = [&]() {
         e = W.sq[k];

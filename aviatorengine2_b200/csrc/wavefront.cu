@@ -226,12 +226,14 @@ __global__ void __launch_bounds__(128, MINB) k_wf_extend_walk(DevScene S, FastVi
     extern __shared__ uint2 stk[];
     const int q = bounce & 1;
     const uint32_t count = W.cnt[q];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t warps = gridDim.x * (blockDim.x / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
+    const uint32_t stride = warps * lanes;
+    uint32_t k = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * lanes + lane;
+    run = min(run, lanes);
     Walker<WT> w;
     WalkStacks<> K;
-    bool active = !DYN && k < count;
-    bool need = DYN, exhausted = false;
+    bool active = !DYN && lane < lanes && k < count;
+    bool need = DYN && lane < lanes, exhausted = false;
     uint32_t cbase = 0, cend = 0;
     if (active) {
         const ae_ray r = W.qray[q][k];
@@ -322,15 +324,17 @@ __global__ void __launch_bounds__(THREADS, MINB * 128 / THREADS)
     k_wf_shadow(DevScene S, FastView V, WfView W, int bounce, uint32_t run) {
     extern __shared__ uint2 stk[];
     const uint32_t count = W.cnt[C_SH];
-    const uint32_t stride = gridDim.x * THREADS;
-    uint32_t k = blockIdx.x * THREADS + threadIdx.x;
+    const uint32_t warps = gridDim.x * (THREADS / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
+    const uint32_t stride = warps * lanes;
+    uint32_t k = (blockIdx.x * (THREADS / 32) + threadIdx.x / 32) * lanes + lane;
+    run = min(run, lanes);
     Walker<WT> w;
     WalkStacks<> K;
     uint32_t e = 0;
     float lim = 0.0f;  // the sample's cut-off |lp - so| - 0.001; the ray itself lives in the walker (w.o, w.d)
     int step = 0;
-    bool active = !DYN && k < count;
-    bool need = DYN, exhausted = false;
+    bool active = !DYN && lane < lanes && k < count;
+    bool need = DYN && lane < lanes, exhausted = false;
     uint32_t cbase = 0, cend = 0;
     // Starts sample k of the queue.
     auto begin = [&]() {
