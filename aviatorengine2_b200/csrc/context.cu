@@ -18,6 +18,8 @@
 #include <vector>
 
 #include "context.h"
+#include "exact_trace.cuh"
+#include "fast.h"
 #include "kernels.h"
 #include "trace_common.cuh"
 
@@ -377,9 +379,15 @@ int ae_upload_scene(ae_ctx *ctx, const ae_object *objects, uint32_t n_objects, c
     c->host_tlas.assign(tlas, tlas + n_nodes);
     c->host_instances.assign(instances, instances + n_instances);
     c->host_lights.assign(light_ids, light_ids + n_lights);
-    c->scene_has_ggx = false;
-    for (uint32_t i = 0; i < n_objects; i++)
-        if (objects[i].colorType == AE_MAT_GGX_METAL) c->scene_has_ggx = true;
+    c->scene_triangles = 0;
+    for (uint32_t i = 0; i < n_instances; i++) c->scene_triangles += instances[i].triangleCount;
+    c->scene_has_ggx = c->scene_has_media = c->scene_has_moving_spheres = false;
+    for (uint32_t i = 0; i < n_objects; i++) {
+        const ae_object &o = objects[i];
+        if (o.colorType == AE_MAT_GGX_METAL) c->scene_has_ggx = true;
+        if (o.colorType == AE_MAT_ISOTROPIC) c->scene_has_media = true;
+        if (o.shapeType == AE_SHAPE_SPHERE && !(o.x == o.x2 && o.y == o.y2 && o.z == o.z2)) c->scene_has_moving_spheres = true;
+    }
     c->scene_uploaded = true;
     c->scene_version++;
     c->scene_version_layout++;
@@ -453,7 +461,8 @@ int ae_render_frame(ae_ctx *ctx, int mode, const ae_gbuffer *gb) {
     switch (mode) {
     case AE_MODE_COMPUTE_ONLY:
         if ((rc = c->timed_begin())) return rc;
-        if ((rc = c->cuda(launch_render_plain(c->scene(), F, c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
+        if ((rc = c->cuda(launch_render_plain(c->scene(), exact_view(c, uint64_t(F.width) * F.height * F.spp), F, c->accum.ptr,
+                                             c->display.ptr, c->frame.ptr, c->stream),
                           "render (compute-only)")))
             return rc;
         return c->timed_end();

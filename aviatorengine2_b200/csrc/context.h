@@ -81,6 +81,8 @@ struct Ctx {
     std::vector<ae_instance> host_instances;
     std::vector<uint32_t> host_lights;
     bool scene_uploaded = false;
+    uint64_t scene_triangles = 0;  // over all instances
+    bool scene_has_media = false, scene_has_moving_spheres = false;
     bool scene_has_ggx = false;  // an object uses AE_MAT_GGX_METAL (not shaded by the hybrid passes)
     uint32_t fault_tile_wait = 0;  // ae_debug_inject(AE_FAULT_TILE_WAIT)
     uint32_t fault_check_limits = 0;  // ae_debug_inject(AE_FAULT_CHECK_LIMITS)
@@ -108,7 +110,7 @@ struct Ctx {
     // Optimised forms.
     FastScene *fast = nullptr;
     bool fast_ready = false;
-    uint64_t fast_version = 0;
+    uint64_t fast_accepted = ~0ull;  // scene_version that prepare_fast last accepted
     Wavefront *wave = nullptr;
     Deferred *deferred = nullptr;
     Refit *refit = nullptr;

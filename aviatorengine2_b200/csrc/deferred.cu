@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "context.h"
+#include "exact_trace.cuh"
 #include "fast.h"
 #include "kernels.h"
 #include "shade.cuh"
@@ -170,12 +171,6 @@ AE_DEV bool occluded_mesh(const DevScene &S, uint32_t ii, f3 o, f3 d, float tn, 
     return false;
 }
 
-// IsRasterProxy, deferred:1011-1017 (renderer/renderer.h:317-323).
-AE_DEV bool is_raster_proxy(const ae_object *obj, const ObjHead &hd) {
-    return hd.shape == AE_SHAPE_BOX && hd.material != AE_MAT_ISOTROPIC && hd.texture == AE_NO_TEXTURE &&
-           ld4(reinterpret_cast<const char *>(obj) + 64).w == 0.0f;
-}
-
 AE_DEV bool hit_object_deferred(const DevScene &S, const ae_object *obj, const ObjHead &hd, f3 o, f3 d, float time,
                                 float tn, float tf, DHit &h, uint32_t &seed) {
     if (hd.material == AE_MAT_ISOTROPIC) return hit_volume_ref(obj, hd.shape, o, d, time, tn, tf, h, seed);
@@ -258,6 +253,35 @@ AE_DEV bool occluded(const DevScene &S, f3 o, f3 d, float time, float tn, float 
         }
     }
     return false;
+}
+
+// The same two traversals answered on the optimised structures where those
+// decide a ray (X->on), by the walks above for the rest.  Kept out of line:
+// the resolve calls them from four places.
+__device__ __noinline__ bool traverse_undecided(const DevScene &S, f3 o, f3 d, float time, float tn, float far_limit,
+                                                bool skip_raster, DHit &out, uint32_t &seed) {
+    return traverse_bounded(S, o, d, time, tn, far_limit, skip_raster, out, seed);
+}
+__device__ __noinline__ bool occluded_undecided(const DevScene &S, f3 o, f3 d, float time, float tn, float tf,
+                                                uint32_t &seed) {
+    return occluded(S, o, d, time, tn, tf, seed);
+}
+template <bool EXACT, int OBJECTS>
+AE_DEV bool traverse_deferred(const DevScene &S, const ExactView &X, f3 o, f3 d, float time, float tn, float far_limit,
+                              DHit &out, uint32_t &seed, uint2 *stk) {
+    if (!EXACT) return traverse_bounded(S, o, d, time, tn, far_limit, OBJECTS == kTracedObjects, out, seed);
+    Best b;
+    const int r = closest_exact<OBJECTS, kSharedStack>(S, X, o, d, time, tn, far_limit, far_limit, b, stk, threadIdx.x, 128);
+    if (r == kUndecided) return traverse_undecided(S, o, d, time, tn, far_limit, OBJECTS == kTracedObjects, out, seed);
+    if (r == kExactHit) exact_hit_record(S, b, o, d, time, out);
+    return r == kExactHit;
+}
+template <bool EXACT>
+AE_DEV bool occluded_deferred(const DevScene &S, const ExactView &X, f3 o, f3 d, float time, float tn, float tf,
+                              uint32_t &seed, uint2 *stk) {
+    if (!EXACT) return occluded(S, o, d, time, tn, tf, seed);
+    const int r = occluded_exact<kSharedStack>(S, X, o, d, time, tn, tf, stk, threadIdx.x, 128);
+    return r == kUndecided ? occluded_undecided(S, o, d, time, tn, tf, seed) : r == kExactHit;
 }
 
 // ---------------------------------------------------------------------------
@@ -362,7 +386,8 @@ AE_DEV void sample_light_d(const ae_object *L, uint32_t shape, f3 from, f3 &p, f
 
 // CalculateDirectLight with the any-hit shadow ray, deferred:1376-1446, then
 // the clamp of ClampedDirectLight, deferred:1556-1569.
-AE_DEV f3 clamped_direct(const DevScene &S, const SurfRec &h, float time, uint32_t &seed) {
+template <bool EXACT>
+AE_DEV f3 clamped_direct(const DevScene &S, const ExactView &X, const SurfRec &h, float time, uint32_t &seed, uint2 *stk) {
     f3 acc = splat(0.0f);
     for (uint32_t i = 0; i < S.n_lights; i++) {
         const ae_object *L = S.objects + __ldg(S.lights + i);
@@ -378,7 +403,7 @@ AE_DEV f3 clamped_direct(const DevScene &S, const SurfRec &h, float time, uint32
         const float ct = dot(h.n, sd);
         if (ct <= 0.0f) continue;
         const f3 so = h.p + h.n * 0.001f;
-        if (!occluded(S, so, sd, time, 0.001f, AE_SUB(dist, 0.001f), seed)) {
+        if (!occluded_deferred<EXACT>(S, X, so, sd, time, 0.001f, AE_SUB(dist, 0.001f), seed, stk)) {
             const char *lb = reinterpret_cast<const char *>(L);
             const float4 m0 = ld4(lb + 80), m1 = ld4(lb + 96);
             const f3 rad = m0.y * mk(m1.x, m1.y, m1.z);
@@ -391,8 +416,9 @@ AE_DEV f3 clamped_direct(const DevScene &S, const SurfRec &h, float time, uint32
 }
 
 // TraceIndirect, deferred:1575-1646.
-AE_DEV f3 trace_indirect(const DevScene &S, const DefParams &P, f3 pd, float time, const SurfRec &surf,
-                         uint32_t &seed) {
+template <bool EXACT>
+AE_DEV f3 trace_indirect(const DevScene &S, const ExactView &X, const DefParams &P, f3 pd, float time,
+                         const SurfRec &surf, uint32_t &seed, uint2 *stk) {
     f3 bd;
     if (!bounce_dir(pd, surf, bd, seed)) return splat(0.0f);
     f3 d = normalize(bd);
@@ -402,7 +428,7 @@ AE_DEV f3 trace_indirect(const DevScene &S, const DefParams &P, f3 pd, float tim
     f3 acc = splat(0.0f);
     for (uint32_t b = 1; b < P.F.depth; b++) {
         DHit h;
-        if (!traverse_bounded(S, o, d, time, 0.001f, 1000000.0f, false, h, seed)) {
+        if (!traverse_deferred<EXACT, kAllObjects>(S, X, o, d, time, 0.001f, 1000000.0f, h, seed, stk)) {
             acc = acc + thr * P.F.sky;
             break;
         }
@@ -411,7 +437,7 @@ AE_DEV f3 trace_indirect(const DevScene &S, const DefParams &P, f3 pd, float tim
             acc = acc + thr * (s.emission * s.albedo);
             break;
         }
-        if (s.type == AE_MAT_LAMBERTIAN) acc = acc + thr * clamped_direct(S, s, time, seed);
+        if (s.type == AE_MAT_LAMBERTIAN) acc = acc + thr * clamped_direct<EXACT>(S, X, s, time, seed, stk);
         f3 nx;
         if (!bounce_dir(d, s, nx, seed)) break;
         d = normalize(nx);
@@ -548,57 +574,76 @@ struct Images {
     uchar4 *display;
 };
 
+// Closest hit over what the rasterizer draws (meshes and raster proxies): the
+// reference's compute-only walk restricted by shape.
+AE_DEV bool traverse_raster(const DevScene &S, f3 o, f3 d, DHit &best) {
+    if (S.n_nodes == 0) return false;
+    const f3 inv = 1.0f / d;
+    int stack[kTlasStack];
+    int sp = 0;
+    stack[sp++] = 0;
+    float tf = kFarStart;
+    bool found = false;
+    while (sp > 0) {
+        const NodeBox n = load_node(S.tlas, uint32_t(stack[--sp]));
+        if (!slab_ref(o, inv, n.lo, n.hi, 0.001f, tf)) continue;
+        if (n.count > 0) {
+            for (int i = 0; i < n.count; i++) {
+                const uint32_t slot = uint32_t(n.left + i);
+                const ae_object *obj = S.objects + slot;
+                const ObjHead hd = load_head(obj);
+                DHit h;
+                bool hit = false;
+                if (hd.shape == AE_SHAPE_MESH) {
+                    const uint32_t ii = __float_as_uint(ld4(reinterpret_cast<const char *>(obj) + 80).z);
+                    hit = hit_mesh_ref(S, ii, o, d, 0.001f, tf, h);
+                } else if (is_raster_proxy(obj, hd)) {
+                    hit = hit_box_ref(obj, o, d, 0.001f, tf, h);
+                }
+                if (hit) {
+                    tf = h.t;
+                    h.slot = slot;
+                    best = h;
+                    found = true;
+                }
+            }
+        } else if (sp + 2 <= kTlasStack) {
+            stack[sp++] = n.left;
+            stack[sp++] = n.right;
+        }
+    }
+    return found;
+}
+__device__ __noinline__ bool raster_undecided(const DevScene &S, f3 o, f3 d, DHit &best) { return traverse_raster(S, o, d, best); }
+
 // The G-buffer through pixel centre + jitter: closest hit over the objects
 // the rasterizer draws.  Writes zero coverage where nothing is drawn, as the
 // raster pass clears its targets (renderer/renderer.cpp:1221-1233).
-__global__ void __launch_bounds__(128) k_gbuffer(DevScene S, DefParams P, GBuf G) {
+template <bool EXACT>
+__global__ void __launch_bounds__(128) k_gbuffer(DevScene S, ExactView X, DefParams P, GBuf G) {
+    extern __shared__ uint2 stk[];
     const uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15);
     const uint32_t y = blockIdx.y * 8 + (threadIdx.x >> 4);
     if (x >= P.F.width || y >= P.F.height) return;
     const size_t px = size_t(y) * P.F.width + x;
     const f3 sample = P.F.pixel0 + AE_ADD(AE_U2F(x), P.jitter_x) * P.F.pixel_u + AE_ADD(AE_U2F(y), P.jitter_y) * P.F.pixel_v;
     const f3 o = P.F.source, d = normalize(sample - o);
-    // Closest hit over meshes and raster proxies: the reference's compute-only
-    // walk restricted by shape.
     float4 pos = make_float4(0, 0, 0, 0), nrm = make_float4(0, 0, 0, 0);
     uchar4 alb = make_uchar4(0, 0, 0, 0);
     float depth = 1.0f;
-    if (S.n_nodes > 0) {
-        const f3 inv = 1.0f / d;
-        int stack[kTlasStack];
-        int sp = 0;
-        stack[sp++] = 0;
-        float tf = kFarStart;
-        bool found = false;
-        DHit best;
-        while (sp > 0) {
-            const NodeBox n = load_node(S.tlas, uint32_t(stack[--sp]));
-            if (!slab_ref(o, inv, n.lo, n.hi, 0.001f, tf)) continue;
-            if (n.count > 0) {
-                for (int i = 0; i < n.count; i++) {
-                    const uint32_t slot = uint32_t(n.left + i);
-                    const ae_object *obj = S.objects + slot;
-                    const ObjHead hd = load_head(obj);
-                    DHit h;
-                    bool hit = false;
-                    if (hd.shape == AE_SHAPE_MESH) {
-                        const uint32_t ii = __float_as_uint(ld4(reinterpret_cast<const char *>(obj) + 80).z);
-                        hit = hit_mesh_ref(S, ii, o, d, 0.001f, tf, h);
-                    } else if (is_raster_proxy(obj, hd)) {
-                        hit = hit_box_ref(obj, o, d, 0.001f, tf, h);
-                    }
-                    if (hit) {
-                        tf = h.t;
-                        h.slot = slot;
-                        best = h;
-                        found = true;
-                    }
-                }
-            } else if (sp + 2 <= kTlasStack) {
-                stack[sp++] = n.left;
-                stack[sp++] = n.right;
-            }
-        }
+    DHit best;
+    bool found;
+    if (EXACT) {
+        Best b;
+        const int r = closest_exact<kRasterObjects, kSharedStack>(S, X, o, d, 0.0f, 0.001f, kFarStart, kFarStart, b, stk,
+                                                                  threadIdx.x, 128);
+        found = r == kExactHit;
+        if (found) exact_hit_record(S, b, o, d, 0.0f, best);
+        else if (r == kUndecided) found = raster_undecided(S, o, d, best);
+    } else {
+        found = traverse_raster(S, o, d, best);
+    }
+    {
         if (found) {
             const ae_object *obj = S.objects + best.slot;
             const MatRec mat = load_mat(obj);
@@ -628,8 +673,9 @@ __global__ void __launch_bounds__(128) k_gbuffer(DevScene S, DefParams P, GBuf G
 
 // ResolvePrimary with HitFromGBuffer, deferred:1452-1548.  Returns 0 sky,
 // 1 raster, 2 analytic.
-AE_DEV int resolve_primary(const DevScene &S, const GBuf &G, size_t px, f3 o, f3 d, float time, SurfRec &hit,
-                           uint32_t &seed) {
+template <bool EXACT>
+AE_DEV int resolve_primary(const DevScene &S, const ExactView &X, const GBuf &G, size_t px, f3 o, f3 d, float time,
+                           SurfRec &hit, uint32_t &seed, uint2 *stk) {
     SurfRec raster;
     bool has_raster = false;
     float far_limit = 1000000.0f;
@@ -655,7 +701,7 @@ AE_DEV int resolve_primary(const DevScene &S, const GBuf &G, size_t px, f3 o, f3
         }
     }
     DHit ah;
-    if (traverse_bounded(S, o, d, time, 0.001f, far_limit, true, ah, seed)) {
+    if (traverse_deferred<EXACT, kTracedObjects>(S, X, o, d, time, 0.001f, far_limit, ah, seed, stk)) {
         hit = surf_from_hit(S, ah, o, d);
         return 2;
     }
@@ -679,8 +725,9 @@ AE_DEV f3 false_colour(uint32_t t) {
 }
 
 // DebugColour, deferred:1667-1722 (WorldFromDepth, deferred:1503-1514).
-AE_DEV f3 debug_colour(const DevScene &S, const DefParams &P, const GBuf &G, size_t px, f3 o, f3 d, float time,
-                       uint32_t &seed) {
+template <bool EXACT>
+AE_DEV f3 debug_colour(const DevScene &S, const ExactView &X, const DefParams &P, const GBuf &G, size_t px, f3 o, f3 d,
+                       float time, uint32_t &seed, uint2 *stk) {
     const float4 pn = G.nrm[px];
     const bool covered = pn.w >= 0.5f;
     const f3 background = mk(0.0f, 0.0f, 0.0f);
@@ -707,14 +754,16 @@ AE_DEV f3 debug_colour(const DevScene &S, const DefParams &P, const GBuf &G, siz
         return splat(AE_MUL(rel, 100.0f));
     }
     SurfRec hit;
-    const int source = resolve_primary(S, G, px, o, d, time, hit, seed);
+    const int source = resolve_primary<EXACT>(S, X, G, px, o, d, time, hit, seed, stk);
     if (P.debug_view == 4) return source != 0 ? false_colour(hit.type) : background;
     if (source == 1) return mk(0.1f, 0.8f, 0.2f);
     if (source == 2) return mk(0.85f, 0.15f, 0.1f);
     return mk(0.1f, 0.15f, 0.5f);
 }
 
-__global__ void __launch_bounds__(128) k_deferred(DevScene S, DefParams P, GBuf G, Images I) {
+template <bool EXACT>
+__global__ void __launch_bounds__(128) k_deferred(DevScene S, ExactView X, DefParams P, GBuf G, Images I) {
+    extern __shared__ uint2 stk[];
     const uint32_t cx = blockIdx.x * 16 + (threadIdx.x & 15);
     const uint32_t cy = blockIdx.y * 8 + (threadIdx.x >> 4);
     if (cx >= P.ext_w || cy >= P.ext_h) return;
@@ -734,7 +783,7 @@ __global__ void __launch_bounds__(128) k_deferred(DevScene S, DefParams P, GBuf 
     const f3 d = normalize(sample - o);
     const float time = rng_next(seed);
     if (P.debug_view != 0) {
-        const f3 c = debug_colour(S, P, G, px, o, d, time, seed);
+        const f3 c = debug_colour<EXACT>(S, X, P, G, px, o, d, time, seed, stk);
         const f3 q = saturate(c);
         I.display[px] = make_uchar4((unsigned char)(int)AE_RINT(AE_MUL(q.x, 255.0f)),
                                     (unsigned char)(int)AE_RINT(AE_MUL(q.y, 255.0f)),
@@ -744,7 +793,7 @@ __global__ void __launch_bounds__(128) k_deferred(DevScene S, DefParams P, GBuf 
     // ResolvePrimary, deferred:1526-1548.
     f3 color = splat(0.0f);
     SurfRec hit;
-    const int source = resolve_primary(S, G, px, o, d, time, hit, seed);
+    const int source = resolve_primary<EXACT>(S, X, G, px, o, d, time, hit, seed, stk);
     const bool has = source != 0;
     if (!has) {
         color = P.F.sky;
@@ -752,8 +801,8 @@ __global__ void __launch_bounds__(128) k_deferred(DevScene S, DefParams P, GBuf 
         color = hit.emission * hit.albedo;
     } else {
         for (uint32_t s = 0; s < P.spp; s++) {
-            if (hit.type == AE_MAT_LAMBERTIAN) color = color + clamped_direct(S, hit, time, seed);
-            color = color + trace_indirect(S, P, d, time, hit, seed);
+            if (hit.type == AE_MAT_LAMBERTIAN) color = color + clamped_direct<EXACT>(S, X, hit, time, seed, stk);
+            color = color + trace_indirect<EXACT>(S, X, P, d, time, hit, seed, stk);
         }
         color = color / AE_U2F(P.spp);
     }
@@ -900,6 +949,16 @@ static DefParams make_def_params(const Ctx *c) {
     return P;
 }
 
+// The hybrid passes on a handful of objects with a handful of triangles: the
+// reference walk is as short there, and has nothing to verify (480x270, G-buffer
+// and resolve: Cornell box, 8 objects and 34 triangles, 28 + 188 against 34 +
+// 229 us; 5 objects with 160 triangles 44 + 201 against 35 + 114 us; 17 with
+// 160 73 + 410 against 75 + 245 us).
+static ExactView hybrid_view(Ctx *c, uint64_t rays) {
+    if (c->n_objects < 16 && c->scene_triangles < 128) return ExactView{};
+    return exact_view(c, rays);
+}
+
 int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     int rc = ensure(c);
     if (rc) return rc;
@@ -937,7 +996,9 @@ int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     if ((rc = c->timed_begin())) return rc;
     if (!(P.reduced && P.F.display_only)) {
         dim3 grid((P.ext_w + 15) / 16, (P.ext_h + 7) / 8);
-        k_deferred<<<grid, 128, 0, c->stream>>>(c->scene(), P, G, I);
+        const ExactView X = P.F.display_only ? ExactView{} : hybrid_view(c, uint64_t(P.ext_w) * P.ext_h * P.spp);
+        if (X.on) k_deferred<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), c->stream>>>(c->scene(), X, P, G, I);
+        else k_deferred<false><<<grid, 128, 0, c->stream>>>(c->scene(), X, P, G, I);
         if ((rc = c->cuda(cudaGetLastError(), "deferred launch"))) return rc;
         c->launches++;
     }
@@ -1007,7 +1068,9 @@ extern "C" int ae_build_gbuffer(ae_ctx *ctx) {
     const DefParams P = make_def_params(c);
     GBuf G{D.gpos.ptr, D.gnrm.ptr, D.galb.ptr, D.gdepth.ptr};
     dim3 grid((P.F.width + 15) / 16, (P.F.height + 7) / 8);
-    k_gbuffer<<<grid, 128, 0, c->stream>>>(c->scene(), P, G);
+    const ExactView X = hybrid_view(c, uint64_t(P.F.width) * P.F.height);
+    if (X.on) k_gbuffer<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), c->stream>>>(c->scene(), X, P, G);
+    else k_gbuffer<false><<<grid, 128, 0, c->stream>>>(c->scene(), X, P, G);
     c->launches++;
     if ((rc = c->cuda(cudaGetLastError(), "G-buffer launch"))) return rc;
     D.have_gbuffer = true;
@@ -1017,13 +1080,16 @@ extern "C" int ae_build_gbuffer(ae_ctx *ctx) {
 // Any hit in [tnear, tmax] with deferred.comp's blocking rules (Occluded,
 // deferred:1115-1171): glass and lights never block; meshes take the any-hit
 // walk (OccludedMesh, deferred:812-854).  One thread per ray.
-__global__ void __launch_bounds__(128) k_any_hit(DevScene S, const ae_ray *__restrict__ rays,
+template <bool EXACT>
+__global__ void __launch_bounds__(128) k_any_hit(DevScene S, ExactView X, const ae_ray *__restrict__ rays,
                                                  const float *__restrict__ tmax, uint32_t n, uint8_t *__restrict__ out) {
+    extern __shared__ uint2 stk[];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const ae_ray r = rays[i];
     uint32_t seed = 1u;
-    out[i] = occluded(S, mk(r.ox, r.oy, r.oz), mk(r.dx, r.dy, r.dz), r.time, r.tnear, tmax[i], seed) ? 1 : 0;
+    out[i] = occluded_deferred<EXACT>(S, X, mk(r.ox, r.oy, r.oz), mk(r.dx, r.dy, r.dz), r.time, r.tnear, tmax[i], seed, stk) ? 1
+                                                                                                                          : 0;
 }
 
 extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, uint32_t n, uint8_t *out) {
@@ -1039,8 +1105,12 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
     int rc = c->cuda(cudaMemcpyAsync(dr.ptr, rays, size_t(n) * sizeof(ae_ray), cudaMemcpyHostToDevice, c->stream), "copy");
     if (!rc) rc = c->cuda(cudaMemcpyAsync(dt.ptr, tmax, size_t(n) * sizeof(float), cudaMemcpyHostToDevice, c->stream), "copy");
     if (rc) return rc;
+    const ExactView X = exact_view(c, n);
     if ((rc = c->timed_begin())) return rc;
-    k_any_hit<<<(n + 127) / 128, 128, 0, c->stream>>>(c->scene(), dr.ptr, dt.ptr, n, dout.ptr);
+    if (X.on)
+        k_any_hit<true><<<(n + 127) / 128, 128, size_t(kSharedStack) * 128 * sizeof(uint2), c->stream>>>(c->scene(), X, dr.ptr,
+                                                                                                     dt.ptr, n, dout.ptr);
+    else k_any_hit<false><<<(n + 127) / 128, 128, 0, c->stream>>>(c->scene(), X, dr.ptr, dt.ptr, n, dout.ptr);
     if ((rc = c->cuda(cudaGetLastError(), "any-hit launch"))) return rc;
     if ((rc = c->timed_end())) return rc;
     rc = c->cuda(cudaMemcpyAsync(out, dout.ptr, n, cudaMemcpyDeviceToHost, c->stream), "copy");

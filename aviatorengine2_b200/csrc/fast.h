@@ -8,6 +8,8 @@ int prepare_fast(Ctx *c);
 // Nodes and triangle records of the listed meshes on the device (fast_build.cu).
 int build_mesh_structures(Ctx *c, FastScene &F);
 int prepare_precision(Ctx *c);
+struct ExactView;
+ExactView exact_view(Ctx *c, uint64_t rays);
 void destroy_fast(Ctx *c);
 cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, bool quant, cudaStream_t st);
 cudaError_t launch_closest_walk(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, cudaStream_t st);

@@ -33,7 +33,7 @@ namespace {
 
 constexpr int kMaxLevels = 32;  // uploads are checked to kBlasStack (24) pending nodes, so at most 23 levels
 // Device words of a build: level sizes, then the flags below.
-enum { W_STACK = kMaxLevels, W_ERROR, W_TOTAL, W_COUNT };
+enum { W_STACK = kMaxLevels, W_ERROR, W_TOTAL, W_FACTOR, W_COUNT };
 enum { E_LEAF = 1, E_QUANT = 2, E_SHARED = 4, E_DEPTH = 8 };
 
 struct Kids {
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(128) k_wide_emit(const ae_bvh_node *__restrict
     bool valid[4];
     for (int k = 0; k < 4; k++) {
         valid[k] = k < K.n;
-        q.child[k] = 0u;
+        q.child[k] = kNoChild;
         if (!valid[k]) continue;
         const uint32_t g = base + K.k[k];
         const ae_bvh_node c = blas[g];
@@ -201,8 +201,12 @@ struct MeshJob {
 };
 static_assert(sizeof(MeshJob) == 16, "four words in the build's tables");
 __global__ void __launch_bounds__(256) k_tri_records(const ae_vertex *__restrict__ v, const uint32_t *__restrict__ idx,
-                                                     const MeshJob *__restrict__ jobs, float4 *__restrict__ out) {
+                                                     const MeshJob *__restrict__ jobs, float4 *__restrict__ out,
+                                                     uint32_t *words) {
     const MeshJob J = jobs[blockIdx.y];
+    // Largest |e1| |e2| / |e1 x e2| of the triangles that the reference test can
+    // accept (exact_trace.cuh), 1 and up; as bits, which order like the floats.
+    uint32_t factor = 0;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < J.tris; t += gridDim.x * blockDim.x) {
         const uint32_t *ix = idx + J.index_base + 3u * t;
         const ae_vertex *a = v + J.vertex_base + ix[0], *b = v + J.vertex_base + ix[1], *c = v + J.vertex_base + ix[2];
@@ -210,7 +214,16 @@ __global__ void __launch_bounds__(256) k_tri_records(const ae_vertex *__restrict
         o[0] = make_float4(a->px, a->py, a->pz, b->px);
         o[1] = make_float4(b->py, b->pz, c->px, c->py);
         o[2] = make_float4(c->pz, 0.0f, 0.0f, 0.0f);
+        const f3 p0 = mk(a->px, a->py, a->pz), e1 = mk(b->px, b->py, b->pz) - p0, e2 = mk(c->px, c->py, c->pz) - p0;
+        const f3 n = cross(e1, e2);
+        const float nn = dot(n, n);
+        if (!(nn < 1e-12f)) {
+            const float f = sqrtf(dot(e1, e1)) * sqrtf(dot(e2, e2)) / sqrtf(nn);
+            factor = max(factor, __float_as_uint(f >= 0.0f ? f : __int_as_float(0x7f800000)));
+        }
     }
+    factor = __reduce_max_sync(0xffffffffu, factor);
+    if ((threadIdx.x & 31u) == 0 && factor) atomicMax(words + W_FACTOR, factor);
 }
 
 // FP16 shading records (layout in wf_common.cuh: PrecView).
@@ -340,14 +353,18 @@ int build_mesh_structures(Ctx *c, FastScene &F) {
         F.max_stack = std::max(F.max_stack, int(w[W_STACK]));
         first_tree += trees;
     }
+    uint32_t factor = 0;
     const uint32_t gx = row_blocks(jobs);
     for_rows(jobs.size(), [&](size_t r, uint32_t rows) {
-        k_tri_records<<<dim3(gx, rows), 256, 0, st>>>(c->vertices.ptr, c->indices.ptr, d_jobs + r, F.tris.ptr);
+        k_tri_records<<<dim3(gx, rows), 256, 0, st>>>(c->vertices.ptr, c->indices.ptr, d_jobs + r, F.tris.ptr, words);
     });
     if ((rc = c->cuda(cudaGetLastError(), "triangle records")) ||
         (rc = c->cuda(cudaMemcpyAsync(host_refs.data(), refs, bases.size() * 4, cudaMemcpyDeviceToHost, st), "tree roots")) ||
+        (rc = c->cuda(cudaMemcpyAsync(&factor, words + W_FACTOR, 4, cudaMemcpyDeviceToHost, st), "triangle factor")) ||
         (rc = c->cuda(cudaStreamSynchronize(st), "triangle records")))
         return rc;
+    std::memcpy(&F.tri_factor, &factor, 4);
+    F.tri_factor = std::max(F.tri_factor, 1.0f);
     for (auto &kv : F.mesh_roots)
         kv.second.first = host_refs[std::lower_bound(bases.begin(), bases.end(), std::get<3>(kv.first)) - bases.begin()];
     return AE_OK;

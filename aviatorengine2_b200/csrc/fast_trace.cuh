@@ -17,22 +17,24 @@
 namespace ae {
 
 // A 4-wide node of the walks, 64 bytes.  `scale` holds, per axis, the biased
-// binary32 exponent of 2^14 times the node's quantum 2^e (bytes 0-2), and the
-// number of children in use (byte 3).  A child's eight bytes are its
-// quantised planes {lo x, lo y, lo z, hi x, hi y, hi z} and the two bytes
-// kPlaneB6, kPlaneB7: one byte permute of the pair with a selector that the
-// ray's direction sign picks gives the bits 0x4000qq00, the float
-// 2 + q 2^-14, so a plane costs one permute and one fma, with no conversion
-// and no subtraction of a bias.  An unused slot carries 0x7fff there, which
-// makes every plane a NaN and the interval test false.
+// binary32 exponent of the node's scale 2^e (bytes 0-2).  A child's eight
+// bytes are its quantised planes {lo x, lo y, lo z, hi x, hi y, hi z} and the two
+// bytes of kPlaneTail: one byte permute of the pair with a selector that the
+// ray's direction sign picks gives the bits 0xc0qq0000, the float -V(q) with
+// V(q) = 2 + q/64 below q = 128 and 4 + (q - 128)/32 from there on (the byte
+// spans the exponent's last bit and seven bits of the mantissa), and plane q
+// lies at o + V(q) 2^e.  So a plane costs one permute and one fma, with no
+// conversion and no subtraction of a bias.  An unused slot carries
+// kPlaneUnused: read as a float, its second word is +inf instead of a negative
+// number, which the interval test takes for an entry distance.
 struct QNode {
-    float ox, oy, oz;        // frame origin, below the node box minimum
+    float ox, oy, oz;        // frame origin, 2 * 2^e below the node box minimum
     uint32_t scale;
     uint2 plane[4];
-    uint32_t child[4];       // interior: node index; leaf: leaf_ref(first, count)
+    uint32_t child[4];       // interior: node index; leaf: leaf_ref(first, count); kNoChild
 };
 static_assert(sizeof(QNode) == 64, "QNode must be 64 bytes");
-constexpr uint32_t kPlaneTail = 0x40000000u, kPlaneUnused = 0x7fff0000u;  // bytes 6-7 of a child's planes
+constexpr uint32_t kPlaneTail = 0xc0000000u, kPlaneUnused = 0x7f800000u;  // bytes 6-7 of a child's planes
 
 // The node layout that ae_build_wide_bvh hands out (include/ae_b200.h).
 struct WideNode {            // 64 B
@@ -46,6 +48,7 @@ struct WideNode {            // 64 B
 };
 static_assert(sizeof(WideNode) == 64, "WideNode must be 64 bytes");
 constexpr uint32_t kLeafBit = 0x80000000u;
+constexpr uint32_t kNoChild = kLeafBit;  // a leaf of count 0
 // A leaf reference: bit 31 set, primitive count in bits 24-30 (1..127), first
 // slot in bits 0-23.  prepare_fast refuses meshes outside those limits.
 constexpr uint32_t kMaxLeafFirst = 1u << 24;
@@ -81,7 +84,7 @@ struct FastScene {
     DevBuf<QNode> nodes;
     DevBuf<float4> tris;     // 3 float4 per triangle
     DevBuf<FastInst> inst;
-    DevBuf<uint4> obj_meta;  // per object slot: shape | material << 8, instance
+    DevBuf<uint4> obj_meta;  // per object slot, see FastView::meta
     DevBuf<uint4> shade16;   // precision form: FP16 normals and UVs, 2 per triangle
     uint32_t shade16_tris = 0;
     // Ray counters of the batch walker (k_closest_walk), one per launch in
@@ -117,6 +120,14 @@ struct FastScene {
     DevBuf<uint32_t> tflag;       // set by the refresh when a box cannot be quantised
     std::vector<int32_t> tlevel_start;
     uint32_t troot = kEmptyTlas, n_tnodes = 0;
+    // What the exact walks need beyond (exact_trace.cuh): the triangles' shape
+    // factor A, the largest mesh-space coordinate, and per object the
+    // intersection of the reference TLAS boxes above it.
+    float tri_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
+    bool has_spheres = false, moving_spheres = false;
+    uint2 nan_ref = {0xffffffffu, 0xffffffffu}, nan_wt = {0xffffffffu, 0xffffffffu};
+    DevBuf<float4> obj_chain;
+    DevBuf<int32_t> tlas_parent;
     int tlas_stack = 0;
     float static_range = 0.0f;    // largest coordinate magnitude of the analytic objects' boxes
     uint64_t tlas_key = ~0ull, sub_key = ~0ull;
@@ -138,16 +149,21 @@ struct FastView {
     const QNode *nodes;
     const float4 *tris;
     const FastInst *inst;
-    const uint4 *meta;      // x: shape | material << 8, y: instance, z: first slot of its reference TLAS leaf
+    const uint4 *meta;      // x: shape | material << 8, y: instance, z: first slot of its reference TLAS leaf,
+                            // w: that leaf's node
     const QNode *tnodes;    // instance-level tree
     uint32_t troot;         // its root: a node index, leaf_ref(slot, 1), or kEmptyTlas
+    // What the reference walk answers a ray whose direction is NaN on every axis
+    // (a path that met a degenerate normal), by triangle test: (object slot,
+    // triangle slot), AE_MISS for none.  See nan_answers in fast.cu.
+    uint2 nan_ref, nan_wt;
 };
 
 // The view of a prepared scene; `inst` and `tnodes` may name another copy of
 // the per-frame arrays (serving frame sets).
 inline FastView fast_view(const FastScene &F, const FastInst *inst = nullptr, const QNode *tnodes = nullptr) {
     return FastView{F.nodes.ptr, F.tris.ptr, inst ? inst : F.inst.ptr, F.obj_meta.ptr, tnodes ? tnodes : F.tnodes.ptr,
-                    F.troot};
+                    F.troot, F.nan_ref, F.nan_wt};
 }
 
 // Best candidate so far.  Equal distances rank by (object rank, leaf rank,
@@ -173,6 +189,20 @@ AE_DEV bool takes(const FastView &V, const Best &b, float t, uint32_t object, ui
     if (object != b.object) return later_object(V, object, b.object);
     if (lrank != b.lrank) return lrank > b.lrank;
     return slot > b.prim;
+}
+
+// A ray without a direction: its answer is the scene's, and known.
+AE_DEV bool no_direction(f3 d) { return d.x != d.x && d.y != d.y && d.z != d.z; }
+template <bool WT>
+AE_DEV void nan_best(const FastView &V, Best &b) {
+    const uint2 h = WT ? V.nan_wt : V.nan_ref;
+    if (h.x == AE_MISS) return;
+    const float nan = __int_as_float(0x7fffffff);
+    const bool sphere = (__ldg(&V.meta[h.x].x) & 0xffu) == AE_SHAPE_SPHERE;
+    b.t = nan;
+    b.alpha = b.beta = sphere ? 0.0f : nan;
+    b.object = h.x;
+    b.prim = h.y;
 }
 
 // HitMeshTriangle (hybrid:564-598), correctly rounded; p1/p2 give e1/e2 by the
@@ -216,9 +246,8 @@ AE_DEV bool tri_test_wt(f3 o, const WtRay &W, float tn, float tf, const float4 &
 
 // Relative widening of slab intervals in the optimised walks: an interval's
 // exit and the best distance are scaled up by 1 + 2^-19 before they are
-// compared with an entry.  That covers the relative rounding of the plane
-// distances (the absolute part, under 2^-8 of a quantum, is kept free by the
-// quantiser), so neither a nearer hit nor one on a box's face is pruned.
+// compared with an entry, so neither a nearer hit nor one on a box's face is
+// pruned by the rounding of the plane distances.
 constexpr float kExitGrow = 1.0000019073486328125f;  // 1 + 2^-19
 
 AE_DEV float max3(float a, float b, float c) {
@@ -234,54 +263,66 @@ AE_DEV float min3(float a, float b, float c) {
 
 // Entry distances of a node's four child boxes; +inf for a child that the ray
 // misses or that starts beyond the best hit.  Distances are in units of the
-// ray parameter; plane q of an axis lies at (o - p)/d + q s/d, evaluated as
-// (2 + q 2^-14) ix + bx with ix = 2^14 s/d and bx = (o - p)/d - 2 ix.
+// ray parameter: plane q of an axis lies at V(q) 2^e / d + (o - p) / d.
 //
-// The walks are bound by issue slots with 11-13 of 32 lanes active, so the
+// The walks are bound by issue slots with 12-15 of 32 lanes active, so the
 // count of instructions here is what a step costs: the permute builds a
 // plane's float directly, the near and far bytes are chosen by the permute's
 // selector instead of by selects, three-operand min and max fold an interval,
-// and an unused slot rejects itself.
-AE_DEV void child_hits(const QNode *nodep, f3 o, f3 inv, float tn, float tf, float tmin[4], uint32_t child[4]) {
+// and an unused slot rejects itself.  NaN distances (a NaN in the ray) drop out
+// of min and max, so an axis without a direction bounds nothing.
+//
+// WIDE: every box is widened by a length whose extent in t is `e` per axis.
+template <bool WIDE>
+AE_DEV void child_test(const QNode *nodep, f3 o, f3 inv, f3 e, float tn, float tf, float tmin[4], uint32_t child[4]) {
     const uint4 *p = reinterpret_cast<const uint4 *>(nodep);
     const uint4 w0 = __ldg(p), pa = __ldg(p + 1), pb = __ldg(p + 2), cr = __ldg(p + 3);
-    const float ix = __uint_as_float(__byte_perm(w0.w, 0u, 0x0444u) >> 1) * inv.x;
-    const float iy = __uint_as_float(__byte_perm(w0.w, 0u, 0x1444u) >> 1) * inv.y;
-    const float iz = __uint_as_float(__byte_perm(w0.w, 0u, 0x2444u) >> 1) * inv.z;
-    const float bx = fmaf(-2.0f, ix, (__uint_as_float(w0.x) - o.x) * inv.x);
-    const float by = fmaf(-2.0f, iy, (__uint_as_float(w0.y) - o.y) * inv.y);
-    const float bz = fmaf(-2.0f, iz, (__uint_as_float(w0.z) - o.z) * inv.z);
-    // Selectors {6, q, 6, 7}: q = 0, 1, 2 for the low planes and 3, 4, 5 for
+    const float ix = __uint_as_float(__byte_perm(w0.w, 0u, 0x0444u) >> 1) * -inv.x;
+    const float iy = __uint_as_float(__byte_perm(w0.w, 0u, 0x1444u) >> 1) * -inv.y;
+    const float iz = __uint_as_float(__byte_perm(w0.w, 0u, 0x2444u) >> 1) * -inv.z;
+    const float bx = (__uint_as_float(w0.x) - o.x) * inv.x;
+    const float by = (__uint_as_float(w0.y) - o.y) * inv.y;
+    const float bz = (__uint_as_float(w0.z) - o.z) * inv.z;
+    const float nbx = WIDE ? bx - e.x : bx, nby = WIDE ? by - e.y : by, nbz = WIDE ? bz - e.z : bz;
+    const float fbx = WIDE ? bx + e.x : bx, fby = WIDE ? by + e.y : by, fbz = WIDE ? bz + e.z : bz;
+    // Selectors {6, 6, q, 7}: q = 0, 1, 2 for the low planes and 3, 4, 5 for
     // the high ones; a negative direction enters through the high plane.
-    const uint32_t nx = 0x7606u ^ (uint32_t(__float_as_int(inv.x) >> 31) & 0x30u), fx = nx ^ 0x30u;
-    const uint32_t ny = 0x7616u ^ (uint32_t(__float_as_int(inv.y) >> 31) & 0x50u), fy = ny ^ 0x50u;
-    const uint32_t nz = 0x7626u ^ (uint32_t(__float_as_int(inv.z) >> 31) & 0x70u), fz = nz ^ 0x70u;
+    const uint32_t nx = 0x7066u ^ (uint32_t(__float_as_int(inv.x) >> 31) & 0x300u), fx = nx ^ 0x300u;
+    const uint32_t ny = 0x7166u ^ (uint32_t(__float_as_int(inv.y) >> 31) & 0x500u), fy = ny ^ 0x500u;
+    const uint32_t nz = 0x7266u ^ (uint32_t(__float_as_int(inv.z) >> 31) & 0x700u), fz = nz ^ 0x700u;
     const float tfg = tf * kExitGrow;
     const uint32_t lo_w[4] = {pa.x, pa.z, pb.x, pb.z}, hi_w[4] = {pa.y, pa.w, pb.y, pb.w};
     child[0] = cr.x; child[1] = cr.y; child[2] = cr.z; child[3] = cr.w;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const float t0x = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], nx)), ix, bx);
-        const float t0y = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], ny)), iy, by);
-        const float t0z = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], nz)), iz, bz);
-        const float t1x = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fx)), ix, bx);
-        const float t1y = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fy)), iy, by);
-        const float t1z = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fz)), iz, bz);
-        const float lo = fmaxf(max3(t0x, t0y, t0z), tn);
-        const float hi = min3(t1x, t1y, t1z) * kExitGrow;
-        tmin[k] = lo <= hi && lo <= tfg ? lo : __int_as_float(0x7f800000);
+        const float t0x = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], nx)), ix, nbx);
+        const float t0y = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], ny)), iy, nby);
+        const float t0z = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], nz)), iz, nbz);
+        const float t1x = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fx)), ix, fbx);
+        const float t1y = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fy)), iy, fby);
+        const float t1z = fmaf(__uint_as_float(__byte_perm(lo_w[k], hi_w[k], fz)), iz, fbz);
+        // -2e37 and below for a slot in use, +inf for an unused one.
+        const float slot = __uint_as_float(hi_w[k]) * 1e37f;
+        const float lo = max3(max3(t0x, t0y, t0z), tn, slot);
+        const float hi = fminf(min3(t1x, t1y, t1z) * kExitGrow, tfg);
+        tmin[k] = lo <= hi ? lo : __int_as_float(0x7f800000);
     }
 }
 
+AE_DEV void child_hits(const QNode *nodep, f3 o, f3 inv, float tn, float tf, float tmin[4], uint32_t child[4]) {
+    child_test<false>(nodep, o, inv, mk(0.0f, 0.0f, 0.0f), tn, tf, tmin, child);
+}
+
 // Safe reciprocal for slab tests: a zero component becomes a huge finite
-// value of the same sign, so products stay finite (no 0 * inf).  The hardware
+// value of the same sign, so products stay finite (no 0 * inf); a power of two,
+// so that a ray in the plane of a box's face is exactly on it.  The hardware
 // reciprocal (within 1 ulp) scales an axis's plane distances by at most 2^-23,
 // inside the intervals' widening; a correctly rounded quotient cost about ten
 // instructions an axis.
 AE_DEV float slab_inv(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fabsf(x) > 1e-20f ? r : copysignf(1e20f, x);
+    return fabsf(x) > 1e-20f ? r : copysignf(73786976294838206464.0f, x);  // 2^66
 }
 
 // Sorts child_hits' four (distance, child) pairs nearest first (misses carry
@@ -407,6 +448,10 @@ AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float
     best.t = kFarStart; best.alpha = 0.0f; best.beta = 0.0f;
     best.object = AE_MISS; best.prim = AE_MISS; best.lrank = 0;
     if (V.troot == kEmptyTlas) return best;
+    if (no_direction(d)) {
+        nan_best<WT>(V, best);
+        return best;
+    }
     const f3 inv = mk(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
     WalkStack<SS> K;
     int sp = 0;

@@ -65,6 +65,10 @@ struct Walker {
         tinv = mk(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
         cur = V.troot;
         phase = (cur & kLeafBit) ? (leaf_count(cur) ? kWalkObject : kWalkDone) : kWalkTlas;
+        if (no_direction(d)) {
+            nan_best<WT>(V, best);
+            phase = kWalkDone;
+        }
     }
 
     // Next stack entry no farther than the best hit, or done; an entry below

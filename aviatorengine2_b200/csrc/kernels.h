@@ -10,6 +10,7 @@ namespace ae {
 
 struct DevScene;
 struct Checks;
+struct ExactView;
 
 // Everything the frame kernels derive from Config once per frame (the camera
 // basis of hybrid:1347-1361), computed on the host with the same intrinsics
@@ -31,7 +32,7 @@ cudaError_t launch_closest_checked(const DevScene &S, const Checks &C, const ae_
 cudaError_t launch_count_plain(const DevScene &S, const ae_ray *rays, uint32_t n, unsigned long long *totals,
                                cudaStream_t st);
 cudaError_t launch_count_paths(const DevScene &S, const FrameParams &F, unsigned long long *totals, cudaStream_t st);
-cudaError_t launch_render_plain(const DevScene &S, const FrameParams &F, float4 *accum, uchar4 *display,
+cudaError_t launch_render_plain(const DevScene &S, const ExactView &X, const FrameParams &F, float4 *accum, uchar4 *display,
                                 float4 *frame, cudaStream_t st);
 
 }  // namespace ae

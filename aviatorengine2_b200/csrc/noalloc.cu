@@ -68,7 +68,7 @@ extern "C" int ae_closest_hit_noalloc(ae_ctx *ctx, const ae_ray *rays, uint32_t 
     // entry point only uses them when they are current and were accepted for
     // this scene (the optimised kernels have no participating media).
     if (variant != AE_VARIANT_PLAIN) {
-        if (!(c->fast_ready && c->fast && c->fast->scene_key == c->scene_version))
+        if (!(c->fast_ready && c->fast && c->fast_accepted == c->scene_version && c->fast->scene_key == c->scene_version))
             return c->fail(AE_ERR_STATE, "call ae_prepare_fast (which allocates) before the no-allocation entry point");
         if (c->fast->has_volumes)
             return c->fail(AE_ERR_STATE, "participating media consume RNG in the reference's visit order; use the "

@@ -7,30 +7,36 @@
 
 namespace ae {
 
-// Frame of one axis for child boxes spanning [lo, hi]: quantum 2^e and
-// origin.  250 quanta cover the span, the origin lies 1/32 quantum below it,
-// and the quantum is at least 2^-20 of the coordinates, so that an origin in
-// binary32 and the walk's rounding stay small against it.  False when the
-// span is beyond the exponent range.
+// V(q) of QNode.
+__device__ inline double plane_value(int q) { return q < 128 ? 2.0 + q / 64.0 : 4.0 + (q - 128) / 32.0; }
+
+// Frame of one axis for child boxes spanning [lo, hi]: the smallest scale 2^e
+// whose planes reach from lo to hi, and an origin with plane 0 at or below lo.
+// The scale is at least 2^-20 of the coordinates.  False when the span is
+// beyond the exponent range.
 __device__ inline bool axis_frame(float lo, float hi, int &e, float &org) {
-    const double need = (double(hi) - double(lo)) / 250.0, mag = fmax(fabs(double(lo)), fabs(double(hi)));
+    const double need = (double(hi) - double(lo)) / 5.96875, mag = fmax(fabs(double(lo)), fabs(double(hi)));
     e = -100;
-    if (need > 0.0) e = max(e, ilogb(need) + 1);
+    if (need > 0.0) e = max(e, ilogb(need));
     if (mag > 0.0) e = max(e, ilogb(mag) - 20);
-    org = __double2float_rd(double(lo) - ldexp(1.0, e) / 32.0);
-    return e <= 113 && isfinite(org);
+    for (;; e++) {
+        org = __double2float_rd(double(lo) - 2.0 * ldexp(1.0, e));
+        if (e > 120 || !isfinite(org)) return false;
+        if (double(org) + plane_value(255) * ldexp(1.0, e) >= double(hi)) return true;
+    }
 }
 
-// Planes of [a, b] in the frame (org, 2^e), rounded outward with 1/128 of a
-// quantum to spare: the walk evaluates a plane to within 2^-8 of a quantum
-// (child_hits), so its box always contains [a, b].
+// Planes of [a, b] in the frame (org, 2^e): the nearest ones outside it, or on
+// it where a plane lies there exactly.
 __device__ inline bool axis_planes(float org, int e, float a, float b, uint32_t &qa, uint32_t &qb) {
-    const double inv = ldexp(1.0, -e);
-    const double la = floor((double(a) - double(org)) * inv - 0.0078125);
-    const double lb = ceil((double(b) - double(org)) * inv + 0.0078125);
-    qa = uint32_t(fmin(fmax(la, 0.0), 255.0));
-    qb = uint32_t(fmin(fmax(lb, 0.0), 255.0));
-    return la >= 0.0 && lb <= 255.0;
+    const double s = ldexp(1.0, e), va = (double(a) - double(org)) / s, vb = (double(b) - double(org)) / s;
+    int lo = int(floor(va < 4.0 ? (va - 2.0) * 64.0 : 128.0 + (va - 4.0) * 32.0));
+    int hi = int(ceil(vb <= 4.0 ? (vb - 2.0) * 64.0 : 128.0 + (vb - 4.0) * 32.0));
+    lo = min(max(lo, 0), 255);
+    hi = min(max(hi, 0), 255);
+    qa = uint32_t(lo);
+    qb = uint32_t(hi);
+    return plane_value(lo) <= va && plane_value(hi) >= vb;
 }
 
 // Fills a node's frame and planes from the boxes of its first `n` children
@@ -53,9 +59,9 @@ __device__ inline bool quantise_node(QNode &q, int n, const float (*box)[6], con
         for (int a = 0; a < 3; a++)
             if (valid[k] && good) good = axis_planes(org[a], e[a], box[k][a], box[k][3 + a], pl[k][a], pl[k][3 + a]) && good;
     q.ox = org[0]; q.oy = org[1]; q.oz = org[2];
-    q.scale = uint32_t(n) << 24;
+    q.scale = 0u;
     if (any && good)
-        for (int a = 0; a < 3; a++) q.scale |= uint32_t(e[a] + 141) << (8 * a);
+        for (int a = 0; a < 3; a++) q.scale |= uint32_t(e[a] + 127) << (8 * a);
     for (int k = 0; k < 4; k++) {
         const bool use = k < n && good && valid[k];
         q.plane[k] = use ? make_uint2(pl[k][0] | pl[k][1] << 8 | pl[k][2] << 16 | pl[k][3] << 24,

@@ -70,44 +70,6 @@ AE_DEV void sample_light(const ae_object *L, uint32_t shape, f3 from, f3 &p, flo
     omega = AE_DIV(area, d2);
 }
 
-// CalculateDirectLight, hybrid:1122-1212.
-// T (optional): touch counters of the shadow traversals.
-AE_DEV f3 direct_light(const DevScene &S, const DHit &h, f3 surf_albedo, float time, uint32_t &seed,
-                       Touch *T = nullptr) {
-    f3 acc = splat(0.0f);
-    for (uint32_t i = 0; i < S.n_lights; i++) {
-        const ae_object *L = S.objects + __ldg(S.lights + i);
-        const ObjHead lh = load_head(L);
-        f3 lp;
-        float omega;
-        sample_light(L, lh.shape, h.p, lp, omega, seed);
-        if (omega <= 0.0f) continue;
-        f3 sd = lp - h.p;
-        const float dist = length(sd);
-        if (dist <= 1e-6f) continue;
-        sd = sd / dist;
-        const float ct = dot(h.n, sd);
-        if (ct <= 0.0f) continue;
-        f3 so = h.p + h.n * 0.001f;
-        bool occluded = false;
-        for (int k = 0; k < 4; k++) {
-            DHit sh;
-            if (!traverse_ref(S, so, sd, time, 0.001f, sh, seed, T)) break;
-            if (sh.t >= AE_SUB(distance(lp, so), 0.001f)) break;
-            const uint32_t mt = load_head(S.objects + sh.slot).material;
-            if (mt == AE_MAT_DIFFUSE_LIGHT) break;
-            if (mt != AE_MAT_DIELECTRIC) { occluded = true; break; }
-            so = sh.p + sd * 0.001f;
-        }
-        if (!occluded) {
-            const MatRec lm = load_mat(L);
-            const f3 rad = lm.emission * lm.albedo;
-            acc = acc + surf_albedo * rad * ct * omega;
-        }
-    }
-    return acc;
-}
-
 // Rough metal with GGX microfacet reflection - an extension: the
 // reference's METAL is a mirror blurred by fuzz (hybrid:988-991).  The model
 // is Walter, Marschner, Li and Torrance, "Microfacet Models for Refraction

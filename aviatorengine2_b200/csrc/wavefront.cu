@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "context.h"
+#include "exact_trace.cuh"
 #include "fast.h"
 #include "fast_trace.cuh"
 #include "kernels.h"
@@ -748,7 +749,7 @@ int render_wavefront(Ctx *c, bool prec) {
     if (hp.F.display_only) {
         // Re-grade only: the compute-only kernel's display-only branch.
         if ((rc = c->timed_begin())) return rc;
-        if ((rc = c->cuda(launch_render_plain(c->scene(), hp.F, c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
+        if ((rc = c->cuda(launch_render_plain(c->scene(), ExactView{}, hp.F, c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
                           "display only")))
             return rc;
         return c->timed_end();
