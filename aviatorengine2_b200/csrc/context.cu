@@ -133,6 +133,44 @@ FrameParams make_frame_params(const ae_config &c) {
     return F;
 }
 
+// Host batches travel in chunks over three streams, so the copies of one chunk
+// overlap the tracing of the others.  Chunks ramp 64K -> 512K rays at the start
+// and back down at the end, so the first kernel starts after a short copy and
+// the last copy back is short.
+std::vector<uint32_t> host_chunks(uint32_t n) {
+    constexpr uint32_t kBig = 1u << 19;
+    static const uint32_t kRamp[3] = {1u << 16, 1u << 17, 1u << 18};
+    std::vector<uint32_t> plan;
+    const uint32_t ramp_total = 2 * (kRamp[0] + kRamp[1] + kRamp[2]);
+    if (n <= ramp_total) {
+        const uint32_t parts = std::max(1u, (n + kRamp[1] - 1) / kRamp[1]);
+        for (uint32_t i = 0; i < parts; i++) plan.push_back(n / parts + (i < n % parts ? 1u : 0u));
+    } else {
+        for (uint32_t r : kRamp) plan.push_back(r);
+        for (uint32_t mid = n - ramp_total; mid > 0;) {
+            const uint32_t m = std::min(kBig, mid);
+            plan.push_back(m);
+            mid -= m;
+        }
+        for (int i = 2; i >= 0; i--) plan.push_back(kRamp[i]);
+    }
+    return plan;
+}
+
+// The side streams of a chunked host batch, ordered behind the work already on
+// the context's stream (an upload or a refit that has not been waited for).
+int ensure_side_streams(Ctx *c) {
+    int rc;
+    if (!c->side_stream && (rc = c->cuda(cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking), "stream"))) return rc;
+    if (!c->side_stream2 && (rc = c->cuda(cudaStreamCreateWithFlags(&c->side_stream2, cudaStreamNonBlocking), "stream"))) return rc;
+    if (!c->order && (rc = c->cuda(cudaEventCreateWithFlags(&c->order, cudaEventDisableTiming), "event"))) return rc;
+    if ((rc = c->cuda(cudaEventRecord(c->order, c->stream), "order streams")) ||
+        (rc = c->cuda(cudaStreamWaitEvent(c->side_stream, c->order, 0), "order streams")) ||
+        (rc = c->cuda(cudaStreamWaitEvent(c->side_stream2, c->order, 0), "order streams")))
+        return rc;
+    return AE_OK;
+}
+
 }  // namespace ae
 
 namespace {
@@ -539,35 +577,12 @@ int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, in
             return c->cuda(cudaStreamSynchronize(c->stream), "closest hit");
         }
     }
-    // Host -> device -> host in chunks over three streams, each with its own
-    // staging slot, so the copies of one chunk overlap the tracing of the
-    // others.  Chunks ramp 64K -> 512K rays at the start and back down at the
-    // end, so the first kernel starts after a short copy and the last copy
-    // back is short.
-    constexpr uint32_t kBig = 1u << 19;
-    static const uint32_t kRamp[3] = {1u << 16, 1u << 17, 1u << 18};
-    std::vector<uint32_t> plan;
-    const uint32_t ramp_total = 2 * (kRamp[0] + kRamp[1] + kRamp[2]);
-    if (n <= ramp_total) {
-        const uint32_t parts = std::max(1u, (n + kRamp[1] - 1) / kRamp[1]);
-        for (uint32_t i = 0; i < parts; i++) plan.push_back(n / parts + (i < n % parts ? 1u : 0u));
-    } else {
-        for (uint32_t r : kRamp) plan.push_back(r);
-        for (uint32_t mid = n - ramp_total; mid > 0;) {
-            const uint32_t m = std::min(kBig, mid);
-            plan.push_back(m);
-            mid -= m;
-        }
-        for (int i = 2; i >= 0; i--) plan.push_back(kRamp[i]);
-    }
+    // Host -> device -> host in chunks (host_chunks), each stream with its own
+    // staging slot.
+    const std::vector<uint32_t> plan = host_chunks(n);
     const uint32_t chunk = *std::max_element(plan.begin(), plan.end());
-    if (!c->side_stream) {
-        if ((rc = c->cuda(cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking), "stream"))) return rc;
-    }
-    if (!c->side_stream2) {
-        if ((rc = c->cuda(cudaStreamCreateWithFlags(&c->side_stream2, cudaStreamNonBlocking), "stream"))) return rc;
-    }
-    for (int k = 0; k < Ctx::kIoSlots; k++)
+    if (plan.size() > 1 && (rc = ensure_side_streams(c))) return rc;
+    for (size_t k = 0; k < std::min<size_t>(Ctx::kIoSlots, plan.size()); k++)
         if (c->io_rays[k].reserve(chunk) || c->io_hits[k].reserve(chunk))
             return c->fail(AE_ERR_OOM, "staging allocation failed");
     cudaStream_t st[Ctx::kIoSlots] = {c->stream, c->side_stream, c->side_stream2};
@@ -584,8 +599,9 @@ int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, in
             return rc;
         off += m;
     }
-    if ((rc = c->cuda(cudaStreamSynchronize(c->side_stream2), "closest hit"))) return rc;
-    if ((rc = c->cuda(cudaStreamSynchronize(c->side_stream), "closest hit"))) return rc;
+    if (plan.size() > 1 && ((rc = c->cuda(cudaStreamSynchronize(c->side_stream2), "closest hit")) ||
+                            (rc = c->cuda(cudaStreamSynchronize(c->side_stream), "closest hit"))))
+        return rc;
     return c->cuda(cudaStreamSynchronize(c->stream), "closest hit");
 }
 

@@ -53,6 +53,7 @@ struct Ctx {
     cudaStream_t side_stream = nullptr;
     cudaStream_t side_stream2 = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t order = nullptr;  // side streams behind `stream` (ensure_side_streams)
     std::string err;
     uint64_t launches = 0;
     bool timed = false;
@@ -106,6 +107,8 @@ struct Ctx {
     static constexpr int kIoSlots = 3;
     DevBuf<ae_ray> io_rays[kIoSlots];
     DevBuf<ae_hit> io_hits[kIoSlots];
+    DevBuf<float> io_bound[kIoSlots];    // any-hit batches: far bounds and answers
+    DevBuf<uint8_t> io_blocked[kIoSlots];
 
     // Optimised forms.
     FastScene *fast = nullptr;
@@ -124,6 +127,8 @@ struct Ctx {
 };
 
 // Implemented by the optimised-kernel translation units.
+std::vector<uint32_t> host_chunks(uint32_t n);
+int ensure_side_streams(Ctx *c);
 int prepare_variant(Ctx *c, int variant);
 int closest_hit_dispatch(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, int variant, cudaStream_t st,
                          bool timed);
