@@ -440,12 +440,12 @@ AE_DEV void trace_mesh(const FastView &V, const FastInst &I, uint32_t slot, f3 o
 // meshes by the 4-wide quantised BLAS.  `stk` is this thread's column of the
 // block's shared-memory stack.  T (optional) counts the touches: instance-tree
 // nodes, object metadata records, instance records, wide BLAS nodes, triangle
-// records.
+// records.  tmax: as Walker::start.
 template <bool WT, int SS = kSharedStack>
 AE_DEV Best closest_fast(const DevScene &S, const FastView &V, f3 o, f3 d, float tn, float time, uint2 *stk, int tid,
-                         int nt, Touch *T = nullptr) {
+                         int nt, Touch *T = nullptr, float tmax = kFarStart) {
     Best best;
-    best.t = kFarStart; best.alpha = 0.0f; best.beta = 0.0f;
+    best.t = tmax; best.alpha = 0.0f; best.beta = 0.0f;
     best.object = AE_MISS; best.prim = AE_MISS; best.lrank = 0;
     if (V.troot == kEmptyTlas) return best;
     if (no_direction(d)) {

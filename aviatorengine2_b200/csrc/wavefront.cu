@@ -52,12 +52,13 @@ struct WfParams {
     uint32_t kahan;  // precision form: compensated accumulation
 };
 
-// Device counters: [0],[1] ray queue sizes (ping-pong), [2] shadow queue,
-// [3] error flags, [4..4+kMaxBounce) extend tile counters, then shadow tiles.
+// Device counters, one per bounce, so that the generate stage can clear them
+// all and no launch between the stages has to: the ray queue's size, the
+// shadow queue's size, and the tiles or runs taken from each.  C_ERR: error
+// flags; C_FAULT: the injected tile-wait failure of ae_debug_inject (0 = none).
 constexpr int kMaxBounce = 64;
-// C_FAULT: the injected tile-wait failure of ae_debug_inject (0 = none).
-enum { C_Q0 = 0, C_Q1 = 1, C_SH = 2, C_ERR = 3, C_TILE = 4, C_SHTILE = 4 + kMaxBounce, C_FAULT = 4 + 2 * kMaxBounce,
-       C_COUNT = 5 + 2 * kMaxBounce };
+enum { C_ERR = 0, C_FAULT = 1, C_Q = 2, C_SH = C_Q + kMaxBounce + 1, C_TILE = C_SH + kMaxBounce,
+       C_SHTILE = C_TILE + kMaxBounce, C_COUNT = C_SHTILE + kMaxBounce };
 
 struct WfView {
     ae_ray *qray[2];
@@ -123,10 +124,8 @@ void destroy_wavefront(Ctx *c) {
 __global__ void __launch_bounds__(256) k_wf_generate(WfView W) {
     const WfParams &P = *W.P;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        W.cnt[C_Q0] = P.n_paths;
-        W.cnt[C_Q1] = 0;
-        W.cnt[C_SH] = 0;
-        for (int k = 0; k < 2 * kMaxBounce; k++) W.cnt[C_TILE + k] = 0;
+        W.cnt[C_Q] = P.n_paths;
+        for (int k = C_Q + 1; k < C_COUNT; k++) W.cnt[k] = 0;
     }
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P.n_paths; p += gridDim.x * blockDim.x) {
         const uint32_t x = p % P.F.width, y = p / P.F.width;
@@ -164,7 +163,7 @@ __global__ void __launch_bounds__(THREADS) k_wf_extend(DevScene S, FastView V, W
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tile_index;
     const int q = bounce & 1;
-    const uint32_t count = W.cnt[q];
+    const uint32_t count = W.cnt[C_Q + bounce];
     // An injected failure (ae_debug_inject) issues no copy and waits on the
     // unarmed phase for a few polls: the timeout path runs with nothing in
     // flight.
@@ -226,11 +225,28 @@ __global__ void __launch_bounds__(128, MINB) k_wf_extend_walk(DevScene S, FastVi
                                                                           uint32_t run) {
     extern __shared__ uint2 stk[];
     const int q = bounce & 1;
-    const uint32_t count = W.cnt[q];
+    const uint32_t count = W.cnt[C_Q + bounce];
     const uint32_t warps = gridDim.x * (blockDim.x / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
     const uint32_t stride = warps * lanes;
     uint32_t k = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * lanes + lane;
-    run = min(run, lanes);
+    if (lanes < 32u) {
+        // Few rays, few of them in a warp: one after another, without the
+        // votes that full warps gain from (500 rays: 100 -> 65 us).
+        for (; lane < lanes && k < count; k += stride) {
+            const ae_ray r = W.qray[q][k];
+            const Best b = closest_fast<WT>(S, V, mk(r.ox, r.oy, r.oz), mk(r.dx, r.dy, r.dz), r.tnear, r.time, stk,
+                                            threadIdx.x, 128);
+            const bool any = b.object != AE_MISS;
+            ae_hit h;
+            h.t = any ? b.t : 0.0f;
+            h.alpha = any ? b.alpha : 0.0f;
+            h.beta = any ? b.beta : 0.0f;
+            h.object = b.object;
+            h.prim = b.prim;
+            W.qhit[k] = h;
+        }
+        return;
+    }
     Walker<WT> w;
     WalkStacks<> K;
     bool active = !DYN && lane < lanes && k < count;
@@ -283,7 +299,7 @@ __global__ void __launch_bounds__(256) k_wf_shade(DevScene S, FastView V, WfView
     if (W.cnt[C_ERR]) return;
     const WfParams &P = *W.P;
     const int q = bounce & 1;
-    const uint32_t count = W.cnt[q];
+    const uint32_t count = W.cnt[C_Q + bounce];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const uint32_t pid = W.qpid[q][k];
         const ae_ray r = W.qray[q][k];
@@ -300,12 +316,12 @@ __global__ void __launch_bounds__(256) k_wf_shade(DevScene S, FastView V, WfView
         W.acc[pid] = make_float4(acc.x, acc.y, acc.z, 0.0f);
         W.seed[pid] = seed;
         // Compaction into the next ray queue and the shadow queue.
-        const uint32_t slot = warp_append(&W.cnt[q ^ 1], next ? 1u : 0u);
+        const uint32_t slot = warp_append(&W.cnt[C_Q + bounce + 1], next ? 1u : 0u);
         if (next) {
             W.qray[q ^ 1][slot] = nr;
             W.qpid[q ^ 1][slot] = pid;
         }
-        const uint32_t sbase = warp_append(&W.cnt[C_SH], n_shadow);
+        const uint32_t sbase = warp_append(&W.cnt[C_SH + bounce], n_shadow);
         if (n_shadow) push_shadow_entries(W.sh, pid * P.n_lights, P.n_lights, W.sq, sbase);
     }
 }
@@ -324,11 +340,33 @@ template <int THREADS, bool WT, bool DYN, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB * 128 / THREADS)
     k_wf_shadow(DevScene S, FastView V, WfView W, int bounce, uint32_t run) {
     extern __shared__ uint2 stk[];
-    const uint32_t count = W.cnt[C_SH];
+    const uint32_t count = W.cnt[C_SH + bounce];
     const uint32_t warps = gridDim.x * (THREADS / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
     const uint32_t stride = warps * lanes;
     uint32_t k = (blockIdx.x * (THREADS / 32) + threadIdx.x / 32) * lanes + lane;
-    run = min(run, lanes);
+    if (lanes < 32u) {
+        // Few samples: as k_wf_extend_walk.
+        for (; lane < lanes && k < count; k += stride) {
+            const uint32_t se = W.sq[k];
+            const float4 o4 = W.sh.o[se], d4 = W.sh.d[se], l4 = W.sh.lp[se];
+            f3 so = mk(o4.x, o4.y, o4.z);
+            const f3 sd = mk(d4.x, d4.y, d4.z), lp = mk(l4.x, l4.y, l4.z);
+            int verdict = 0;
+            for (int i = 0; i < 4; i++) {
+                const float bound = AE_SUB(distance(lp, so), 0.001f);
+                const Best b = closest_fast<WT>(S, V, so, sd, 0.001f, d4.w, stk, threadIdx.x, 128, nullptr, bound);
+                verdict = 0;
+                if (b.object == AE_MISS || !(b.t < bound)) break;
+                const uint32_t mt = load_head(S.objects + b.object).material;
+                verdict = mt == AE_MAT_DIFFUSE_LIGHT ? 0 : (mt != AE_MAT_DIELECTRIC ? 1 : 2);
+                if (verdict != 2) break;
+                so = (so + sd * b.t) + sd * 0.001f;
+                verdict = 0;
+            }
+            W.sh.occ[se] = uint8_t(verdict);
+        }
+        return;
+    }
     Walker<WT> w;
     WalkStacks<> K;
     uint32_t e = 0;
@@ -392,7 +430,7 @@ __global__ void __launch_bounds__(THREADS, MINB * 128 / THREADS)
 __global__ void __launch_bounds__(256) k_wf_connect(WfView W, int bounce) {
     const WfParams &P = *W.P;
     const int q = bounce & 1;
-    const uint32_t count = W.cnt[q];
+    const uint32_t count = W.cnt[C_Q + bounce];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const uint32_t pid = W.qpid[q][k];
         if (!W.nee[pid]) continue;
@@ -402,12 +440,6 @@ __global__ void __launch_bounds__(256) k_wf_connect(WfView W, int bounce) {
         const f3 acc = mk(a4.x, a4.y, a4.z) + mk(t4.x, t4.y, t4.z) * dl;
         W.acc[pid] = make_float4(acc.x, acc.y, acc.z, 0.0f);
     }
-}
-
-// The shadow queue of a bounce starts empty; the next ray queue too.
-__global__ void k_wf_reset(WfView W, int bounce) {
-    W.cnt[(bounce & 1) ^ 1] = 0;
-    W.cnt[C_SH] = 0;
 }
 
 // Finish: this sample's path radiance into the pixel's sum; at the last
@@ -616,7 +648,6 @@ static int record_sample(Ctx *c, cudaStream_t st, int cfg_index, const Grids &G,
     const size_t esmem = G.esmem;
     k_wf_generate<<<grid256, 256, 0, st>>>(W);
     for (uint32_t b = 0; b < c->config.depth; b++) {
-        k_wf_reset<<<1, 1, 0, st>>>(W, int(b));
         // Camera rays are coherent: the autotuned tile-staged extend.  Bounce
         // queues are not: the step-wise walk keeps warps full (measured 6 %
         // more paths/s on the 10M-triangle scene).
@@ -631,7 +662,7 @@ static int record_sample(Ctx *c, cudaStream_t st, int cfg_index, const Grids &G,
     return c->cuda(cudaGetLastError(), "wavefront launch");
 }
 
-static uint64_t launches_per_sample(const Ctx *c) { return 2 + 5ull * c->config.depth; }
+static uint64_t launches_per_sample(const Ctx *c) { return 2 + 4ull * c->config.depth; }
 
 // Times every extend configuration on this scene's first bounce and keeps
 // the fastest.
@@ -649,7 +680,6 @@ static int autotune(Ctx *c) {
         float total = 0.0f;
         for (int rep = 0; rep < 2; rep++) {
             k_wf_generate<<<Wf.sms * 8, 256, 0, c->stream>>>(W);
-            k_wf_reset<<<1, 1, 0, c->stream>>>(W, 0);
             cudaEventRecord(c->ev0, c->stream);
             e.fn<<<egrid, e.threads, extend_smem(e.threads, e.stack), c->stream>>>(S, V, W, 0);
             cudaEventRecord(c->ev1, c->stream);
@@ -658,7 +688,7 @@ static int autotune(Ctx *c) {
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, c->ev0, c->ev1);
             if (rep == 1) total = ms;
-            c->launches += 3;
+            c->launches += 2;
         }
         Wf.tune_ms[k] = total;
         if (total < best_ms) { best_ms = total; best = k; }
@@ -694,11 +724,10 @@ static int autotune_walkers(Ctx *c, bool prec) {
     const ExtendCfg &e = kExtendCfgs[prec][ci];
     cudaStream_t st = c->stream;
     k_wf_generate<<<G.grid256, 256, 0, st>>>(W);
-    k_wf_reset<<<1, 1, 0, st>>>(W, 0);
     e.fn<<<G.egrid, e.threads, G.esmem, st>>>(S, V, W, 0);
     if (prec) k_wf_shade<true><<<G.grid256, 256, 0, st>>>(S, V, W, 0);
     else k_wf_shade<false><<<G.grid256, 256, 0, st>>>(S, V, W, 0);
-    c->launches += 4;
+    c->launches += 3;
     int rc = c->cuda(cudaGetLastError(), "autotune");
     if (rc) return rc;
     for (int stage = 0; stage < 2; stage++) {
