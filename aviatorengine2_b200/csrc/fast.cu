@@ -438,12 +438,8 @@ __global__ void k_object_boxes(const uint4 *__restrict__ meta, const FastInst *_
 // children), and its children are re-quantised in the node's new frame.  A
 // child whose box is empty or not finite becomes an unused slot.  Sets *bad
 // when a box cannot be quantised conservatively.
-__global__ void k_instance_tree_level(QNode *__restrict__ nodes, float *__restrict__ nbox,
-                                      const float *__restrict__ obj_box, const int32_t *__restrict__ level,
-                                      int32_t count, uint32_t *bad) {
-    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int32_t ni = level[k];
+__device__ void instance_tree_node(QNode *__restrict__ nodes, float *nbox, const float *__restrict__ obj_box, int32_t ni,
+                                   uint32_t *bad) {
     QNode q = nodes[ni];
     int n = 0;
     while (n < 4 && q.child[n] != kNoChild) n++;
@@ -463,6 +459,33 @@ __global__ void k_instance_tree_level(QNode *__restrict__ nodes, float *__restri
     nodes[ni] = q;
     float *o = nbox + 6 * size_t(ni);
     for (int a = 0; a < 6; a++) o[a] = u[a];
+}
+__global__ void k_instance_tree_level(QNode *nodes, float *nbox, const float *obj_box, const int32_t *level, int32_t count,
+                                      uint32_t *bad) {
+    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < count) instance_tree_node(nodes, nbox, obj_box, level[k], bad);
+}
+// All levels by one block (as k_refit_levels, refit.cu).
+__global__ void __launch_bounds__(256) k_instance_tree_levels(QNode *nodes, float *nbox, const float *obj_box,
+                                                              const int32_t *order, const int32_t *start, int32_t levels,
+                                                              uint32_t *bad) {
+    for (int32_t l = 0; l < levels; l++) {
+        for (int32_t k = start[l] + int32_t(threadIdx.x); k < start[l + 1]; k += int32_t(blockDim.x))
+            instance_tree_node(nodes, nbox, obj_box, order[k], bad);
+        __syncthreads();
+    }
+}
+
+// Instance records after a refit: the transforms of the uploaded instances.
+__global__ void k_move_instances(FastInst *__restrict__ inst, const ae_instance *__restrict__ from, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const ae_instance m = from[i];
+    FastInst f = inst[i];
+    f.px = m.px; f.py = m.py; f.pz = m.pz; f.scale = m.scale;
+    f.qx = m.qx; f.qy = m.qy; f.qz = m.qz; f.qw = m.qw;
+    f.inv_scale = m.scale != 0.0f && m.scale != 1.0f ? AE_DIV(1.0f, m.scale) : 1.0f;
+    inst[i] = f;
 }
 
 // Per object, the intersection of the reference TLAS boxes above it, leaf to
@@ -565,7 +588,8 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
     }
     const size_t nn = std::max<size_t>(out.size(), 1);
     if (F.tnodes.reserve(nn) || F.tbox.reserve(nn * 6) || F.tlevels.reserve(std::max<size_t>(order.size(), 1)) ||
-        F.obj_box.reserve(size_t(n) * 6) || F.static_box.reserve(size_t(n) * 6) || F.tflag.reserve(1))
+        F.obj_box.reserve(size_t(n) * 6) || F.static_box.reserve(size_t(n) * 6) || F.tflag.reserve(1) ||
+        F.tlevel_start_dev.reserve(F.tlevel_start.size()))
         return c->fail(AE_ERR_OOM, "instance tree");
     int rc;
     // Links and child counts; the refresh writes frames and planes.
@@ -580,6 +604,8 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
         ((rc = c->cuda(cudaMemcpyAsync(F.tnodes.ptr, dev.data(), dev.size() * sizeof(QNode), cudaMemcpyHostToDevice,
                                        c->stream), "upload instance tree")) ||
          (rc = c->cuda(cudaMemcpyAsync(F.tlevels.ptr, order.data(), order.size() * sizeof(int32_t),
+                                       cudaMemcpyHostToDevice, c->stream), "upload instance tree levels")) ||
+         (rc = c->cuda(cudaMemcpyAsync(F.tlevel_start_dev.ptr, F.tlevel_start.data(), F.tlevel_start.size() * sizeof(int32_t),
                                        cudaMemcpyHostToDevice, c->stream), "upload instance tree levels"))))
         return rc;
     if ((rc = c->cuda(cudaMemcpyAsync(F.static_box.ptr, stat.data(), stat.size() * sizeof(float), cudaMemcpyHostToDevice,
@@ -601,9 +627,9 @@ static int refresh_instance_tree(Ctx *c, FastScene &F) {
         const ae_object &o = c->host_objects[s];
         if (o.shapeType == AE_SHAPE_MESH) {
             const ae_instance &m = c->host_instances[o.instanceIndex];
-            const FastScene::MeshSub &ms = F.mesh_sub.at(std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase));
             const float sc = (m.scale != 0.0f && m.scale != 1.0f) ? std::fabs(m.scale) : 1.0f;
-            const float r = std::max(std::fabs(m.px), std::max(std::fabs(m.py), std::fabs(m.pz))) + 1.75f * sc * ms.radius;
+            const float r = std::max(std::fabs(m.px), std::max(std::fabs(m.py), std::fabs(m.pz))) +
+                            1.75f * sc * F.inst_radius[o.instanceIndex];
             range = std::max(range, r);
         }
     }
@@ -619,7 +645,12 @@ static int refresh_instance_tree(Ctx *c, FastScene &F) {
     if ((rc = c->cuda(cudaMemsetAsync(F.tflag.ptr, 0, sizeof(uint32_t), c->stream), "instance tree flag"))) return rc;
     k_object_boxes<<<(n * 32 + 255) / 256, 256, 0, c->stream>>>(F.obj_meta.ptr, F.inst.ptr, F.sub_boxes.ptr, F.sub_refs.ptr,
                                                                  F.static_box.ptr, n, margin, F.obj_box.ptr);
-    for (size_t l = 0; l + 1 < F.tlevel_start.size(); l++) {
+    const bool one_block = F.n_tnodes <= 1024;
+    if (one_block)
+        k_instance_tree_levels<<<1, 256, 0, c->stream>>>(F.tnodes.ptr, F.tbox.ptr, F.obj_box.ptr, F.tlevels.ptr,
+                                                         F.tlevel_start_dev.ptr, int32_t(F.tlevel_start.size()) - 1,
+                                                         F.tflag.ptr);
+    for (size_t l = 0; !one_block && l + 1 < F.tlevel_start.size(); l++) {
         const int32_t cnt = F.tlevel_start[l + 1] - F.tlevel_start[l];
         if (cnt <= 0) continue;
         k_instance_tree_level<<<(cnt + 127) / 128, 128, 0, c->stream>>>(F.tnodes.ptr, F.tbox.ptr, F.obj_box.ptr,
@@ -719,9 +750,14 @@ int prepare_fast(Ctx *c) {
         F.geometry_key = c->geometry_version;
         F.geometry_dirty = true;
     }
+    // Only transforms moved since the last build (ae_refit_instances keeps the
+    // meshes and the layout): the records are on the device already, and their
+    // transforms come from the instances that the refit uploaded.
+    const bool moved = !F.geometry_dirty && F.tlas_key == c->scene_version_layout && F.sub_key == c->geometry_version &&
+                       F.inst_radius.size() == c->n_instances;
     // Geometry-derived part: rebuilt when new meshes appear.
     bool rebuilt = false;
-    for (uint32_t i = 0; i < c->n_instances; i++) {
+    for (uint32_t i = 0; !moved && i < c->n_instances; i++) {
         const ae_instance &m = c->host_instances[i];
         const auto key = std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase);
         if (F.mesh_roots.count(key)) continue;
@@ -759,7 +795,10 @@ int prepare_fast(Ctx *c) {
         F.geometry_dirty = false;
     }
     // Scene-derived part: instances and object metadata, per upload.
-    if (F.scene_key != c->scene_version || rebuilt) {
+    if (moved && F.scene_key != c->scene_version && c->n_instances)
+        k_move_instances<<<(c->n_instances + 127) / 128, 128, 0, c->stream>>>(F.inst.ptr, c->instances.ptr, c->n_instances);
+    if (!moved && (F.scene_key != c->scene_version || rebuilt)) {
+        F.inst_radius.assign(c->n_instances, 0.0f);
         std::vector<FastInst> fi(std::max<uint32_t>(c->n_instances, 1));
         for (uint32_t i = 0; i < c->n_instances; i++) {
             const ae_instance &m = c->host_instances[i];
@@ -772,6 +811,7 @@ int prepare_fast(Ctx *c) {
             const FastScene::MeshSub &ms = F.mesh_sub.at(std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase));
             f.inv_scale = m.scale != 0.0f && m.scale != 1.0f ? 1.0f / m.scale : 1.0f;
             f.sub = ms.index;
+            F.inst_radius[i] = ms.radius;
         }
         // Each object's rank comes from the reference TLAS leaf that holds it.
         std::vector<uint32_t> leaf_first_of(std::max<uint32_t>(c->n_objects, 1), 0u);
@@ -821,6 +861,8 @@ int prepare_fast(Ctx *c) {
             F.tlas_key = c->scene_version_layout;
             F.sub_key = c->geometry_version;
         }
+    }
+    if (F.scene_key != c->scene_version || rebuilt) {
         if ((rc = refresh_instance_tree(c, F))) return rc;
         if ((rc = c->cuda(cudaStreamSynchronize(c->stream), "prepare fast"))) return rc;
         if (F.n_tnodes) {

@@ -119,6 +119,8 @@ struct FastScene {
     DevBuf<int32_t> tlevels;      // tree nodes by depth, deepest first
     DevBuf<uint32_t> tflag;       // set by the refresh when a box cannot be quantised
     std::vector<int32_t> tlevel_start;
+    DevBuf<int32_t> tlevel_start_dev;
+    std::vector<float> inst_radius;  // per instance: its mesh's largest local coordinate
     uint32_t troot = kEmptyTlas, n_tnodes = 0;
     // What the exact walks need beyond (exact_trace.cuh): the triangles' shape
     // factor A, the largest mesh-space coordinate, and per object the

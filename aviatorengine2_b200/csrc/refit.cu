@@ -34,6 +34,7 @@ struct Refit {
     DevBuf<float> local_bounds;   // 6 floats per instance: its mesh's local box
     DevBuf<int32_t> level_nodes;  // TLAS node ids grouped by depth, deepest first
     std::vector<int32_t> level_start;
+    DevBuf<int32_t> level_start_dev;
     uint64_t topology_version = ~0ull;
     std::map<std::tuple<uint32_t, uint32_t, uint32_t>, ae_aabb> mesh_box;  // (vertexBase, indexBase, tris)
 };
@@ -43,9 +44,10 @@ void destroy_refit(Ctx *c) {
     c->refit = nullptr;
 }
 
-// One thread per object: mesh objects get a new world box and transform.
+// One thread per object: mesh objects get a new world box and transform, and
+// keep the replaced one as the previous transform.
 __global__ void k_refit_objects(ae_object *objects, uint32_t n_objects, const ae_instance *inst,
-                                const float *local_bounds, float *obj_box) {
+                                const ae_instance *old_inst, const float *local_bounds, float *obj_box) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_objects) return;
     ae_object &o = objects[s];
@@ -70,19 +72,11 @@ __global__ void k_refit_objects(ae_object *objects, uint32_t n_objects, const ae
     // scene/shapes.h:176-183: the vector part with w made non-negative).
     o.x2 = o.x; o.y2 = o.y; o.z2 = o.z;
     o.x = I.px; o.y = I.py; o.z = I.pz;
-}
-
-// Previous rotation from the instance record being replaced.
-__global__ void k_refit_prev_rotation(ae_object *objects, uint32_t n_objects, const ae_instance *old_inst) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_objects) return;
-    ae_object &o = objects[s];
-    if (o.shapeType != AE_SHAPE_MESH) return;
-    const ae_instance I = old_inst[o.instanceIndex];
-    const bool neg = I.qw < 0.0f;
-    o.prevRotX = neg ? -I.qx : I.qx;
-    o.prevRotY = neg ? -I.qy : I.qy;
-    o.prevRotZ = neg ? -I.qz : I.qz;
+    const ae_instance P = old_inst[o.instanceIndex];
+    const bool neg = P.qw < 0.0f;
+    o.prevRotX = neg ? -P.qx : P.qx;
+    o.prevRotY = neg ? -P.qy : P.qy;
+    o.prevRotZ = neg ? -P.qz : P.qz;
 }
 
 // Non-mesh objects keep their stored world box; computed once per topology
@@ -95,12 +89,8 @@ __device__ __forceinline__ void widen(float &lo, float &hi) {
     }
 }
 
-// One level of the bottom-up pass; nodes of a level are independent.
-__global__ void k_refit_level(ae_bvh_node *nodes, float *raw, const float *obj_box, const int32_t *level,
-                              int32_t count) {
-    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int32_t ni = level[k];
+// One node of the bottom-up pass; nodes of a level are independent.
+__device__ void refit_node(ae_bvh_node *nodes, float *raw, const float *obj_box, int32_t ni) {
     ae_bvh_node &n = nodes[ni];
     float b[6];
     if (n.count > 0) {
@@ -120,6 +110,22 @@ __global__ void k_refit_level(ae_bvh_node *nodes, float *raw, const float *obj_b
     for (int a = 0; a < 3; a++) widen(lo[a], hi[a]);
     n.min_x = lo[0]; n.min_y = lo[1]; n.min_z = lo[2];
     n.max_x = hi[0]; n.max_y = hi[1]; n.max_z = hi[2];
+}
+__global__ void k_refit_level(ae_bvh_node *nodes, float *raw, const float *obj_box, const int32_t *level,
+                              int32_t count) {
+    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < count) refit_node(nodes, raw, obj_box, level[k]);
+}
+// All levels, deepest first, by one block: a small tree's levels are shorter
+// than the gaps between their launches (516 objects: 11 launches, 38 us -> 1,
+// 14 us).
+__global__ void __launch_bounds__(1024) k_refit_levels(ae_bvh_node *nodes, float *raw, const float *obj_box,
+                                                       const int32_t *order, const int32_t *start, int32_t levels) {
+    for (int32_t l = 0; l < levels; l++) {
+        for (int32_t k = start[l] + int32_t(threadIdx.x); k < start[l + 1]; k += int32_t(blockDim.x))
+            refit_node(nodes, raw, obj_box, order[k]);
+        __syncthreads();
+    }
 }
 
 }  // namespace ae
@@ -214,13 +220,16 @@ extern "C" int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uin
             std::memcpy(&ob[6 * s], &b, 24);
         }
         if (R.raw.reserve(size_t(std::max(nn, 1u)) * 6) || R.local_bounds.reserve(lb.size()) ||
-            R.level_nodes.reserve(std::max<size_t>(order.size(), 1)) || R.inst_in.reserve(std::max(n, 1u)) ||
+            R.level_nodes.reserve(std::max<size_t>(order.size(), 1)) ||
+            R.level_start_dev.reserve(R.level_start.size()) || R.inst_in.reserve(std::max(n, 1u)) ||
             c->obj_box.reserve(ob.size()))
             return c->fail(AE_ERR_OOM, "refit buffers");
         if ((rc = c->cuda(cudaMemcpyAsync(R.local_bounds.ptr, lb.data(), lb.size() * 4, cudaMemcpyHostToDevice, c->stream),
                           "upload")) ||
             (rc = c->cuda(cudaMemcpyAsync(R.level_nodes.ptr, order.data(), order.size() * 4, cudaMemcpyHostToDevice,
                                           c->stream), "upload")) ||
+            (rc = c->cuda(cudaMemcpyAsync(R.level_start_dev.ptr, R.level_start.data(), R.level_start.size() * 4,
+                                          cudaMemcpyHostToDevice, c->stream), "upload")) ||
             (rc = c->cuda(cudaMemcpyAsync(c->obj_box.ptr, ob.data(), ob.size() * 4, cudaMemcpyHostToDevice, c->stream),
                           "upload")))
             return rc;
@@ -232,14 +241,20 @@ extern "C" int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uin
         return rc;
     if ((rc = c->timed_begin())) return rc;
     const int T = 256;
-    // Previous rotation from the instance buffer before it is replaced.
-    k_refit_prev_rotation<<<(no + T - 1) / T, T, 0, c->stream>>>(c->objects.ptr, no, c->instances.ptr);
-    k_refit_objects<<<(no + T - 1) / T, T, 0, c->stream>>>(c->objects.ptr, no, R.inst_in.ptr, R.local_bounds.ptr,
-                                                          c->obj_box.ptr);
+    k_refit_objects<<<(no + T - 1) / T, T, 0, c->stream>>>(c->objects.ptr, no, R.inst_in.ptr, c->instances.ptr,
+                                                          R.local_bounds.ptr, c->obj_box.ptr);
     if ((rc = c->cuda(cudaMemcpyAsync(c->instances.ptr, R.inst_in.ptr, size_t(n) * sizeof(ae_instance),
                                       cudaMemcpyDeviceToDevice, c->stream), "instances")))
         return rc;
-    for (size_t l = 0; l + 1 < R.level_start.size(); l++) {
+    // One block reaches about 200 nodes a microsecond and a launch costs three:
+    // from a few thousand nodes on, a level is worth its own launch.
+    const bool one_block = nn <= 8192;
+    if (one_block) {
+        k_refit_levels<<<1, 1024, 0, c->stream>>>(c->tlas.ptr, R.raw.ptr, c->obj_box.ptr, R.level_nodes.ptr,
+                                                  R.level_start_dev.ptr, int32_t(R.level_start.size()) - 1);
+        c->launches++;
+    }
+    for (size_t l = 0; !one_block && l + 1 < R.level_start.size(); l++) {
         const int32_t cnt = R.level_start[l + 1] - R.level_start[l];
         if (cnt <= 0) continue;
         k_refit_level<<<(cnt + T - 1) / T, T, 0, c->stream>>>(c->tlas.ptr, R.raw.ptr, c->obj_box.ptr,

@@ -92,8 +92,9 @@ struct Wavefront {
     DevBuf<WfParams> params;
     DevBuf<float4> ksum, kcomp;
     WfParams *host_params = nullptr;  // pinned
+    bool params_busy = false;         // a copy out of it may still be pending
     cudaGraphExec_t graph = nullptr;
-    uint64_t graph_key = ~0ull;
+    std::vector<uint64_t> graph_key;  // everything the captured launches hold (graph_key_of)
     int sms = 148;
     // autotuned extend configuration
     int ext_threads = 128, ext_stack = 24;
@@ -662,6 +663,23 @@ static int record_sample(Ctx *c, cudaStream_t st, int cfg_index, const Grids &G,
     return c->cuda(cudaGetLastError(), "wavefront launch");
 }
 
+// Every argument and launch shape that record_sample bakes into the graph.
+static std::vector<uint64_t> graph_key_of(Ctx *c, bool prec, int cfg_index) {
+    const Wavefront &Wf = *c->wave;
+    const DevScene S = c->scene();
+    const FastView V = fast_view(*c->fast);
+    const WfView W = view_of(c);
+    auto p = [](const void *x) { return uint64_t(reinterpret_cast<uintptr_t>(x)); };
+    return {p(S.objects), p(S.tlas), p(S.lights), p(S.vertices), p(S.indices), p(S.blas), p(S.instances), S.n_objects,
+            S.n_nodes, S.n_lights, S.n_instances, p(S.tex), p(S.srgb), S.tex_w, S.tex_h, S.tex_layers,
+            p(V.nodes), p(V.tris), p(V.inst), p(V.meta), p(V.tnodes), V.troot, V.nan_ref.x, V.nan_ref.y, V.nan_wt.x, V.nan_wt.y,
+            p(W.qray[0]), p(W.qray[1]), p(W.qpid[0]), p(W.qpid[1]), p(W.qhit), p(W.thr), p(W.acc), p(W.col), p(W.pend),
+            p(W.seed), p(W.nee), p(W.sh.o), p(W.sh.d), p(W.sh.lp), p(W.sh.c), p(W.sh.valid), p(W.sh.occ), p(W.sq), p(W.cnt),
+            p(W.P), p(W.accum), p(W.frame), p(W.display), p(W.ksum), p(W.kcomp), p(W.prec.shade16),
+            uint64_t(prec), c->config.depth, uint64_t(cfg_index), Wf.shadow_run[prec], Wf.walk_run[prec],
+            uint64_t(Wf.shadow_mb[prec]), uint64_t(Wf.walk_mb[prec]), uint64_t(Wf.sms)};
+}
+
 static uint64_t launches_per_sample(const Ctx *c) { return 2 + 4ull * c->config.depth; }
 
 // Times every extend configuration on this scene's first bounce and keeps
@@ -785,6 +803,7 @@ int render_wavefront(Ctx *c, bool prec) {
     }
     if (!Wf.tuned || !Wf.walk_tuned[prec]) {
         if ((rc = c->cuda(cudaStreamSynchronize(c->stream), "params"))) return rc;
+        Wf.params_busy = true;
         *Wf.host_params = hp;
         if ((rc = c->cuda(cudaMemcpyAsync(Wf.params.ptr, Wf.host_params, sizeof(WfParams), cudaMemcpyHostToDevice,
                                           c->stream), "params")))
@@ -792,10 +811,10 @@ int render_wavefront(Ctx *c, bool prec) {
         if (!Wf.tuned && (rc = autotune(c))) return rc;
         if (!Wf.walk_tuned[prec] && (rc = autotune_walkers(c, prec))) return rc;
     }
-    // One graph per (scene upload, frame shape); frame parameters travel
-    // through device memory so the graph is replayed unchanged.
-    const uint64_t key = (c->scene_version << 21) ^ (uint64_t(prec) << 20) ^ (uint64_t(c->config.depth) << 8) ^
-                         hp.n_lights;
+    // The captured graph is replayed while its launches' arguments and shapes
+    // stay the same (a refit changes neither); frame parameters travel through
+    // device memory.
+    std::vector<uint64_t> key = graph_key_of(c, prec, best_cfg_index(Wf));
     if (!Wf.graph || Wf.graph_key != key) {
         if (Wf.graph) { cudaGraphExecDestroy(Wf.graph); Wf.graph = nullptr; }
         cudaGraph_t g;
@@ -809,19 +828,21 @@ int render_wavefront(Ctx *c, bool prec) {
         ce = cudaGraphInstantiate(&Wf.graph, g, 0);
         cudaGraphDestroy(g);
         if ((rc = c->cuda(ce, "graph instantiate"))) return rc;
-        Wf.graph_key = key;
+        Wf.graph_key.swap(key);
     }
     // The error word counts this frame only; the fault word carries an
     // injected failure (ae_debug_inject) into the extend kernels.
-    if ((rc = c->cuda(cudaMemsetAsync(Wf.cnt.ptr + C_ERR, 0, sizeof(uint32_t), c->stream), "reset error word")) ||
-        (rc = c->cuda(cudaMemsetAsync(Wf.cnt.ptr + C_FAULT, c->fault_tile_wait ? 0xff : 0, sizeof(uint32_t),
-                                      c->stream), "fault word")))
+    static_assert(C_FAULT == C_ERR + 1, "cleared together");
+    if ((rc = c->cuda(cudaMemsetAsync(Wf.cnt.ptr + C_ERR, 0, 2 * sizeof(uint32_t), c->stream), "reset error word")) ||
+        (c->fault_tile_wait &&
+         (rc = c->cuda(cudaMemsetAsync(Wf.cnt.ptr + C_FAULT, 0xff, sizeof(uint32_t), c->stream), "fault word"))))
         return rc;
     if ((rc = c->timed_begin())) return rc;
     for (uint32_t s = 0; s < hp.spp; s++) {
         hp.sample = s;
         // The pinned block is rewritten only after the previous copy finished.
-        if ((rc = c->cuda(cudaStreamSynchronize(c->stream), "params"))) return rc;
+        if (Wf.params_busy && (rc = c->cuda(cudaStreamSynchronize(c->stream), "params"))) return rc;
+        Wf.params_busy = true;
         *Wf.host_params = hp;
         if ((rc = c->cuda(cudaMemcpyAsync(Wf.params.ptr, Wf.host_params, sizeof(WfParams), cudaMemcpyHostToDevice,
                                           c->stream), "params")))
@@ -837,6 +858,7 @@ int render_wavefront(Ctx *c, bool prec) {
                       "read error word")) ||
         (rc = c->cuda(cudaStreamSynchronize(c->stream), "frame")))
         return rc;
+    Wf.params_busy = false;
     if (e) return c->fail(AE_ERR_TIMEOUT, "a bounded queue-tile wait gave up on the device; the frame is incomplete");
     return AE_OK;
 }
