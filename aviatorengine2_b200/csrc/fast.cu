@@ -60,6 +60,7 @@ namespace {
 struct Box {
     float lo[3], hi[3];
 };
+static_assert(sizeof(Box) == 24, "the device's boxes");
 Box node_box(const ae_bvh_node &n) { return Box{{n.min_x, n.min_y, n.min_z}, {n.max_x, n.max_y, n.max_z}}; }
 float half_area(const Box &b) {
     const float dx = b.hi[0] - b.lo[0], dy = b.hi[1] - b.lo[1], dz = b.hi[2] - b.lo[2];
@@ -196,28 +197,6 @@ uint32_t mesh_sub_boxes(const ae_bvh_node *bin, std::vector<float> &out) {
         out.insert(out.end(), b, b + 6);
     }
     return uint32_t(level.size());
-}
-
-// World box of a mesh instance from its sub-boxes (double precision; the
-// device refresh computes the conservative version of the same bound).
-Box instance_box_host(const ae_instance &m, const float *sub, uint32_t count) {
-    const double s = (m.scale != 0.0f && m.scale != 1.0f) ? double(m.scale) : 1.0;
-    const double qx = m.qx, qy = m.qy, qz = m.qz, qw = m.qw;
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (uint32_t b = 0; b < count; b++) {
-        const float *x = sub + 6 * size_t(b);
-        for (int k = 0; k < 8; k++) {
-            const double v[3] = {(k & 1 ? x[3] : x[0]) * s, (k & 2 ? x[4] : x[1]) * s, (k & 4 ? x[5] : x[2]) * s};
-            const double t[3] = {2 * (qy * v[2] - qz * v[1]), 2 * (qz * v[0] - qx * v[2]), 2 * (qx * v[1] - qy * v[0])};
-            const double w[3] = {v[0] + qw * t[0] + (qy * t[2] - qz * t[1]) + m.px,
-                                 v[1] + qw * t[1] + (qz * t[0] - qx * t[2]) + m.py,
-                                 v[2] + qw * t[2] + (qx * t[1] - qy * t[0]) + m.pz};
-            for (int a = 0; a < 3; a++) { lo[a] = std::min(lo[a], w[a]); hi[a] = std::max(hi[a], w[a]); }
-        }
-    }
-    Box r;
-    for (int a = 0; a < 3; a++) { r.lo[a] = float(lo[a]); r.hi[a] = float(hi[a]); }
-    return r;
 }
 
 // Binary tree over object boxes with one object per leaf, in ae_bvh_node
@@ -519,14 +498,24 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
     F.static_range = 0.0f;
     if (n == 0) return AE_OK;
     if (n >= kMaxLeafFirst) return c->fail(AE_ERR_LAYOUT, "%u objects: the instance tree addresses at most %u", n, kMaxLeafFirst);
+    // Mesh objects' boxes by the refresh kernel (no margin): 256 sub-boxes of
+    // eight corners an instance took the host 20 us each.
+    if (F.obj_box.reserve(size_t(n) * 6) || F.static_box.reserve(size_t(n) * 6)) return c->fail(AE_ERR_OOM, "instance tree");
+    k_object_boxes<<<(n * 32 + 255) / 256, 256, 0, c->stream>>>(F.obj_meta.ptr, F.inst.ptr, F.sub_boxes.ptr, F.sub_refs.ptr,
+                                                                 F.static_box.ptr, n, 0.0f, F.obj_box.ptr);
+    std::vector<float> world(size_t(n) * 6);
+    int rc;
+    if ((rc = c->cuda(cudaGetLastError(), "object boxes")) ||
+        (rc = c->cuda(cudaMemcpyAsync(world.data(), F.obj_box.ptr, world.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                      c->stream), "object boxes")) ||
+        (rc = c->cuda(cudaStreamSynchronize(c->stream), "object boxes")))
+        return rc;
     std::vector<Box> boxes(n);
     std::vector<float> stat(size_t(n) * 6, 0.0f);
     for (uint32_t s = 0; s < n; s++) {
         const ae_object &o = c->host_objects[s];
         if (o.shapeType == AE_SHAPE_MESH) {
-            const ae_instance &m = c->host_instances[o.instanceIndex];
-            const FastScene::MeshSub &ms = F.mesh_sub.at(std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase));
-            boxes[s] = instance_box_host(m, F.host_sub.data() + 6 * size_t(ms.first), ms.count);
+            std::memcpy(&boxes[s], &world[6 * size_t(s)], 24);
         } else {
             const ae_aabb b = analytic_box(o);
             boxes[s] = Box{{b.min_x, b.min_y, b.min_z}, {b.max_x, b.max_y, b.max_z}};
@@ -588,10 +577,9 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
     }
     const size_t nn = std::max<size_t>(out.size(), 1);
     if (F.tnodes.reserve(nn) || F.tbox.reserve(nn * 6) || F.tlevels.reserve(std::max<size_t>(order.size(), 1)) ||
-        F.obj_box.reserve(size_t(n) * 6) || F.static_box.reserve(size_t(n) * 6) || F.tflag.reserve(1) ||
+        F.tflag.reserve(1) ||
         F.tlevel_start_dev.reserve(F.tlevel_start.size()))
         return c->fail(AE_ERR_OOM, "instance tree");
-    int rc;
     // Links and child counts; the refresh writes frames and planes.
     std::vector<QNode> dev(out.size(), QNode{});
     for (size_t i = 0; i < out.size(); i++) {
