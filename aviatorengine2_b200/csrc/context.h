@@ -107,6 +107,8 @@ struct Ctx {
     static constexpr int kIoSlots = 3;
     DevBuf<ae_ray> io_rays[kIoSlots];
     DevBuf<ae_hit> io_hits[kIoSlots];
+    static constexpr uint32_t kSmallRays = 4096;
+    void *small_io = nullptr;            // page-locked: kSmallRays rays, then their hits
     DevBuf<float> io_bound[kIoSlots];    // any-hit batches: far bounds and answers
     DevBuf<uint8_t> io_blocked[kIoSlots];
 

@@ -13,6 +13,7 @@ Ctx::~Ctx() {
     destroy_refit(this);
     if (side_stream) cudaStreamDestroy(side_stream);
     if (side_stream2) cudaStreamDestroy(side_stream2);
+    if (small_io) cudaFreeHost(small_io);
     if (order) cudaEventDestroy(order);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);

@@ -27,7 +27,7 @@ def traced():
     ctx.close()
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 129, 2072, 2073, 2368, 2369, 4737, 33152, 33153, 37888, 37889, 60000])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 129, 2072, 2073, 2368, 2369, 4096, 4097, 4737, 33152, 33153, 37888, 37889, 60000])
 def test_small_batches(traced, n):
     ctx, rays, want = traced
     for v, w in ((_lib.VARIANT_FAST, _lib.VARIANT_PLAIN), (_lib.VARIANT_FAST_WALK, _lib.VARIANT_PLAIN),
