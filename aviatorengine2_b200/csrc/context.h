@@ -115,6 +115,10 @@ struct Ctx {
     // Optimised forms.
     FastScene *fast = nullptr;
     bool fast_ready = false;
+    // exact_view: rays traced without structures since the scene or the geometry
+    // changed, and the scene that they could not be built for.
+    uint64_t plain_scene = ~0ull, plain_geometry = ~0ull, plain_scene_rays = 0, plain_geometry_rays = 0;
+    uint64_t exact_refused = ~0ull;
     uint64_t fast_accepted = ~0ull;  // scene_version that prepare_fast last accepted
     Wavefront *wave = nullptr;
     Deferred *deferred = nullptr;

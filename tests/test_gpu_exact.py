@@ -1,9 +1,6 @@
 """The plain forms' traversals on the optimised structures (compute-only
 frames, G-buffer, deferred resolve, any hit) against the reference walks they
 stand for: bit for bit, tolerance zero.  The same call takes either path by a
-rule on sizes: a context without prepared structures answers batches of fewer
-than 256 rays an object with the reference walk, and a prepared one does not.
-Scenes with coincident surfaces, shared edges under rays aimed at vertices and
 edges, axis-parallel rays, grazing rays, thin triangles, scaled and mirrored
 looks from far outside, analytic shapes, textures and refits."""
 import numpy as np
@@ -88,17 +85,27 @@ def test_rays(s, n, seed):
 test_rays.__test__ = False
 
 
+def both_any_hits(s, rays, tmax):
+    """(exact walk, reference walk): a prepared context, and contexts that are
+    asked too little to prepare."""
+    with Context(96, 64) as ctx:
+        ctx.upload(s)
+        ctx.prepare_fast()
+        got = ctx.any_hit(rays, tmax)
+    want = []
+    for k in range(0, len(rays), 150_000):
+        with Context(96, 64) as ctx:
+            ctx.upload(s)
+            want.append(ctx.any_hit(rays[k:k + 150_000], tmax[k:k + 150_000]))
+    return got, np.concatenate(want)
+
+
 @pytest.mark.parametrize("scene", [field, boxes])
 def test_any_hit(scene):
     s = scene()
     n = 400_000
     rays, tmax = test_rays(s, n, 5)
-    with Context(96, 64) as plain, Context(96, 64) as ctx:
-        plain.upload(s)
-        ctx.upload(s)
-        got = ctx.any_hit(rays, tmax)
-        part = 200 * len(s.objects)
-        want = np.concatenate([plain.any_hit(rays[k:k + part], tmax[k:k + part]) for k in range(0, n, part)])
+    got, want = both_any_hits(s, rays, tmax)
     assert np.array_equal(got, want)
     assert 0.05 < want.mean() < 0.99
 
@@ -115,12 +122,7 @@ def test_any_hit_of_odd_rays():
         rays[f][pick] = rng.choice(odd, pick.sum())
     pick = rng.random(n) < 0.1
     tmax[pick] = rng.choice(odd, pick.sum())
-    with Context(96, 64) as plain, Context(96, 64) as ctx:
-        plain.upload(s)
-        ctx.upload(s)
-        got = ctx.any_hit(rays, tmax)
-        part = 200 * len(s.objects)
-        want = np.concatenate([plain.any_hit(rays[k:k + part], tmax[k:k + part]) for k in range(0, n, part)])
+    got, want = both_any_hits(s, rays, tmax)
     assert np.array_equal(got, want)
 
 
