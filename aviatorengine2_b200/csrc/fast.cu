@@ -4,17 +4,18 @@
 //   * per distinct mesh, a 4-wide BVH collapsed from the reference's binary
 //     BLAS (scene/bvh.h).  Collapsing only merges interior nodes, so every
 //     leaf - and therefore every triangle slot - is the reference's.  A node
-//     is 64 bytes: the node box origin, one power-of-two scale per axis and
-//     four child boxes quantised to 8 bits, rounded outward so a decoded box
-//     always contains the exact one (no hit can be lost);
+//     is 64 bytes: a frame (origin, one power-of-two scale per axis) and four
+//     child boxes quantised to 8 bits, rounded outward so a decoded box always
+//     contains the exact one (no hit can be lost); built on the device
+//     (fast_build.cu, quantise.cuh);
 //   * triangles in leaf-slot order as 48-byte records {p0, p1, p2}: one
 //     contiguous read per leaf instead of an index fetch plus three vertex
 //     fetches;
 //   * per instance a 48-byte record with the transform and the mesh's node
 //     and triangle bases.
 //
-// Traversal is nearest-child-first with the far children on a shared-memory
-// stack that also stores each entry's entry distance, so a popped subtree
+// Traversal is nearest-child-first with the far children on one stack for
+// both trees (its first entries in shared memory) that also stores each entry's entry distance, so a popped subtree
 // farther than the current hit is skipped without touching its node.
 //
 // Equal distances: the reference's depth-first walk (hybrid:862-917,
@@ -43,6 +44,7 @@
 
 #include "context.h"
 #include "exact_trace.cuh"
+#include "quad_walk.cuh"
 #include "fast.h"
 #include "fast_trace.cuh"
 #include "fast_walk.cuh"
@@ -499,7 +501,8 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
     if (n == 0) return AE_OK;
     if (n >= kMaxLeafFirst) return c->fail(AE_ERR_LAYOUT, "%u objects: the instance tree addresses at most %u", n, kMaxLeafFirst);
     // Mesh objects' boxes by the refresh kernel (no margin): 256 sub-boxes of
-    // eight corners an instance took the host 20 us each.
+    // eight corners an instance took the host 10 us each (1,024 instances: prepare
+    // 14.6 -> 3.8 ms).
     if (F.obj_box.reserve(size_t(n) * 6) || F.static_box.reserve(size_t(n) * 6)) return c->fail(AE_ERR_OOM, "instance tree");
     k_object_boxes<<<(n * 32 + 255) / 256, 256, 0, c->stream>>>(F.obj_meta.ptr, F.inst.ptr, F.sub_boxes.ptr, F.sub_refs.ptr,
                                                                  F.static_box.ptr, n, 0.0f, F.obj_box.ptr);
@@ -933,8 +936,8 @@ void destroy_fast(Ctx *c) {
 
 // Closest hit over a ray batch; one thread per ray.  The occupancy bound
 // (8 blocks of 128 per SM, so at most 64 registers) was chosen by timing on
-// the B200: 12 % more rays/s than the unbounded 79-register build, whose
-// 6 resident blocks left the latency-bound walk short of warps.
+// the B200: 1080p camera rays 772 us, against 788 us at 7 and 854 us at 6
+// blocks.
 template <bool WT>
 __global__ void __launch_bounds__(128, 8) k_closest_fast(DevScene S, FastView V, const ae_ray *__restrict__ rays,
                                                       uint32_t n, uint32_t lanes, ae_hit *__restrict__ hits) {
@@ -1109,6 +1112,7 @@ cudaError_t launch_closest_walk(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         per_sm = std::max(per_sm, 1);
     }
+    if (spread_quads(n, uint32_t(sms) * 8u * 4u)) return launch_closest_fast(c, rays, n, hits, false, st);
     const uint32_t grid = std::min<uint32_t>(uint32_t(per_sm) * uint32_t(sms), (n + 3) / 4);  // at least a ray a warp
     if (n < kWalkDynamicMin) {
         k_closest_walk<false><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, hits, nullptr);
@@ -1139,6 +1143,28 @@ cudaError_t launch_count_fast(Ctx *c, const ae_ray *rays, uint32_t n, bool quant
     return cudaGetLastError();
 }
 
+// Closest hit of a small batch, a quad of lanes a ray (quad_walk.cuh), `quads`
+// of them in each warp.
+template <bool WT>
+__global__ void __launch_bounds__(128) k_closest_quad(DevScene S, FastView V, const ae_ray *__restrict__ rays, uint32_t n,
+                                                      uint32_t quads, ae_hit *__restrict__ hits) {
+    extern __shared__ uint2 stk[];
+    const uint32_t q = (threadIdx.x & 31u) >> 2, i = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * quads + q;
+    if (q >= quads || i >= n) return;
+    const float4 *rp = reinterpret_cast<const float4 *>(rays + i);
+    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+    const Best best = closest_quad<WT>(S, V, mk(r0.x, r0.y, r0.z), mk(r1.x, r1.y, r1.z), r0.w, r1.w, stk);
+    if (threadIdx.x & 3u) return;
+    const bool any = best.object != AE_MISS;
+    ae_hit h;
+    h.t = any ? best.t : 0.0f;
+    h.alpha = any ? best.alpha : 0.0f;
+    h.beta = any ? best.beta : 0.0f;
+    h.object = best.object;
+    h.prim = best.prim;
+    hits[i] = h;
+}
+
 cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, bool quant, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     FastScene &F = *c->fast;
@@ -1153,7 +1179,14 @@ cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         sms = std::max(sms, 1);
     }
-    const uint32_t per_block = threads / 32, lanes = spread_lanes(n, uint32_t(sms) * 8u * per_block);
+    const uint32_t per_block = threads / 32;
+    if (const uint32_t quads = spread_quads(n, uint32_t(sms) * 8u * per_block)) {
+        const uint32_t grid = (n + per_block * quads - 1) / (per_block * quads);
+        if (quant) k_closest_quad<true><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, quads, hits);
+        else k_closest_quad<false><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, quads, hits);
+        return cudaGetLastError();
+    }
+    const uint32_t lanes = spread_lanes(n, uint32_t(sms) * 8u * per_block);
     const uint32_t grid = uint32_t((uint64_t(n) + per_block * lanes - 1) / (per_block * lanes));
     if (quant) {
         k_closest_fast<true><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, lanes, hits);

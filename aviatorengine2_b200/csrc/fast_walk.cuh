@@ -21,11 +21,10 @@ namespace ae {
 enum : uint32_t { kWalkTlas = 0, kWalkObject = 1, kWalkBlas = 2, kWalkDone = 3 };
 
 // Minimum resident 128-thread blocks per SM asked of the compiler for every
-// kernel built on Walker (extend and shadow, wavefront and serving): caps them
-// at 72 registers.  Measured at 1920x1080 on the 10M-triangle wavefront scene:
-// 7 blocks (28-108 bytes of spills) beat both the unbounded build (79-87
-// registers, 6 blocks) and 8 blocks (64 registers, 110-280 bytes of spills) -
-// wavefront frame 177 ms against 192 ms and 179 ms.
+// serving kernel built on Walker: caps them at 72 registers.  Chosen on an
+// earlier form of the walk, where 7 blocks beat 6 and 8 (1080p frame of the
+// 10M-triangle scene 177 ms against 192 and 179 ms).  The batch walker takes 8,
+// and the wavefront's stages are timed at 6 and 7.
 constexpr int kWalkBlocksPerSm = 7;
 
 // The walk's stack beyond its shared-memory part.  Kept out of Walker so its
@@ -181,6 +180,13 @@ struct Walker {
 __host__ __device__ inline uint32_t spread_lanes(uint32_t count, uint32_t warps) {
     const uint32_t half = (warps + 1u) / 2u, l = count / half + (count % half ? 1u : 0u);
     return l > 16u ? 32u : (l ? l : 1u);
+}
+
+// How many quads of each warp take a ray (quad_walk.cuh), or 0 where eight in
+// half of the warps do not reach (20,000 rays: 149 us either way).
+__host__ __device__ inline uint32_t spread_quads(uint32_t count, uint32_t warps) {
+    const uint32_t half = (warps + 1u) / 2u, q = count / half + (count % half ? 1u : 0u);
+    return q > 8u ? 0u : (q ? q : 1u);
 }
 
 // Run assignment for a persistent walker grid: the lanes of a warp that need

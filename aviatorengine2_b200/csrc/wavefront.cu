@@ -40,6 +40,7 @@
 #include "shade.cuh"
 #include "trace_common.cuh"
 #include "fast_walk.cuh"
+#include "quad_walk.cuh"
 #include "wf_common.cuh"
 
 namespace ae {
@@ -230,6 +231,22 @@ __global__ void __launch_bounds__(128, MINB) k_wf_extend_walk(DevScene S, FastVi
     const uint32_t warps = gridDim.x * (blockDim.x / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
     const uint32_t stride = warps * lanes;
     uint32_t k = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * lanes + lane;
+    if (const uint32_t quads = spread_quads(count, warps)) {
+        const uint32_t i = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * quads + lane / 4;
+        if (lane / 4 >= quads || i >= count) return;
+        const ae_ray r = W.qray[q][i];
+        const Best b = closest_quad<WT>(S, V, mk(r.ox, r.oy, r.oz), mk(r.dx, r.dy, r.dz), r.tnear, r.time, stk);
+        if (lane & 3u) return;
+        const bool any = b.object != AE_MISS;
+        ae_hit h;
+        h.t = any ? b.t : 0.0f;
+        h.alpha = any ? b.alpha : 0.0f;
+        h.beta = any ? b.beta : 0.0f;
+        h.object = b.object;
+        h.prim = b.prim;
+        W.qhit[i] = h;
+        return;
+    }
     if (lanes < 32u) {
         // Few rays, few of them in a warp: one after another, without the
         // votes that full warps gain from (500 rays: 100 -> 65 us).
@@ -345,9 +362,11 @@ __global__ void __launch_bounds__(THREADS, MINB * 128 / THREADS)
     const uint32_t warps = gridDim.x * (THREADS / 32), lanes = spread_lanes(count, warps), lane = threadIdx.x & 31u;
     const uint32_t stride = warps * lanes;
     uint32_t k = (blockIdx.x * (THREADS / 32) + threadIdx.x / 32) * lanes + lane;
+    const uint32_t quads = spread_quads(count, warps);
     if (lanes < 32u) {
         // Few samples: as k_wf_extend_walk.
-        for (; lane < lanes && k < count; k += stride) {
+        const uint32_t per = quads ? quads : lanes, in = quads ? lane / 4 : lane;
+        for (k = (blockIdx.x * (THREADS / 32) + threadIdx.x / 32) * per + in; in < per && k < count; k += warps * per) {
             const uint32_t se = W.sq[k];
             const float4 o4 = W.sh.o[se], d4 = W.sh.d[se], l4 = W.sh.lp[se];
             f3 so = mk(o4.x, o4.y, o4.z);
@@ -355,7 +374,8 @@ __global__ void __launch_bounds__(THREADS, MINB * 128 / THREADS)
             int verdict = 0;
             for (int i = 0; i < 4; i++) {
                 const float bound = AE_SUB(distance(lp, so), 0.001f);
-                const Best b = closest_fast<WT>(S, V, so, sd, 0.001f, d4.w, stk, threadIdx.x, 128, nullptr, bound);
+                const Best b = quads ? closest_quad<WT>(S, V, so, sd, 0.001f, d4.w, stk, bound)
+                                     : closest_fast<WT>(S, V, so, sd, 0.001f, d4.w, stk, threadIdx.x, 128, nullptr, bound);
                 verdict = 0;
                 if (b.object == AE_MISS || !(b.t < bound)) break;
                 const uint32_t mt = load_head(S.objects + b.object).material;
