@@ -880,10 +880,10 @@ int prepare_fast(Ctx *c) {
 // Structures that are not current are brought up to date once the rays that
 // the reference walk has traced without them (this call's included) would
 // have paid for it, so a scene that is asked little never pays, and one that
-// is asked much pays about once.  Against the reference walk a ray saves 4 to 8
-// ns (visibility segments 4.6, hybrid pixels 8); the build took 0.4 ms for the
-// Cornell box, 2.4 ms for 260 objects of 250,000 triangles and 3.8 ms for 1,040
-// of 2M, and after a move 0.15 ms for 520 objects.
+// is asked much pays about once.  Against the reference walk a ray saves about
+// 5 ns (visibility segments 4.6); the build took 0.4 ms for the Cornell box, 2.4
+// ms for 260 objects of 250,000 triangles and 3.8 ms for 1,040 of 2M; a move
+// refreshes the instance tree alone.
 ExactView exact_view(Ctx *c, uint64_t rays) {
     ExactView X;
     std::memset(&X, 0, sizeof(X));

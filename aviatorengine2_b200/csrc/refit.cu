@@ -117,8 +117,7 @@ __global__ void k_refit_level(ae_bvh_node *nodes, float *raw, const float *obj_b
     if (k < count) refit_node(nodes, raw, obj_box, level[k]);
 }
 // All levels, deepest first, by one block: a small tree's levels are shorter
-// than the gaps between their launches (516 objects: 11 launches, 38 us -> 1,
-// 14 us).
+// than the gaps between their launches (516 objects: 11 launches become one).
 __global__ void __launch_bounds__(1024) k_refit_levels(ae_bvh_node *nodes, float *raw, const float *obj_box,
                                                        const int32_t *order, const int32_t *start, int32_t levels) {
     for (int32_t l = 0; l < levels; l++) {
@@ -246,8 +245,8 @@ extern "C" int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uin
     if ((rc = c->cuda(cudaMemcpyAsync(c->instances.ptr, R.inst_in.ptr, size_t(n) * sizeof(ae_instance),
                                       cudaMemcpyDeviceToDevice, c->stream), "instances")))
         return rc;
-    // One block reaches about 200 nodes a microsecond and a launch costs three:
-    // from a few thousand nodes on, a level is worth its own launch.
+    // From a few thousand nodes on, a level fills more than one block and is
+    // worth its own launch.
     const bool one_block = nn <= 8192;
     if (one_block) {
         k_refit_levels<<<1, 1024, 0, c->stream>>>(c->tlas.ptr, R.raw.ptr, c->obj_box.ptr, R.level_nodes.ptr,
