@@ -28,7 +28,7 @@ namespace ae {
 // kPlaneUnused: read as a float, its second word is +inf instead of a negative
 // number, which the interval test takes for an entry distance.
 struct QNode {
-    float ox, oy, oz;        // frame origin, 2 * 2^e below the node box minimum
+    float ox, oy, oz;        // frame origin, a little over 2 * 2^e below the node box minimum
     uint32_t scale;
     uint2 plane[4];
     uint32_t child[4];       // interior: node index; leaf: leaf_ref(first, count); kNoChild
@@ -248,8 +248,9 @@ AE_DEV bool tri_test_wt(f3 o, const WtRay &W, float tn, float tf, const float4 &
 
 // Relative widening of slab intervals in the optimised walks: an interval's
 // exit and the best distance are scaled up by 1 + 2^-19 before they are
-// compared with an entry, so neither a nearer hit nor one on a box's face is
-// pruned by the rounding of the plane distances.
+// compared with an entry.  Together with the planes' room (kPlaneRoom,
+// quantise.cuh) that covers the rounding of the plane distances: neither a
+// nearer hit nor one on a box's face is pruned.
 constexpr float kExitGrow = 1.0000019073486328125f;  // 1 + 2^-19
 
 AE_DEV float max3(float a, float b, float c) {
