@@ -270,6 +270,7 @@ ae_ctx *ae_create(const ae_settings *s) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, s->device);
     if (e != cudaSuccess) {
         fprintf(stderr, "ae_create: %s\n", cudaGetErrorString(e));
         cudaGetLastError();

@@ -57,6 +57,7 @@ struct Ctx {
     std::string err;
     uint64_t launches = 0;
     bool timed = false;
+    int sms = 1;  // multiprocessors of the context's device
 
     // Geometry, uploaded once (UploadMeshGeometry).
     DevBuf<ae_vertex> vertices;

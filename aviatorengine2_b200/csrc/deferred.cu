@@ -1118,7 +1118,7 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
     uint32_t off = 0;
     for (size_t i = 0; i < plan.size(); i++) {
         const int k = int(i % Ctx::kIoSlots);
-        const uint32_t m = plan[i], lanes = spread_lanes(m, 148u * 8u * 4u), per_block = 4u * lanes;
+        const uint32_t m = plan[i], lanes = spread_lanes(m, uint32_t(c->sms) * 8u * 4u), per_block = 4u * lanes;
         const uint32_t grid = (m + per_block - 1) / per_block;
         if ((rc = c->cuda(cudaMemcpyAsync(c->io_rays[k].ptr, rays + off, size_t(m) * sizeof(ae_ray), cudaMemcpyHostToDevice,
                                           st[k]), "copy rays")) ||

@@ -1102,18 +1102,17 @@ cudaError_t launch_closest_walk(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
     FastView V = fast_view(F);
     const int threads = 128;
     const size_t smem = size_t(kSharedStack) * threads * sizeof(uint2);
-    static int per_sm = 0, sms = 0;
-    if (!per_sm) {
-        cudaFuncSetAttribute(k_closest_walk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        cudaFuncSetAttribute(k_closest_walk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_closest_walk<true>, threads, smem);
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        per_sm = std::max(per_sm, 1);
-    }
-    if (spread_quads(n, uint32_t(sms) * 8u * 4u)) return launch_closest_fast(c, rays, n, hits, false, st);
-    const uint32_t grid = std::min<uint32_t>(uint32_t(per_sm) * uint32_t(sms), (n + 3) / 4);  // at least a ray a warp
+    // A property of the kernel on this architecture.  Contexts on other threads
+    // may get here at the same time: the initialiser runs once and the others
+    // wait for it.
+    static const int per_sm = [&] {
+        int blocks = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_closest_walk<true>, threads, smem) != cudaSuccess)
+            cudaGetLastError();
+        return std::max(blocks, 1);
+    }();
+    if (spread_quads(n, uint32_t(c->sms) * 8u * 4u)) return launch_closest_fast(c, rays, n, hits, false, st);
+    const uint32_t grid = std::min<uint32_t>(uint32_t(per_sm) * uint32_t(c->sms), (n + 3) / 4);  // at least a ray a warp
     if (n < kWalkDynamicMin) {
         k_closest_walk<false><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, hits, nullptr);
         return cudaGetLastError();
@@ -1172,21 +1171,14 @@ cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *
     const int threads = 128;
     const size_t smem = size_t(kSharedStack) * threads * sizeof(uint2);
     // Fewer rays than the GPU holds at once: fewer of them in each warp.
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        sms = std::max(sms, 1);
-    }
-    const uint32_t per_block = threads / 32;
-    if (const uint32_t quads = spread_quads(n, uint32_t(sms) * 8u * per_block)) {
+    const uint32_t per_block = threads / 32, warps = uint32_t(c->sms) * 8u * per_block;
+    if (const uint32_t quads = spread_quads(n, warps)) {
         const uint32_t grid = (n + per_block * quads - 1) / (per_block * quads);
         if (quant) k_closest_quad<true><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, quads, hits);
         else k_closest_quad<false><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, quads, hits);
         return cudaGetLastError();
     }
-    const uint32_t lanes = spread_lanes(n, uint32_t(sms) * 8u * per_block);
+    const uint32_t lanes = spread_lanes(n, warps);
     const uint32_t grid = uint32_t((uint64_t(n) + per_block * lanes - 1) / (per_block * lanes));
     if (quant) {
         k_closest_fast<true><<<grid, threads, smem, st>>>(c->scene(), V, rays, n, lanes, hits);

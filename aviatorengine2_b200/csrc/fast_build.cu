@@ -307,7 +307,7 @@ int build_mesh_structures(Ctx *c, FastScene &F) {
             return rc;
         k_wide_roots<<<(trees + 127) / 128, 128, 0, st>>>(c->blas.ptr, tb, trees, owner, front, words);
         for (int l = 0; l < kBlasStack + 1; l++)
-            k_wide_level<<<148 * 4, 128, 0, st>>>(c->blas.ptr, owner, front + (l & 1 ? nb : 0),
+            k_wide_level<<<c->sms * 4, 128, 0, st>>>(c->blas.ptr, owner, front + (l & 1 ? nb : 0),
                                                   front + (l & 1 ? 0 : nb), words, l);
         k_wide_scan<<<blocks, 1024, 0, st>>>(owner, nb, index, sums);
         k_wide_scan_sums<<<1, 1024, 0, st>>>(sums, blocks, words);

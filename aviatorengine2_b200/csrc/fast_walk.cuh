@@ -15,6 +15,7 @@
 // equal distances), so the Best it returns is bit-identical.
 #pragma once
 #include "fast_trace.cuh"
+#include "spread.h"
 
 namespace ae {
 
@@ -166,28 +167,6 @@ struct Walker {
         return phase == kWalkDone;
     }
 };
-
-// How many lanes of each warp take rays when `count` rays meet the `warps`
-// warps that a launch has resident: all 32, or, with few rays, so few that the
-// rays occupy about half of the warps.  Lanes that diverge then wait for fewer
-// neighbours, which is what a small launch's time is made of (it lasts as long
-// as its slowest rays), and idle warps cost nothing.  Random rays through 200
-// instances, one ray a thread / step-wise walk, all lanes -> spread: 500 rays
-// 165 -> 65 / 155 -> 100 us, 8,000 rays 193 -> 115 / 184 -> 135 us, 20,000
-// rays 197 -> 149 / 175 -> 172 us.  From a quarter of the lanes on, full warps
-// issue less and win (50,000 rays: 199 -> 213 us on the walk), hence the limit
-// of 16.
-__host__ __device__ inline uint32_t spread_lanes(uint32_t count, uint32_t warps) {
-    const uint32_t half = (warps + 1u) / 2u, l = count / half + (count % half ? 1u : 0u);
-    return l > 16u ? 32u : (l ? l : 1u);
-}
-
-// How many quads of each warp take a ray (quad_walk.cuh), or 0 where eight in
-// half of the warps do not reach (20,000 rays: 149 us either way).
-__host__ __device__ inline uint32_t spread_quads(uint32_t count, uint32_t warps) {
-    const uint32_t half = (warps + 1u) / 2u, q = count / half + (count % half ? 1u : 0u);
-    return q > 8u ? 0u : (q ? q : 1u);
-}
 
 // Run assignment for a persistent walker grid: the lanes of a warp that need
 // work (need) take the next indices of the warp's current run of `run`
