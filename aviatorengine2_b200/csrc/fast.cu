@@ -527,25 +527,12 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
                 F.static_range = std::max(F.static_range, std::max(std::fabs(boxes[s].lo[a]), std::fabs(boxes[s].hi[a])));
         }
     }
-    // A hit on a sphere may lie off its surface by 2^-23 |oc|^2 / r (the
-    // discriminant's rounding): room for that, for origins up to 16 times the
-    // scene's coordinates (ExactView::max_origin).
-    F.has_spheres = false;
-    double reach = 0.0;
-    for (const Box &b : boxes)
-        for (int a = 0; a < 3; a++) reach = std::max(reach, double(std::max(std::fabs(b.lo[a]), std::fabs(b.hi[a]))));
+    // For the exact walks' widening: the smallest sphere (0 for a radius that
+    // is no positive number).
+    F.sphere_min = 3.402823466e38f;
     for (uint32_t s = 0; s < n; s++) {
         const ae_object &o = c->host_objects[s];
-        if (o.shapeType != AE_SHAPE_SPHERE) continue;
-        F.has_spheres = true;
-        const float more = float(std::ldexp(reach * reach / std::max(std::fabs(double(o.radius)), 1e-6), -14));
-        if (!(more < 1e30f)) continue;
-        for (int a = 0; a < 3; a++) {
-            boxes[s].lo[a] -= more;
-            boxes[s].hi[a] += more;
-            stat[6 * size_t(s) + a] = boxes[s].lo[a];
-            stat[6 * size_t(s) + 3 + a] = boxes[s].hi[a];
-        }
+        if (o.shapeType == AE_SHAPE_SPHERE) F.sphere_min = std::min(F.sphere_min, o.radius > 0.0f ? o.radius : 0.0f);
     }
     ObjectTree T{boxes, {}, {}};
     T.idx.resize(n);
@@ -924,7 +911,17 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
     X.k = std::ldexp(F.tri_factor, -17);
     X.world_r = F.range;
     X.mesh_r = F.mesh_range;
-    X.max_origin = F.has_spheres ? 16.0f * F.range : 3.0e38f;
+    X.max_origin = 3.0e38f;
+    if (F.sphere_min < 3.402823466e38f) {
+        // Origins for which the spheres' widening stays below 2^-8 of the
+        // scene; none, and no exact walk, where even the scene's own reach
+        // asks for more.
+        const double k = std::ldexp(1.0, -19) / double(F.sphere_min), r = double(F.range);
+        const double reach = std::sqrt(std::ldexp(r, -8) / k);
+        if (!(reach > 2.0 * r)) return X;
+        X.sphere_k = float(k);
+        X.max_origin = float(std::min(reach - 2.0 * r, 3.0e38));
+    }
     X.on = 1;
     return X;
 }

@@ -126,7 +126,7 @@ struct FastScene {
     // factor A, the largest mesh-space coordinate, and per object the
     // intersection of the reference TLAS boxes above it.
     float tri_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
-    bool has_spheres = false, moving_spheres = false;
+    float sphere_min = 3.402823466e38f;  // smallest radius
     uint2 nan_ref = {0xffffffffu, 0xffffffffu}, nan_wt = {0xffffffffu, 0xffffffffu};
     DevBuf<float4> obj_chain;
     DevBuf<int32_t> tlas_parent;
