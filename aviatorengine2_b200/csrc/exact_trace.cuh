@@ -19,7 +19,7 @@
 //
 // C: an accepted triangle's hit point o + d t lies within
 // eps = A 2^-17 (|o| + R) of the triangle, A = |e1| |e2| / |e1 x e2| at most over the
-// scene's triangles: the binary32 errors of the plane distance and of the
+// scene's triangles and its planar objects (by their edges): the binary32 errors of the plane distance and of the
 // barycentric test (both under 2^-21 (|o| + R) in the plane's normal, that times
 // A within the plane), with a factor of eight to spare.  The walk here widens
 // every box by eps (4 eps in world space, which covers the instance

@@ -528,11 +528,19 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
         }
     }
     // For the exact walks' widening: the smallest sphere (0 for a radius that
-    // is no positive number).
+    // is no positive number) and the shape factor of the planar objects that
+    // the reference test can accept.
     F.sphere_min = 3.402823466e38f;
+    F.planar_factor = 1.0f;
     for (uint32_t s = 0; s < n; s++) {
         const ae_object &o = c->host_objects[s];
         if (o.shapeType == AE_SHAPE_SPHERE) F.sphere_min = std::min(F.sphere_min, o.radius > 0.0f ? o.radius : 0.0f);
+        if (o.shapeType != AE_SHAPE_QUAD && o.shapeType != AE_SHAPE_TRIANGLE) continue;
+        const f3 u = mk(o.u_x, o.u_y, o.u_z), v = mk(o.v_x, o.v_y, o.v_z), nn = cross(u, v);
+        const float n2 = dot(nn, nn);
+        if (n2 < 1e-8f) continue;
+        const double f = std::sqrt(double(dot(u, u))) * std::sqrt(double(dot(v, v))) / std::sqrt(double(n2));
+        F.planar_factor = f < 1e30 ? std::max(F.planar_factor, float(f)) : 3.402823466e38f;
     }
     ObjectTree T{boxes, {}, {}};
     T.idx.resize(n);
@@ -905,10 +913,11 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
         return X;
     }
     const FastScene &F = *c->fast;
-    if (!(F.tri_factor <= 4096.0f)) return X;
+    const float factor = std::max(F.tri_factor, F.planar_factor);
+    if (!(factor <= 4096.0f)) return X;
     X.V = fast_view(F);
     X.chain = F.obj_chain.ptr;
-    X.k = std::ldexp(F.tri_factor, -17);
+    X.k = std::ldexp(factor, -17);
     X.world_r = F.range;
     X.mesh_r = F.mesh_range;
     X.max_origin = 3.0e38f;

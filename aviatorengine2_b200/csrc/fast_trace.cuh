@@ -122,10 +122,10 @@ struct FastScene {
     DevBuf<int32_t> tlevel_start_dev;
     std::vector<float> inst_radius;  // per instance: its mesh's largest local coordinate
     uint32_t troot = kEmptyTlas, n_tnodes = 0;
-    // What the exact walks need beyond (exact_trace.cuh): the triangles' shape
-    // factor A, the largest mesh-space coordinate, and per object the
+    // What the exact walks need beyond (exact_trace.cuh): the shape factor A of
+    // the meshes' triangles and of the planar objects, the largest mesh-space coordinate, and per object the
     // intersection of the reference TLAS boxes above it.
-    float tri_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
+    float tri_factor = 1.0f, planar_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
     float sphere_min = 3.402823466e38f;  // smallest radius
     uint2 nan_ref = {0xffffffffu, 0xffffffffu}, nan_wt = {0xffffffffu, 0xffffffffu};
     DevBuf<float4> obj_chain;

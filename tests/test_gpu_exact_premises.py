@@ -129,3 +129,27 @@ def test_boxes_beside_a_ground_sphere():
         L.check(L.lib().ae_trace_counters_variant(ctx.handle, ctypes.c_void_p(rays.data_ptr()), n, L.VARIANT_FAST,
                                                   L.ptr(count)), ctx.handle)
         assert count[1] < 10 * n
+
+
+@pytest.mark.parametrize("shape", [L.SHAPE_QUAD, L.SHAPE_TRIANGLE])
+@pytest.mark.parametrize("width", [1e-4, 5e-3])
+def test_skewed_planar_objects(shape, width):
+    """Edges nearly parallel (shape factors of 100,000 and 2,000): the normal's
+    rounding tilts the plane, and rays are accepted far off the shape."""
+    rng = np.random.default_rng(4)
+    lib = scenes.MeshLibrary()
+    a = rng.normal(size=3)
+    a /= np.linalg.norm(a)
+    b = np.cross(a, rng.normal(size=3))
+    b /= np.linalg.norm(b)
+    u, v = 10.0 * a, 9.0 * a + width * b
+    at = np.array([(-4.0, -3.0, -5.0), (3.0, 4.0, 5.0)])
+    ents = [scenes.entity(shape, L.MAT_LAMBERTIAN, p, u=tuple(u), v=tuple(v)) for p in at] + [small_mesh(lib)]
+    s = finish(ents, lib, "skewed")
+    n = 140_000
+    away = 1.5 * rng.uniform(-1, 1, (n, 2)) ** 5
+    p = at[rng.integers(0, 2, n)] + rng.uniform(0, 19, (n, 1)) * a + away[:, :1] * np.cross(a, b) + away[:, 1:] * b
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays, dist = rays_to(p - rng.choice([3.0, 30.0, 300.0], (n, 1)) * d, p, rng)
+    agree(s, rays, (dist * 1.5).astype(np.float32))
