@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -155,6 +156,18 @@ std::vector<uint32_t> host_chunks(uint32_t n) {
         for (int i = 2; i >= 0; i--) plan.push_back(kRamp[i]);
     }
     return plan;
+}
+
+// Whether every instance's quaternion has length 1 to 2^-18 in the square (a
+// normalised binary32 one is within 2^-21).  Then its conjugate, by which the
+// walks take a ray to the mesh, inverts the rotation by which the instance's
+// box was made to 2^-16 of the mesh's size, a quarter of the boxes' margin.
+bool unit_rotations(const ae_instance *inst, uint32_t n) {
+    for (uint32_t i = 0; i < n; i++) {
+        const double x = inst[i].qx, y = inst[i].qy, z = inst[i].qz, w = inst[i].qw;
+        if (!(std::fabs(x * x + y * y + z * z + w * w - 1.0) <= std::ldexp(1.0, -18))) return false;
+    }
+    return true;
 }
 
 // The side streams of a chunked host batch, ordered behind the work already on
@@ -427,6 +440,7 @@ int ae_upload_scene(ae_ctx *ctx, const ae_object *objects, uint32_t n_objects, c
         if (o.colorType == AE_MAT_ISOTROPIC) c->scene_has_media = true;
         if (o.shapeType == AE_SHAPE_SPHERE && !(o.x == o.x2 && o.y == o.y2 && o.z == o.z2)) c->scene_has_moving_spheres = true;
     }
+    c->scene_rigid = unit_rotations(instances, n_instances);
     c->scene_uploaded = true;
     c->scene_version++;
     c->scene_version_layout++;

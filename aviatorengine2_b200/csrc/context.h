@@ -85,6 +85,7 @@ struct Ctx {
     bool scene_uploaded = false;
     uint64_t scene_triangles = 0;  // over all instances
     bool scene_has_media = false, scene_has_moving_spheres = false;
+    bool scene_rigid = true;  // unit_rotations of the current instances
     bool scene_has_ggx = false;  // an object uses AE_MAT_GGX_METAL (not shaded by the hybrid passes)
     uint32_t fault_tile_wait = 0;  // ae_debug_inject(AE_FAULT_TILE_WAIT)
     uint32_t fault_check_limits = 0;  // ae_debug_inject(AE_FAULT_CHECK_LIMITS)
@@ -135,6 +136,7 @@ struct Ctx {
 
 // Implemented by the optimised-kernel translation units.
 std::vector<uint32_t> host_chunks(uint32_t n);
+bool unit_rotations(const ae_instance *inst, uint32_t n);
 int ensure_side_streams(Ctx *c);
 int prepare_variant(Ctx *c, int variant);
 int closest_hit_dispatch(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, int variant, cudaStream_t st,

@@ -869,8 +869,9 @@ int prepare_fast(Ctx *c) {
 // The exact walks' view of the scene (exact_trace.cuh) for a frame or batch of
 // `rays` starting rays; off where the plain walks have to answer: participating
 // media (they draw random numbers in visit order), spheres that move within a
-// frame (their boxes hold one position), triangles so thin that the widening
-// would swallow the scene, or structures that cannot be built.
+// frame (their boxes hold one position), rotations that are not of unit length
+// (unit_rotations), triangles so thin that the widening would swallow the
+// scene, or structures that cannot be built.
 //
 // Structures that are not current are brought up to date once the rays that
 // the reference walk has traced without them (this call's included) would
@@ -882,7 +883,7 @@ int prepare_fast(Ctx *c) {
 ExactView exact_view(Ctx *c, uint64_t rays) {
     ExactView X;
     std::memset(&X, 0, sizeof(X));
-    if (c->scene_has_media || c->scene_has_moving_spheres || c->n_nodes == 0 || c->exact_refused == c->scene_version) return X;
+    if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0 || c->exact_refused == c->scene_version) return X;
     const bool built = c->fast && c->fast->geometry_key == c->geometry_version && !c->fast->geometry_dirty;
     if (!built || c->fast->scene_key != c->scene_version) {
         if (c->plain_scene != c->scene_version) c->plain_scene_rays = 0;

@@ -153,3 +153,61 @@ def test_skewed_planar_objects(shape, width):
     d /= np.linalg.norm(d, axis=1, keepdims=True)
     rays, dist = rays_to(p - rng.choice([3.0, 30.0, 300.0], (n, 1)) * d, p, rng)
     agree(s, rays, (dist * 1.5).astype(np.float32))
+
+
+@pytest.mark.parametrize("norm", [0.9995, 1.0005, 0.9, 1.0 + 1e-7])
+def test_quaternions_off_unit_length(norm):
+    """The walks' transform to a mesh's space uses the conjugate, which is the
+    inverse of a unit quaternion only."""
+    rng = np.random.default_rng(5)
+    lib = scenes.MeshLibrary()
+    ents = [scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (0, 0, 0), rotation=scenes.yaw_quat(np.pi / 2),
+                          mesh=lib.add(*scenes.box_mesh((5, 5, 5)))),
+            scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (-8, -8, -8), u=(1.0, 0, 0), v=(0, 1.0, 0)),
+            scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (7, 7, 8), u=(1.0, 0, 0), v=(0, 1.0, 0))]
+    s = finish(ents, lib, "quaternion")
+    for q in ("qx", "qy", "qz", "qw"):
+        s.instances[q] *= np.float32(norm)
+    n = 140_000
+    # Points in the outermost shell of the box, seen almost along its faces.
+    grow = 1.0 / norm ** 2 if norm < 1 else 1.0
+    p = rng.uniform(-5, 5, (n, 3))
+    axis = rng.choice([0, 2], n)
+    p[np.arange(n), axis] = rng.choice([-1.0, 1.0], n) * 5.0 * rng.uniform(min(grow, 1.0) - 2e-4, max(grow, 1.0) + 1.5e-3, n)
+    side = np.stack([np.where(axis == 0, 0.0, 1.0), rng.normal(size=n) * 0.2, np.where(axis == 0, 1.0, 0.0)], 1)
+    rays, dist = rays_to(p - 25.0 * side, p, rng, 1e-3)
+    agree(s, rays, (dist * 2.0).astype(np.float32))
+
+
+def test_refit_to_quaternions_off_unit_length():
+    """The same by a refit, and back."""
+    rng = np.random.default_rng(9)
+    lib = scenes.MeshLibrary()
+    ents = [scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (0, 0, 0), rotation=scenes.yaw_quat(np.pi / 2),
+                          mesh=lib.add(*scenes.box_mesh((5, 5, 5)))),
+            scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (-8, -8, -8), u=(16.0, 0, 0), v=(0, 1.0, 0)),
+            scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (7, 7, 8), u=(1.0, 0, 0), v=(0, 1.0, 0))]
+    s = finish(ents, lib, "quaternion")
+    off = s.instances.copy()
+    for q in ("qx", "qy", "qz", "qw"):
+        off[q] *= np.float32(0.95)
+    n = 60_000
+    p = rng.uniform(-6.2, 6.2, (n, 3))
+    rays, dist = rays_to(p + 25.0 * rng.normal(size=(n, 3)), p, rng)
+    tmax = (dist * 2.0).astype(np.float32)
+    got = []
+    for prepared in (True, False):
+        answers = []
+        for pose in (off, s.instances):
+            with scenes_context(s) as ctx:
+                if prepared:
+                    ctx.prepare_fast()
+                ctx.refit_instances(off)
+                if pose is not off:
+                    ctx.refit_instances(pose)
+                if prepared:
+                    ctx.prepare_fast()
+                answers.append(ctx.any_hit(rays, tmax))
+        got.append(answers)
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    assert not np.array_equal(got[1][0], got[1][1])
