@@ -36,7 +36,9 @@
 // 486 objects a ray instead of 2.2 when all walks' boxes were widened so).
 //
 // The slab tests above w: in the mesh, the triangle's own bounding box lies
-// inside every node above it; in the instance tree, `chain` holds the
+// inside every node above it (the build checks that, leaf_enclosed in
+// fast_build.cu; the walks are off for a scene with a tree where it does not);
+// in the instance tree, `chain` holds the
 // intersection of all boxes above the object (flat leaves are widened beyond
 // their parents, so the leaf's box alone would not do).
 //

@@ -871,7 +871,8 @@ int prepare_fast(Ctx *c) {
 // media (they draw random numbers in visit order), spheres that move within a
 // frame (their boxes hold one position), rotations that are not of unit length
 // (unit_rotations), triangles so thin that the widening would swallow the
-// scene, or structures that cannot be built.
+// scene, uploaded trees whose boxes do not hold their triangles, or structures
+// that cannot be built.
 //
 // Structures that are not current are brought up to date once the rays that
 // the reference walk has traced without them (this call's included) would
@@ -915,7 +916,7 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
     }
     const FastScene &F = *c->fast;
     const float factor = std::max(F.tri_factor, F.planar_factor);
-    if (!(factor <= 4096.0f)) return X;
+    if (!(factor <= 4096.0f) || F.loose_trees) return X;
     X.V = fast_view(F);
     X.chain = F.obj_chain.ptr;
     X.k = std::ldexp(factor, -17);

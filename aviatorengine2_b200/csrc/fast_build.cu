@@ -33,7 +33,7 @@ namespace {
 
 constexpr int kMaxLevels = 32;  // uploads are checked to kBlasStack (24) pending nodes, so at most 23 levels
 // Device words of a build: level sizes, then the flags below.
-enum { W_STACK = kMaxLevels, W_ERROR, W_TOTAL, W_FACTOR, W_COUNT };
+enum { W_STACK = kMaxLevels, W_ERROR, W_TOTAL, W_LOOSE, W_COUNT };
 enum { E_LEAF = 1, E_QUANT = 2, E_SHARED = 4, E_DEPTH = 8 };
 
 struct Kids {
@@ -41,17 +41,37 @@ struct Kids {
     int n;
 };
 
+// The intersection of a node's box and those above it.
+struct Clip {
+    float lo[3], hi[3];
+};
+__device__ Clip clip_to(const Clip &c, const ae_bvh_node &n) {
+    const float lo[3] = {n.min_x, n.min_y, n.min_z}, hi[3] = {n.max_x, n.max_y, n.max_z};
+    Clip r;
+    for (int a = 0; a < 3; a++) {
+        // A NaN bound stays, and holds nothing.
+        r.lo[a] = lo[a] > c.lo[a] || lo[a] != lo[a] ? lo[a] : c.lo[a];
+        r.hi[a] = hi[a] < c.hi[a] || hi[a] != hi[a] ? hi[a] : c.hi[a];
+    }
+    return r;
+}
+
 __device__ float node_half_area(const ae_bvh_node &n) {
     const float dx = __fsub_rn(n.max_x, n.min_x), dy = __fsub_rn(n.max_y, n.min_y), dz = __fsub_rn(n.max_z, n.min_z);
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dy), __fmul_rn(dy, dz)), __fmul_rn(dz, dx));
 }
 
-// The children of binary node i gathered into up to four.
-__device__ Kids gather_kids(const ae_bvh_node *bin, uint32_t i) {
+// The children of binary node i gathered into up to four.  clip (optional): on
+// entry clip[0] is node i's, on return each child's.
+__device__ Kids gather_kids(const ae_bvh_node *bin, uint32_t i, Clip *clip = nullptr) {
     Kids K;
     K.k[0] = uint32_t(bin[i].left);
     K.k[1] = uint32_t(bin[i].right);
     K.n = 2;
+    if (clip) {
+        clip[1] = clip_to(clip[0], bin[K.k[1]]);
+        clip[0] = clip_to(clip[0], bin[K.k[0]]);
+    }
     while (K.n < 4) {
         int best = -1;
         float area = -1.0f;
@@ -62,24 +82,76 @@ __device__ Kids gather_kids(const ae_bvh_node *bin, uint32_t i) {
         }
         if (best < 0) break;
         const uint32_t open = K.k[best];
-        for (int j = K.n; j > best + 1; j--) K.k[j] = K.k[j - 1];
+        for (int j = K.n; j > best + 1; j--) {
+            K.k[j] = K.k[j - 1];
+            if (clip) clip[j] = clip[j - 1];
+        }
         K.k[best] = uint32_t(bin[open].left);
         K.k[best + 1] = uint32_t(bin[open].right);
+        if (clip) {
+            clip[best + 1] = clip_to(clip[best], bin[K.k[best + 1]]);
+            clip[best] = clip_to(clip[best], bin[K.k[best]]);
+        }
         K.n++;
     }
     return K;
 }
 
+// A mesh: one grid row of the record kernels.
+struct MeshJob {
+    uint32_t vertex_base, index_base, tris, tri_base;
+};
+static_assert(sizeof(MeshJob) == 16, "four words in the build's tables");
+
+// All trees of a build by first node, ascending, and the meshes of each: those
+// numbered first_job[t] to first_job[t + 1].
+struct Trees {
+    const uint32_t *base, *first_job;
+    uint32_t count;
+    const MeshJob *jobs;
+    const float4 *tris;
+};
+
+// Whether a leaf's triangles lie in the boxes above them, in every mesh that
+// uses the tree (the exact walks count on it, exact_trace.cuh; the boxes of the
+// nodes need not nest: flat ones are thicker than what they hold).
+__device__ bool leaf_enclosed(const Trees &T, uint32_t base, const ae_bvh_node &leaf, const Clip &c) {
+    uint32_t a = 0, b = T.count - 1;
+    while (a < b) {
+        const uint32_t m = (a + b) / 2;
+        if (T.base[m] < base) a = m + 1;
+        else b = m;
+    }
+    for (uint32_t j = T.first_job[a]; j < T.first_job[a + 1]; j++) {
+        const MeshJob J = T.jobs[j];
+        for (int32_t k = 0; k < leaf.count; k++) {
+            if (uint32_t(leaf.left + k) >= J.tris) continue;
+            const float4 *r = T.tris + 3 * (size_t(J.tri_base) + leaf.left + k);
+            const float4 r0 = r[0], r1 = r[1], r2 = r[2];
+            const float p[3][3] = {{r0.x, r0.y, r0.z}, {r0.w, r1.x, r1.y}, {r1.z, r1.w, r2.x}};
+            for (int v = 0; v < 3; v++)
+                for (int x = 0; x < 3; x++)
+                    if (!(p[v][x] >= c.lo[x] && p[v][x] <= c.hi[x])) return false;
+        }
+    }
+    return true;
+}
+__device__ Clip no_clip() {
+    const float inf = __int_as_float(0x7f800000);
+    return Clip{{-inf, -inf, -inf}, {inf, inf, inf}};
+}
+
 // Roots of the trees into the first level.  owner[i] is 1 + the tree's first
 // node for the binary nodes that become 4-wide nodes, 0 for the rest.
 __global__ void k_wide_roots(const ae_bvh_node *__restrict__ blas, const uint32_t *__restrict__ base, uint32_t trees,
-                             uint32_t *owner, uint2 *front, uint32_t *words) {
+                             uint32_t *owner, Clip *clips, uint2 *front, uint32_t *words) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= trees || blas[base[t]].count > 0) return;
     if (atomicExch(owner + base[t], base[t] + 1u)) {
         atomicOr(words + W_ERROR, uint32_t(E_SHARED));
         return;
     }
+    clips[base[t]] = clip_to(no_clip(), blas[base[t]]);
     front[atomicAdd(words, 1u)] = make_uint2(base[t], 0u);
 }
 
@@ -87,11 +159,13 @@ __global__ void k_wide_roots(const ae_bvh_node *__restrict__ blas, const uint32_
 // holds when it reaches the node).
 __global__ void __launch_bounds__(128) k_wide_level(const ae_bvh_node *__restrict__ blas, uint32_t *owner,
                                                     const uint2 *__restrict__ front, uint2 *__restrict__ next,
-                                                    uint32_t *words, int level) {
+                                                    Clip *clips, Trees T, uint32_t *words, int level) {
     const uint32_t count = words[level];
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
         const uint32_t i = front[j].x, base = owner[i] - 1u;
-        const Kids K = gather_kids(blas + base, i - base);
+        Clip clip[4];
+        clip[0] = clips[i];
+        const Kids K = gather_kids(blas + base, i - base, clip);
         const uint32_t need = front[j].y + uint32_t(K.n - 1);
         atomicMax(words + W_STACK, need);
         for (int k = 0; k < K.n; k++) {
@@ -100,8 +174,10 @@ __global__ void __launch_bounds__(128) k_wide_level(const ae_bvh_node *__restric
             if (c.count > 0) {
                 if (uint32_t(c.count) > kMaxLeafCount || uint32_t(c.left) >= kMaxLeafFirst)
                     atomicOr(words + W_ERROR, uint32_t(E_LEAF));
+                else if (!leaf_enclosed(T, base, c, clip[k])) words[W_LOOSE] = 1u;
                 continue;
             }
+            clips[g] = clip[k];
             if (atomicExch(owner + g, base + 1u)) atomicOr(words + W_ERROR, uint32_t(E_SHARED));
             else if (level + 1 <= kBlasStack) next[atomicAdd(words + level + 1, 1u)] = make_uint2(g, need);
             else atomicOr(words + W_ERROR, uint32_t(E_DEPTH));
@@ -154,7 +230,7 @@ __global__ void __launch_bounds__(1024) k_wide_scan_sums(uint32_t *sums, uint32_
 // Root references of the trees, first node offset by `first`.
 __global__ void k_wide_root_refs(const ae_bvh_node *__restrict__ blas, const uint32_t *__restrict__ base,
                                  uint32_t trees, const uint32_t *__restrict__ index,
-                                 const uint32_t *__restrict__ sums, uint32_t first, uint32_t *words,
+                                 const uint32_t *__restrict__ sums, uint32_t first, Trees T, uint32_t *words,
                                  uint32_t *__restrict__ ref) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= trees) return;
@@ -162,6 +238,7 @@ __global__ void k_wide_root_refs(const ae_bvh_node *__restrict__ blas, const uin
     if (r.count > 0) {
         if (uint32_t(r.count) > kMaxLeafCount || uint32_t(r.left) >= kMaxLeafFirst)
             atomicOr(words + W_ERROR, uint32_t(E_LEAF));
+        else if (!leaf_enclosed(T, base[t], r, clip_to(no_clip(), r))) words[W_LOOSE] = 1u;
         ref[t] = leaf_ref(uint32_t(r.left) & 0xffffffu, uint32_t(r.count) & 0x7fu);
     } else {
         ref[t] = first + index[base[t]] + sums[base[t] >> 10];
@@ -196,13 +273,9 @@ __global__ void __launch_bounds__(128) k_wide_emit(const ae_bvh_node *__restrict
 }
 
 // Triangle records in slot order, one mesh per grid row.
-struct MeshJob {
-    uint32_t vertex_base, index_base, tris, tri_base;
-};
-static_assert(sizeof(MeshJob) == 16, "four words in the build's tables");
 __global__ void __launch_bounds__(256) k_tri_records(const ae_vertex *__restrict__ v, const uint32_t *__restrict__ idx,
                                                      const MeshJob *__restrict__ jobs, float4 *__restrict__ out,
-                                                     uint32_t *words) {
+                                                     uint32_t *most) {
     const MeshJob J = jobs[blockIdx.y];
     // Largest |e1| |e2| / |e1 x e2| of the triangles that the reference test can
     // accept (exact_trace.cuh), 1 and up; as bits, which order like the floats.
@@ -223,7 +296,7 @@ __global__ void __launch_bounds__(256) k_tri_records(const ae_vertex *__restrict
         }
     }
     factor = __reduce_max_sync(0xffffffffu, factor);
-    if ((threadIdx.x & 31u) == 0 && factor) atomicMax(words + W_FACTOR, factor);
+    if ((threadIdx.x & 31u) == 0 && factor) atomicMax(most, factor);
 }
 
 // FP16 shading records (layout in wf_common.cuh: PrecView).
@@ -247,10 +320,18 @@ template <class F> void for_rows(size_t rows, F launch) {
     for (size_t r = 0; r < rows; r += 65535) launch(r, uint32_t(std::min<size_t>(65535, rows - r)));
 }
 
-std::vector<MeshJob> mesh_jobs(const FastScene &F) {
-    std::vector<MeshJob> jobs;
+// The listed meshes by their trees' first nodes, and (optional) those.
+std::vector<MeshJob> mesh_jobs(const FastScene &F, std::vector<uint32_t> *tree = nullptr) {
+    std::vector<std::pair<uint32_t, MeshJob>> list;
     for (const auto &kv : F.mesh_roots)
-        jobs.push_back(MeshJob{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first), kv.second.second});
+        list.emplace_back(std::get<3>(kv.first), MeshJob{std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first),
+                                                         kv.second.second});
+    std::stable_sort(list.begin(), list.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
+    std::vector<MeshJob> jobs;
+    for (const auto &x : list) {
+        jobs.push_back(x.second);
+        if (tree) tree->push_back(x.first);
+    }
     return jobs;
 }
 uint32_t row_blocks(const std::vector<MeshJob> &jobs) {
@@ -265,35 +346,51 @@ uint32_t row_blocks(const std::vector<MeshJob> &jobs) {
 // (their root references are filled in), replacing what was there.
 int build_mesh_structures(Ctx *c, FastScene &F) {
     const uint32_t nb = uint32_t(c->n_blas);
-    std::vector<uint32_t> bases;
-    for (const auto &kv : F.mesh_roots) bases.push_back(std::get<3>(kv.first));
-    std::sort(bases.begin(), bases.end());
-    bases.erase(std::unique(bases.begin(), bases.end()), bases.end());
-    const std::vector<MeshJob> jobs = mesh_jobs(F);
+    std::vector<uint32_t> bases, first_job, tree_of;
+    const std::vector<MeshJob> jobs = mesh_jobs(F, &tree_of);
+    for (size_t j = 0; j < jobs.size(); j++)
+        if (!j || tree_of[j] != tree_of[j - 1]) {
+            bases.push_back(tree_of[j]);
+            first_job.push_back(uint32_t(j));
+        }
+    first_job.push_back(uint32_t(jobs.size()));
     F.max_stack = 0;
     F.n_nodes = 0;
     const uint32_t blocks = (nb + 1023u) / 1024u;
     if (F.tris.reserve(std::max<size_t>(size_t(F.n_tris) * 3, 1))) return c->fail(AE_ERR_OOM, "fast scene buffers");
     if (bases.empty()) return F.nodes.reserve(1) ? c->fail(AE_ERR_OOM, "fast scene buffers") : AE_OK;
-    // One scratch allocation, freed on return: the host tables (jobs, roots),
-    // then the build's arrays.
-    const size_t at_base = jobs.size() * 4, at_refs = at_base + bases.size(), at_words = at_refs + bases.size(),
-                 at_sums = at_words + W_COUNT, at_owner = at_sums + blocks, at_index = at_owner + nb,
-                 at_front = (at_index + nb + 1) & ~size_t(1);
+    // One scratch allocation, freed on return: the host tables (jobs, roots, each
+    // root's first job), then the build's arrays.
+    const size_t at_base = jobs.size() * 4, at_first = at_base + bases.size(), at_refs = at_first + first_job.size(),
+                 at_most = at_refs + bases.size(), at_words = at_most + 1, at_sums = at_words + W_COUNT,
+                 at_owner = at_sums + blocks, at_index = at_owner + nb, at_clips = at_index + nb,
+                 at_front = (at_clips + 6 * size_t(nb) + 1) & ~size_t(1);
+    static_assert(sizeof(Clip) == 24, "six words a node");
     DevBuf<uint32_t> scratch;
     if (scratch.reserve(at_front + 4 * size_t(nb))) return c->fail(AE_ERR_OOM, "fast scene build scratch");
     const MeshJob *d_jobs = reinterpret_cast<const MeshJob *>(scratch.ptr);
     uint32_t *const d_base = scratch.ptr + at_base, *const refs = scratch.ptr + at_refs,
              *const words = scratch.ptr + at_words, *const sums = scratch.ptr + at_sums,
-             *const owner = scratch.ptr + at_owner, *const index = scratch.ptr + at_index;
+             *const owner = scratch.ptr + at_owner, *const index = scratch.ptr + at_index,
+             *const most = scratch.ptr + at_most;
+    Clip *const clips = reinterpret_cast<Clip *>(scratch.ptr + at_clips);
+    const Trees T{d_base, scratch.ptr + at_first, uint32_t(bases.size()), d_jobs, F.tris.ptr};
     uint2 *const front = reinterpret_cast<uint2 *>(scratch.ptr + at_front);
     cudaStream_t st = c->stream;
     int rc;
     std::vector<uint32_t> tables(at_refs);
     std::memcpy(tables.data(), jobs.data(), jobs.size() * sizeof(MeshJob));
     std::copy(bases.begin(), bases.end(), tables.begin() + at_base);
-    if ((rc = c->cuda(cudaMemcpyAsync(scratch.ptr, tables.data(), at_refs * 4, cudaMemcpyHostToDevice, st), "mesh tables")))
+    std::copy(first_job.begin(), first_job.end(), tables.begin() + at_first);
+    if ((rc = c->cuda(cudaMemcpyAsync(scratch.ptr, tables.data(), at_refs * 4, cudaMemcpyHostToDevice, st), "mesh tables")) ||
+        (rc = c->cuda(cudaMemsetAsync(most, 0, 4, st), "triangle factor")))
         return rc;
+    const uint32_t gx = row_blocks(jobs);
+    for_rows(jobs.size(), [&](size_t r, uint32_t rows) {
+        k_tri_records<<<dim3(gx, rows), 256, 0, st>>>(c->vertices.ptr, c->indices.ptr, d_jobs + r, F.tris.ptr, most);
+    });
+    if ((rc = c->cuda(cudaGetLastError(), "triangle records"))) return rc;
+    F.loose_trees = false;
     std::vector<uint32_t> host_refs(bases.size());
     // All trees in one build.  Trees that share nodes (one's root inside
     // another's range) are built one after another instead, each with its
@@ -305,14 +402,14 @@ int build_mesh_structures(Ctx *c, FastScene &F) {
         if ((rc = c->cuda(cudaMemsetAsync(owner, 0, size_t(nb) * 4, st), "marks")) ||
             (rc = c->cuda(cudaMemsetAsync(words, 0, W_COUNT * 4, st), "build words")))
             return rc;
-        k_wide_roots<<<(trees + 127) / 128, 128, 0, st>>>(c->blas.ptr, tb, trees, owner, front, words);
+        k_wide_roots<<<(trees + 127) / 128, 128, 0, st>>>(c->blas.ptr, tb, trees, owner, clips, front, words);
         for (int l = 0; l < kBlasStack + 1; l++)
             k_wide_level<<<c->sms * 4, 128, 0, st>>>(c->blas.ptr, owner, front + (l & 1 ? nb : 0),
-                                                  front + (l & 1 ? 0 : nb), words, l);
+                                                  front + (l & 1 ? 0 : nb), clips, T, words, l);
         k_wide_scan<<<blocks, 1024, 0, st>>>(owner, nb, index, sums);
         k_wide_scan_sums<<<1, 1024, 0, st>>>(sums, blocks, words);
         k_wide_root_refs<<<(trees + 127) / 128, 128, 0, st>>>(c->blas.ptr, tb, trees, index, sums, F.n_nodes,
-                                                              words, refs + first_tree);
+                                                              T, words, refs + first_tree);
         uint32_t w[W_COUNT];
         if ((rc = c->cuda(cudaGetLastError(), "4-wide collapse")) ||
             (rc = c->cuda(cudaMemcpyAsync(w, words, sizeof(w), cudaMemcpyDeviceToHost, st), "build words")) ||
@@ -349,18 +446,14 @@ int build_mesh_structures(Ctx *c, FastScene &F) {
             (rc = c->cuda(cudaStreamSynchronize(st), "4-wide nodes")))
             return rc;
         if (w[W_ERROR] & E_QUANT) return c->fail(AE_ERR_LAYOUT, "4-wide BVH: a child box cannot be quantised conservatively");
+        F.loose_trees = F.loose_trees || w[W_LOOSE];
         F.n_nodes = uint32_t(total);
         F.max_stack = std::max(F.max_stack, int(w[W_STACK]));
         first_tree += trees;
     }
     uint32_t factor = 0;
-    const uint32_t gx = row_blocks(jobs);
-    for_rows(jobs.size(), [&](size_t r, uint32_t rows) {
-        k_tri_records<<<dim3(gx, rows), 256, 0, st>>>(c->vertices.ptr, c->indices.ptr, d_jobs + r, F.tris.ptr, words);
-    });
-    if ((rc = c->cuda(cudaGetLastError(), "triangle records")) ||
-        (rc = c->cuda(cudaMemcpyAsync(host_refs.data(), refs, bases.size() * 4, cudaMemcpyDeviceToHost, st), "tree roots")) ||
-        (rc = c->cuda(cudaMemcpyAsync(&factor, words + W_FACTOR, 4, cudaMemcpyDeviceToHost, st), "triangle factor")) ||
+    if ((rc = c->cuda(cudaMemcpyAsync(host_refs.data(), refs, bases.size() * 4, cudaMemcpyDeviceToHost, st), "tree roots")) ||
+        (rc = c->cuda(cudaMemcpyAsync(&factor, most, 4, cudaMemcpyDeviceToHost, st), "triangle factor")) ||
         (rc = c->cuda(cudaStreamSynchronize(st), "triangle records")))
         return rc;
     std::memcpy(&F.tri_factor, &factor, 4);

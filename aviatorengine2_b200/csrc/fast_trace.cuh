@@ -126,6 +126,7 @@ struct FastScene {
     // the meshes' triangles and of the planar objects, the largest mesh-space coordinate, and per object the
     // intersection of the reference TLAS boxes above it.
     float tri_factor = 1.0f, planar_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
+    bool loose_trees = false;  // a triangle reaches out of a box above it in its tree
     float sphere_min = 3.402823466e38f;  // smallest radius
     uint2 nan_ref = {0xffffffffu, 0xffffffffu}, nan_wt = {0xffffffffu, 0xffffffffu};
     DevBuf<float4> obj_chain;

@@ -211,3 +211,56 @@ def test_refit_to_quaternions_off_unit_length():
         got.append(answers)
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
     assert not np.array_equal(got[1][0], got[1][1])
+
+
+@pytest.mark.parametrize("what", ["nodes", "leaves", "root leaf"])
+def test_trees_that_do_not_enclose(what):
+    """BLAS boxes smaller than what lies below them cut hits off in the
+    reference walk."""
+    rng = np.random.default_rng(6)
+    lib = scenes.MeshLibrary()
+    mesh = scenes.icosphere(3, 4.0)
+    if what == "root leaf":
+        mesh = (mesh[0], mesh[1][:6])
+    ents = [scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (0, 0, 0), mesh=lib.add(*mesh)),
+            scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (-8, -8, -8), u=(16.0, 0, 0), v=(0, 1.0, 0))]
+    s = finish(ents, lib, "loose tree")
+    b = s.blas
+    assert (len(b) == 1) == (what == "root leaf")
+    pick = b["count"] == 0 if what == "nodes" else b["count"] > 0
+    if what == "nodes":
+        pick[0] = False
+    for x in "xyz":
+        mid = 0.5 * (b["min_" + x] + b["max_" + x])
+        b["min_" + x][pick] = (mid + 0.6 * (b["min_" + x] - mid))[pick]
+        b["max_" + x][pick] = (mid + 0.6 * (b["max_" + x] - mid))[pick]
+    p = rng.normal(size=(100_000, 3))
+    p *= 4.0 * rng.uniform(0.2, 1.0, (len(p), 1)) / np.linalg.norm(p, axis=1, keepdims=True)
+    if what == "root leaf":
+        tri = np.stack([mesh[0][x][mesh[1]] for x in ("px", "py", "pz")], 1).astype(np.float64).reshape(-1, 3, 3)
+        w = rng.dirichlet((1, 1, 1), len(p))
+        p = np.einsum("nk,nkc->nc", w, tri[rng.integers(0, len(tri), len(p))])
+    rays, dist = rays_to((3.0, 5.0, 14.0), p, rng, 2.0)
+    agree(s, rays, (dist * 1.2).astype(np.float32))
+
+
+def test_two_meshes_on_one_tree():
+    """A tree that two meshes name and that holds one of them only."""
+    rng = np.random.default_rng(10)
+    lib = scenes.MeshLibrary()
+    v, i = scenes.icosphere(3, 3.0)
+    small = lib.add(v, i)
+    w = v.copy()
+    for x in ("px", "py", "pz"):
+        w[x] *= 1.4
+    big = lib.add(w, i)
+    ents = [scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (x, 0, 0), mesh=m) for x, m in ((-6, small), (6, big))]
+    ents.append(scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (-12, -8, -8), u=(24.0, 0, 0), v=(0, 1.0, 0)))
+    s = finish(ents, lib, "two meshes")
+    assert len(s.instances) == 2
+    s.instances["blasBase"] = s.instances["blasBase"].min()
+    p = rng.normal(size=(100_000, 3))
+    p *= 4.2 * rng.uniform(0.2, 1.0, (len(p), 1)) / np.linalg.norm(p, axis=1, keepdims=True)
+    p[:, 0] += rng.choice([-6.0, 6.0], len(p))
+    rays, dist = rays_to((3.0, 5.0, 20.0), p, rng, 2.0)
+    agree(s, rays, (dist * 1.2).astype(np.float32))
