@@ -29,11 +29,12 @@
 // larger of r and the distance of origin and centre: the discriminant's
 // terms, each of D^2 |d|^2, are rounded 16 times (2^-24 each), and the square
 // root of r^2 + x is at most r + x / 2r.  World boxes are widened by four times
-// that for the scene's smallest sphere and D <= |o| + 2 R.  Rays for which this
-// exceeds 2^-8 of the scene (small spheres seen from far, beside a ground
-// sphere) are walked by the reference walk: in a ground sphere's scene every
-// such box would hold every small sphere (484 spheres of 0.2 on one of 1,000:
-// 486 objects a ray instead of 2.2 when all walks' boxes were widened so).
+// that, taken over the spheres with D <= |o| + |c| + r, which is a quadratic in
+// |o| (sphere_a and so on).  Rays for which this exceeds 2^-8 of the scene (tiny
+// spheres seen from far) are walked by the reference walk.  One bound from the
+// scene's size and the smallest radius would not do: beside a ground sphere of
+// 1,000 it widens every box past all 484 spheres of 0.2 on it (486 objects a
+// ray instead of 2.2).
 //
 // The slab tests above w: in the mesh, the triangle's own bounding box lies
 // inside every node above it (the build checks that, leaf_enclosed in
@@ -63,7 +64,7 @@ struct ExactView {
     const float4 *chain;       // per object slot: box minimum, box maximum
     float k;                   // A 2^-17
     float world_r, mesh_r;     // largest coordinates in world space and in any mesh's space
-    float sphere_k;            // 2^-19 / smallest radius, 0 without spheres
+    float sphere_a, sphere_b, sphere_c;  // 2^-19 (max 1/r, 2 max q/r, max q^2/r), 0 without spheres
     float max_origin;          // rays from farther out (1-norm) are left to the reference walk
     uint32_t on;               // 0: the scene needs the reference walk (see exact_view)
 };
@@ -72,8 +73,8 @@ constexpr float kBand = 1.00006103515625f;  // 1 + 2^-14
 
 AE_DEV float norm1(f3 v) { return fabsf(v.x) + fabsf(v.y) + fabsf(v.z); }
 AE_DEV float world_eps(const ExactView &X, f3 o) {
-    const float reach = norm1(o) + 2.0f * X.world_r;
-    return fmaf(X.sphere_k * reach, reach, 4.0f * X.k * (norm1(o) + X.world_r));
+    const float n = norm1(o);
+    return fmaf(fmaf(X.sphere_a, n, X.sphere_b), n, X.sphere_c) + 4.0f * X.k * (n + X.world_r);
 }
 AE_DEV f3 widening(float eps, f3 inv) { return eps * mk(fabsf(inv.x), fabsf(inv.y), fabsf(inv.z)); }
 // Components for which 1/d and its products with box distances stay finite

@@ -527,14 +527,20 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
                 F.static_range = std::max(F.static_range, std::max(std::fabs(boxes[s].lo[a]), std::fabs(boxes[s].hi[a])));
         }
     }
-    // For the exact walks' widening: the smallest sphere (0 for a radius that
-    // is no positive number) and the shape factor of the planar objects that
-    // the reference test can accept.
-    F.sphere_min = 3.402823466e38f;
+    // For the exact walks' widening: the spheres (a radius that is no positive
+    // number leaves no finite bound) and the shape factor of the planar objects
+    // that the reference test can accept.
+    for (double &x : F.sphere) x = 0.0;
     F.planar_factor = 1.0f;
     for (uint32_t s = 0; s < n; s++) {
         const ae_object &o = c->host_objects[s];
-        if (o.shapeType == AE_SHAPE_SPHERE) F.sphere_min = std::min(F.sphere_min, o.radius > 0.0f ? o.radius : 0.0f);
+        if (o.shapeType == AE_SHAPE_SPHERE) {
+            const double r = o.radius > 0.0f ? double(o.radius) : 0.0;
+            const double q = std::sqrt(double(o.x) * o.x + double(o.y) * o.y + double(o.z) * o.z) + r;
+            const double bound[3] = {1.0 / r, q / r, q * q / r};
+            for (int k = 0; k < 3; k++)
+                if (!(bound[k] <= F.sphere[k])) F.sphere[k] = bound[k];  // a NaN too
+        }
         if (o.shapeType != AE_SHAPE_QUAD && o.shapeType != AE_SHAPE_TRIANGLE) continue;
         const f3 u = mk(o.u_x, o.u_y, o.u_z), v = mk(o.v_x, o.v_y, o.v_z), nn = cross(u, v);
         const float n2 = dot(nn, nn);
@@ -923,15 +929,16 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
     X.world_r = F.range;
     X.mesh_r = F.mesh_range;
     X.max_origin = 3.0e38f;
-    if (F.sphere_min < 3.402823466e38f) {
+    if (F.sphere[0] != 0.0) {
         // Origins for which the spheres' widening stays below 2^-8 of the
-        // scene; none, and no exact walk, where even the scene's own reach
-        // asks for more.
-        const double k = std::ldexp(1.0, -19) / double(F.sphere_min), r = double(F.range);
-        const double reach = std::sqrt(std::ldexp(r, -8) / k);
-        if (!(reach > 2.0 * r)) return X;
-        X.sphere_k = float(k);
-        X.max_origin = float(std::min(reach - 2.0 * r, 3.0e38));
+        // scene; no exact walk where there is none.
+        const double a = std::ldexp(F.sphere[0], -19), b = std::ldexp(F.sphere[1], -19), q = std::ldexp(F.sphere[2], -19);
+        const double most = (std::sqrt(b * b + a * (std::ldexp(double(F.range), -8) - q)) - b) / a;
+        if (!(most > 0.0 && a < 1e30 && b < 1e30)) return X;
+        X.sphere_a = float(a);
+        X.sphere_b = float(2.0 * b);
+        X.sphere_c = float(q);
+        X.max_origin = float(std::min(most, 3.0e38));
     }
     X.on = 1;
     return X;

@@ -127,7 +127,7 @@ struct FastScene {
     // intersection of the reference TLAS boxes above it.
     float tri_factor = 1.0f, planar_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
     bool loose_trees = false;  // a triangle reaches out of a box above it in its tree
-    float sphere_min = 3.402823466e38f;  // smallest radius
+    double sphere[3] = {};     // largest 1/r, q/r and q^2/r over the spheres, q = |centre| + r
     uint2 nan_ref = {0xffffffffu, 0xffffffffu}, nan_wt = {0xffffffffu, 0xffffffffu};
     DevBuf<float4> obj_chain;
     DevBuf<int32_t> tlas_parent;
