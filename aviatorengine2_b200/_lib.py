@@ -92,6 +92,7 @@ POLICY_REQUEST, POLICY_MOVE, POLICY_CANCEL = 0, 1, 2
 CLAIM_OLDEST_FIRST, CLAIM_SHARED = 0, 1
 STATUS = {0: "AE_OK", -1: "AE_ERR_INVALID", -2: "AE_ERR_OOM", -3: "AE_ERR_OVERSIZE", -4: "AE_ERR_LAYOUT",
           -5: "AE_ERR_CUDA", -6: "AE_ERR_TIMEOUT", -7: "AE_ERR_STATE", -8: "AE_ERR_REJECTED", -9: "AE_ERR_CANCELLED"}
+PLAIN_WALK_AUTO, PLAIN_WALK_PREPARED, PLAIN_WALK_REFERENCE = 0, 1, 2
 FAULT_TILE_WAIT = 1
 FAULT_CHECK_LIMITS = 2
 CHECK_STACK, CHECK_INDEX = 1, 2
@@ -153,6 +154,8 @@ SIGNATURES = {
     "ae_stream": (_P, [_P]),
     "ae_launch_count": (ctypes.c_uint64, [_P]),
     "ae_prepare_fast": (_I, [_P]),
+    "ae_set_plain_walk": (_I, [_P, _I]),
+    "ae_plain_walk_used": (_I, [_P, _P]),
     "ae_refit_instances": (_I, [_P, _P, _U32]),
     "ae_rebuild_scene": (_I, [_P, _P, _U32, _P]),
     "ae_scene_sizes": (_I, [_P, _P, _P, _P, _P]),

@@ -492,6 +492,22 @@ int ae_debug_inject(ae_ctx *ctx, int fault, uint32_t on) {
     return AE_OK;
 }
 
+int ae_set_plain_walk(ae_ctx *ctx, int mode) {
+    Ctx *c = reinterpret_cast<Ctx *>(ctx);
+    if (!c) return AE_ERR_INVALID;
+    if (mode != AE_PLAIN_WALK_AUTO && mode != AE_PLAIN_WALK_PREPARED && mode != AE_PLAIN_WALK_REFERENCE)
+        return c->fail(AE_ERR_INVALID, "unknown plain walk %d", mode);
+    c->plain_walk = mode;
+    return AE_OK;
+}
+
+int ae_plain_walk_used(const ae_ctx *ctx, int32_t *on_structures) {
+    const Ctx *c = reinterpret_cast<const Ctx *>(ctx);
+    if (!c || !on_structures) return AE_ERR_INVALID;
+    *on_structures = c->plain_exact ? 1 : 0;
+    return AE_OK;
+}
+
 int ae_debug_flags(ae_ctx *ctx, uint32_t *flags) {
     Ctx *c = reinterpret_cast<Ctx *>(ctx);
     if (!c || !flags) return AE_ERR_INVALID;

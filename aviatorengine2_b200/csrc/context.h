@@ -121,6 +121,8 @@ struct Ctx {
     // changed, and the scene that they could not be built for.
     uint64_t plain_scene = ~0ull, plain_geometry = ~0ull, plain_scene_rays = 0, plain_geometry_rays = 0;
     uint64_t exact_refused = ~0ull;
+    int plain_walk = AE_PLAIN_WALK_AUTO;
+    bool plain_exact = false;  // the last plain form traced on the structures
     uint64_t fast_accepted = ~0ull;  // scene_version that prepare_fast last accepted
     Wavefront *wave = nullptr;
     Deferred *deferred = nullptr;

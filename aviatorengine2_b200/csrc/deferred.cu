@@ -958,7 +958,10 @@ static DefParams make_def_params(const Ctx *c) {
 // 229 us; 5 objects with 160 triangles 44 + 201 against 35 + 114 us; 17 with
 // 160 73 + 410 against 75 + 245 us).
 static ExactView hybrid_view(Ctx *c, uint64_t rays) {
-    if (c->n_objects < 16 && c->scene_triangles < 128) return ExactView{};
+    if (c->n_objects < 16 && c->scene_triangles < 128) {
+        c->plain_exact = false;
+        return ExactView{};
+    }
     return exact_view(c, rays);
 }
 

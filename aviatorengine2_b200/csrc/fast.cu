@@ -890,9 +890,12 @@ int prepare_fast(Ctx *c) {
 ExactView exact_view(Ctx *c, uint64_t rays) {
     ExactView X;
     std::memset(&X, 0, sizeof(X));
+    c->plain_exact = false;
+    if (c->plain_walk == AE_PLAIN_WALK_REFERENCE) return X;
     if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0 || c->exact_refused == c->scene_version) return X;
     const bool built = c->fast && c->fast->geometry_key == c->geometry_version && !c->fast->geometry_dirty;
     if (!built || c->fast->scene_key != c->scene_version) {
+        if (c->plain_walk != AE_PLAIN_WALK_AUTO) return X;
         if (c->plain_scene != c->scene_version) c->plain_scene_rays = 0;
         if (c->plain_geometry != c->geometry_version) c->plain_geometry_rays = 0;
         c->plain_scene = c->scene_version;
@@ -905,6 +908,11 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
                             : moved  ? 1.0e5 + 100.0 * objects
                                      : 2.0e5 + 1500.0 * objects;
         if (saved < cost) return X;
+        // A build allocates and synchronises, which a stream that is being
+        // captured does not allow.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) cudaGetLastError();
+        if (capture != cudaStreamCaptureStatusNone) return X;
     }
     // What the caller asked for is not an optimised form: a failure here is
     // not its failure, and ae_closest_hit_noalloc still wants its own
@@ -912,7 +920,12 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
     const bool ready = c->fast_ready;
     const uint64_t accepted = c->fast_accepted;
     std::string err = c->err;
+    // Another stream of this thread may be under capture, which a global-mode
+    // capture would let the allocations break.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     const int rc = prepare_fast(c);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     c->fast_ready = ready;
     c->fast_accepted = accepted;
     c->err.swap(err);
@@ -941,6 +954,7 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
         X.max_origin = float(std::min(most, 3.0e38));
     }
     X.on = 1;
+    c->plain_exact = true;
     return X;
 }
 

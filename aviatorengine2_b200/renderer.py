@@ -220,6 +220,17 @@ class Context:
         self._chk(lib().ae_wavefront_set_walk_runs(self._h, 1 if precision else 0, shadow_run, extend_run,
                                                    shadow_blocks, extend_blocks))
 
+    def set_plain_walk(self, mode):
+        """Which walk compute-only frames, the hybrid passes and any hit take
+        (PLAIN_WALK_*; ae_set_plain_walk)."""
+        self._chk(lib().ae_set_plain_walk(self._h, mode))
+
+    def plain_walk_used(self):
+        """Whether the last such call traced on the optimised structures."""
+        v = ctypes.c_int32()
+        self._chk(lib().ae_plain_walk_used(self._h, ctypes.byref(v)))
+        return bool(v.value)
+
     def image_error(self, reference, which=_lib.IMAGE_ACCUM, eps=1e-3):
         """FP64 error of an image against a reference (H, W, 4) float64 image,
         reduced on the GPU: (mean relative, mean absolute, max absolute, rms)."""

@@ -442,7 +442,10 @@ typedef struct ae_gbuffer {
 /* One dispatch: the compute-only megakernel (hybrid:1328-1404), or the
  * deferred resolve (deferred:1879-2010) followed by the temporal upsample
  * (upsample:280-390) when config.traceScale < 1, or the wavefront path
- * tracer.  Uses the config set by ae_set_config (batch/frameIndex included). */
+ * tracer.  Uses the config set by ae_set_config (batch/frameIndex included).
+ * The compute-only form is one launch on the context's stream, except that a
+ * call may first build the optimised structures (ae_set_plain_walk says when,
+ * and how to rule it out). */
 int ae_render_frame(ae_ctx *ctx, int mode, const ae_gbuffer *gbuffer);
 
 /* Produce the G-buffer on the device by ray casting the primary hit with the
@@ -593,6 +596,27 @@ int ae_rebuild_scene(ae_ctx *ctx, const ae_entity *entities, uint32_t n, const a
  * (replaces the per-frame CPU rebuild of renderer/renderer.cpp:1087-1130
  * when only transforms changed). */
 int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uint32_t n);
+
+/* Which walk the plain forms' traversals take: compute-only frames, G-buffer
+ * and deferred resolve, any hit.  The answers are the same bit for bit; what
+ * differs is time, memory and what a call may do.
+ *   AE_PLAIN_WALK_AUTO (a new context's): on the optimised structures where
+ *     they are current, and a call builds them once the rays traced without
+ *     them would have paid for it.  That call allocates and waits for the
+ *     context's stream; no call builds while that stream is being captured.
+ *   AE_PLAIN_WALK_PREPARED: on the structures where they are current
+ *     (ae_prepare_fast, or an optimised form's call, after the last upload or
+ *     refit), on the reference walk otherwise.  Compute-only frames then
+ *     neither allocate nor wait.
+ *   AE_PLAIN_WALK_REFERENCE: always the reference walk.
+ * Participating media, spheres that move within a frame, rotations off unit
+ * length and trees whose boxes do not hold their triangles take the reference
+ * walk in every mode.  No counterpart in the reference. */
+enum { AE_PLAIN_WALK_AUTO = 0, AE_PLAIN_WALK_PREPARED = 1, AE_PLAIN_WALK_REFERENCE = 2 };
+int ae_set_plain_walk(ae_ctx *ctx, int mode);
+/* 1 when the context's last plain-form call traced on the optimised
+ * structures, 0 when it took the reference walk (or traced nothing). */
+int ae_plain_walk_used(const ae_ctx *ctx, int32_t *on_structures);
 
 /* Copies of the device's per-frame arrays as the kernels see them (after any
  * refit): objects, TLAS nodes, instances, each sized as last uploaded.  Null
