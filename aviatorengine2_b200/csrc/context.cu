@@ -530,8 +530,9 @@ int ae_render_frame(ae_ctx *ctx, int mode, const ae_gbuffer *gb) {
     switch (mode) {
     case AE_MODE_COMPUTE_ONLY:
         if ((rc = c->timed_begin())) return rc;
-        if ((rc = c->cuda(launch_render_plain(c->scene(), exact_view(c, uint64_t(F.width) * F.height * F.spp), F, c->accum.ptr,
-                                             c->display.ptr, c->frame.ptr, c->stream),
+        if ((rc = c->cuda(launch_render_plain(c->scene(),
+                                             exact_view(c, F.display_only ? 0 : uint64_t(F.width) * F.height * F.spp), F,
+                                             c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
                           "render (compute-only)")))
             return rc;
         return c->timed_end();

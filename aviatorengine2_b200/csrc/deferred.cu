@@ -958,11 +958,8 @@ static DefParams make_def_params(const Ctx *c) {
 // 229 us; 5 objects with 160 triangles 44 + 201 against 35 + 114 us; 17 with
 // 160 73 + 410 against 75 + 245 us).
 static ExactView hybrid_view(Ctx *c, uint64_t rays) {
-    if (c->n_objects < 16 && c->scene_triangles < 128) {
-        c->plain_exact = false;
-        return ExactView{};
-    }
-    return exact_view(c, rays);
+    const bool small = c->n_objects < 16 && c->scene_triangles < 128;
+    return exact_view(c, small ? 0 : rays);
 }
 
 int render_deferred(Ctx *c, const ae_gbuffer *gb) {
@@ -1002,7 +999,7 @@ int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     if ((rc = c->timed_begin())) return rc;
     if (!(P.reduced && P.F.display_only)) {
         dim3 grid((P.ext_w + 15) / 16, (P.ext_h + 7) / 8);
-        const ExactView X = P.F.display_only ? ExactView{} : hybrid_view(c, uint64_t(P.ext_w) * P.ext_h * P.spp);
+        const ExactView X = hybrid_view(c, P.F.display_only ? 0 : uint64_t(P.ext_w) * P.ext_h * P.spp);
         if (X.on) k_deferred<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), c->stream>>>(c->scene(), X, P, G, I);
         else k_deferred<false><<<grid, 128, 0, c->stream>>>(c->scene(), X, P, G, I);
         if ((rc = c->cuda(cudaGetLastError(), "deferred launch"))) return rc;

@@ -873,7 +873,8 @@ int prepare_fast(Ctx *c) {
 }
 
 // The exact walks' view of the scene (exact_trace.cuh) for a frame or batch of
-// `rays` starting rays; off where the plain walks have to answer: participating
+// `rays` starting rays; off for a call that traces none (a frame that only
+// grades its image again) and where the plain walks have to answer: participating
 // media (they draw random numbers in visit order), spheres that move within a
 // frame (their boxes hold one position), rotations that are not of unit length
 // (unit_rotations), triangles so thin that the widening would swallow the
@@ -891,7 +892,7 @@ ExactView exact_view(Ctx *c, uint64_t rays) {
     ExactView X;
     std::memset(&X, 0, sizeof(X));
     c->plain_exact = false;
-    if (c->plain_walk == AE_PLAIN_WALK_REFERENCE) return X;
+    if (rays == 0 || c->plain_walk == AE_PLAIN_WALK_REFERENCE) return X;
     if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0 || c->exact_refused == c->scene_version) return X;
     const bool built = c->fast && c->fast->geometry_key == c->geometry_version && !c->fast->geometry_dirty;
     if (!built || c->fast->scene_key != c->scene_version) {

@@ -402,7 +402,7 @@ cudaError_t launch_count_paths(const DevScene &S, const FrameParams &F, unsigned
 cudaError_t launch_render_plain(const DevScene &S, const ExactView &X, const FrameParams &F, float4 *accum,
                                 uchar4 *display, float4 *frame, cudaStream_t st) {
     dim3 grid((F.width + 15) / 16, (F.height + 7) / 8);
-    if (X.on && !F.display_only)
+    if (X.on)
         k_render_plain<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), st>>>(S, X, F, accum, display, frame);
     else
         k_render_plain<false><<<grid, 128, 0, st>>>(S, X, F, accum, display, frame);

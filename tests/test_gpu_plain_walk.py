@@ -152,3 +152,22 @@ def test_capture():
         ctx.render_frame(L.MODE_COMPUTE_ONLY)
         assert ctx.plain_walk_used()
         del heavy, light
+
+
+def test_display_only_frames_trace_nothing():
+    """Grading an image again builds no structures, however large the image,
+    and does not count towards the build of a later frame."""
+    s = field()
+    with Context(1024, 1024) as ctx:
+        ctx.upload(s)
+        cfg = ctx.get_config().copy()
+        cfg["samples"], cfg["displayOnly"] = 8, 1
+        ctx.set_config(cfg)
+        live = L.lib().ae_debug_live_allocations()
+        for _ in range(4):
+            ctx.render_frame(L.MODE_COMPUTE_ONLY)
+        assert L.lib().ae_debug_live_allocations() == live and not ctx.plain_walk_used()
+        rays = np.zeros(64, L.RAY)
+        rays["dx"], rays["tnear"] = 1.0, 0.001
+        ctx.any_hit(rays, np.ones(64, np.float32))
+        assert not ctx.plain_walk_used()
