@@ -542,7 +542,7 @@ int ae_render_frame(ae_ctx *ctx, int mode, const ae_gbuffer *gb) {
     case AE_MODE_COMPUTE_ONLY:
     {
         // The view first: building its structures is not the frame's kernel time.
-        const ExactView X = exact_view(c, F.display_only ? 0 : uint64_t(F.width) * F.height * F.spp);
+        const ExactView X = exact_view(c, kPlainCompute, F.display_only ? 0 : uint64_t(F.width) * F.height * F.spp);
         if ((rc = c->timed_begin())) return rc;
         if ((rc = c->cuda(launch_render_plain(c->scene(), X, F, c->accum.ptr, c->display.ptr, c->frame.ptr, c->stream),
                           "render (compute-only)")))

@@ -121,9 +121,11 @@ struct Ctx {
     // Optimised forms.
     FastScene *fast = nullptr;
     bool fast_ready = false;
-    // exact_view: rays traced without structures since the scene or the geometry
-    // changed, and the scene that they could not be built for.
-    uint64_t plain_scene = ~0ull, plain_geometry = ~0ull, plain_scene_rays = 0, plain_geometry_rays = 0;
+    // exact_view: nanoseconds that structures would have saved the calls without
+    // them since the scene or the geometry changed, and the scene that they could
+    // not be built for.
+    uint64_t plain_scene = ~0ull, plain_geometry = ~0ull;
+    double plain_scene_ns = 0.0, plain_geometry_ns = 0.0;
     uint64_t exact_refused = ~0ull;
     int plain_walk = AE_PLAIN_WALK_AUTO;
     bool plain_exact = false;  // the last plain form traced on the structures

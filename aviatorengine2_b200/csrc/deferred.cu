@@ -952,16 +952,6 @@ static DefParams make_def_params(const Ctx *c) {
     return P;
 }
 
-// The hybrid passes on a handful of objects with a handful of triangles: the
-// reference walk is as short there, and has nothing to verify (480x270, G-buffer
-// and resolve: Cornell box, 8 objects and 34 triangles, 28 + 188 against 34 +
-// 229 us; 5 objects with 160 triangles 44 + 201 against 35 + 114 us; 17 with
-// 160 73 + 410 against 75 + 245 us).
-static ExactView hybrid_view(Ctx *c, uint64_t rays) {
-    const bool small = c->n_objects < 16 && c->scene_triangles < 128;
-    return exact_view(c, small ? 0 : rays);
-}
-
 int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     int rc = ensure(c);
     if (rc) return rc;
@@ -997,7 +987,7 @@ int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     Images I{D.accum[wslot].ptr, D.geom[wslot].ptr, D.reduced.ptr, D.accum[rslot].ptr, D.geom[rslot].ptr,
              c->display.ptr};
     // Before the timed part: building structures is not the frame's kernel time.
-    const ExactView X = hybrid_view(c, P.F.display_only ? 0 : uint64_t(P.ext_w) * P.ext_h * P.spp);
+    const ExactView X = exact_view(c, kPlainHybrid, P.F.display_only ? 0 : uint64_t(P.ext_w) * P.ext_h * P.spp);
     if ((rc = c->timed_begin())) return rc;
     if (!(P.reduced && P.F.display_only)) {
         dim3 grid((P.ext_w + 15) / 16, (P.ext_h + 7) / 8);
@@ -1072,7 +1062,7 @@ extern "C" int ae_build_gbuffer(ae_ctx *ctx) {
     const DefParams P = make_def_params(c);
     GBuf G{D.gpos.ptr, D.gnrm.ptr, D.galb.ptr, D.gdepth.ptr};
     dim3 grid((P.F.width + 15) / 16, (P.F.height + 7) / 8);
-    const ExactView X = hybrid_view(c, uint64_t(P.F.width) * P.F.height);
+    const ExactView X = exact_view(c, kPlainHybrid, uint64_t(P.F.width) * P.F.height);
     if (X.on) k_gbuffer<true><<<grid, 128, size_t(kSharedStack) * 128 * sizeof(uint2), c->stream>>>(c->scene(), X, P, G);
     else k_gbuffer<false><<<grid, 128, 0, c->stream>>>(c->scene(), X, P, G);
     c->launches++;
@@ -1112,7 +1102,7 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
     for (size_t k = 0; k < std::min<size_t>(Ctx::kIoSlots, plan.size()); k++)
         if (c->io_rays[k].reserve(chunk) || c->io_bound[k].reserve(chunk) || c->io_blocked[k].reserve(chunk))
             return c->fail(AE_ERR_OOM, "any-hit buffers");
-    const ExactView X = exact_view(c, n);
+    const ExactView X = exact_view(c, kPlainAnyHit, n);
     int rc;
     if (plan.size() > 1 && (rc = ensure_side_streams(c))) return rc;
     if ((rc = ensure_chunk_events(c, plan.size()))) return rc;

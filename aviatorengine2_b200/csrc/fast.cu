@@ -881,33 +881,59 @@ int prepare_fast(Ctx *c) {
 // scene, uploaded trees whose boxes do not hold their triangles, or structures
 // that cannot be built.
 //
-// Structures that are not current are brought up to date once the rays that
-// the reference walk has traced without them (this call's included) would
-// have paid for it, so a scene that is asked little never pays, and one that
-// is asked much pays about once.  Against the reference walk a ray saves about
-// 5 ns (visibility segments 4.6); the build took 0.4 ms for the Cornell box, 2.4
-// ms for 260 objects of 250,000 triangles and 3.8 ms for 1,040 of 2M; a move
-// refreshes the instance tree alone.
-ExactView exact_view(Ctx *c, uint64_t rays) {
+// Structures that are not current are brought up to date once they would have
+// saved the calls made without them (this one included) what they cost, so a
+// scene that is asked little never pays, and one that is asked much pays about
+// once.  Both sides are times of whole calls on new scenes (means of three):
+//
+//   prepare, with its allocations and host work, ms: Cornell box 0.37, textured
+//   box (11 objects, 1,290 triangles) 0.46, 62,410 triangles in 64 instances
+//   1.8, 249,848 in 256 2.5, 523,270 in 200 2.4, 2.1M in 64 2.9, 2.0M in 1,024
+//   4.4;
+//   saved for each starting ray, ns: compute-only frames 18 (62,410 triangles,
+//   depth 4), 54 (249,848, depth 8), 14 (229,894, depth 2), 1.1 (textured box,
+//   depth 6), 0.35 (Cornell box, depth 8); hybrid frames, a ray each for
+//   G-buffer and resolve, 1.8 (249,848, 4 lights), 33 (2.0M, 16 lights), 0.6
+//   (17 objects of 160 triangles); any hit 5.2 (523,270), 3.2 (2.1M).
+//
+// On a handful of objects with a handful of triangles the reference walk is as
+// short and has nothing to verify: any hit 0.072 against 0.090 ms for 200,003
+// segments in the Cornell box, hybrid frames of 480x270 216 against 263 us (5
+// objects with 160 triangles 245 against 149 us).  AUTO leaves those calls to
+// it.  A move refreshes the instance tree alone.
+static double saved_ns(const Ctx *c, PlainForm form, bool small) {
+    const bool big = c->scene_triangles >= 10000;
+    const double depth = double(std::min(c->config.depth, 8u));
+    switch (form) {
+    case kPlainCompute: return small ? 0.3 : (big ? 5.0 : 0.15) * depth;
+    case kPlainHybrid: return big ? 0.4 * (1.0 + double(c->n_lights)) : 0.5;
+    default: return big ? 5.0 : 0.5;
+    }
+}
+static double build_ns(const Ctx *c) {
+    return 0.5e6 + (c->n_indices >= 30000 ? 1.4e6 : 0.0) + 1800.0 * double(c->n_objects) + 0.13 * double(c->n_indices);
+}
+ExactView exact_view(Ctx *c, PlainForm form, uint64_t rays) {
     ExactView X;
     std::memset(&X, 0, sizeof(X));
     c->plain_exact = false;
     if (rays == 0 || c->plain_walk == AE_PLAIN_WALK_REFERENCE) return X;
     if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0 || c->exact_refused == c->scene_version) return X;
+    const bool small = c->n_objects < 16 && c->scene_triangles < 128;
+    if (small && form != kPlainCompute && c->plain_walk == AE_PLAIN_WALK_AUTO) return X;
     const bool built = c->fast && c->fast->geometry_key == c->geometry_version && !c->fast->geometry_dirty;
     if (!built || c->fast->scene_key != c->scene_version) {
         if (c->plain_walk != AE_PLAIN_WALK_AUTO) return X;
-        if (c->plain_scene != c->scene_version) c->plain_scene_rays = 0;
-        if (c->plain_geometry != c->geometry_version) c->plain_geometry_rays = 0;
+        if (c->plain_scene != c->scene_version) c->plain_scene_ns = 0.0;
+        if (c->plain_geometry != c->geometry_version) c->plain_geometry_ns = 0.0;
         c->plain_scene = c->scene_version;
         c->plain_geometry = c->geometry_version;
-        c->plain_scene_rays += rays;
-        c->plain_geometry_rays += rays;
+        const double now = double(rays) * saved_ns(c, form, small);
+        c->plain_scene_ns += now;
+        c->plain_geometry_ns += now;
         const bool moved = built && c->fast->tlas_key == c->scene_version_layout;
-        const double objects = double(c->n_objects), saved = 5.0 * double(built ? c->plain_scene_rays : c->plain_geometry_rays);
-        const double cost = !built   ? 1.0e6 + 2000.0 * objects + 0.5 * double(c->n_indices)
-                            : moved  ? 1.0e5 + 100.0 * objects
-                                     : 2.0e5 + 1500.0 * objects;
+        const double objects = double(c->n_objects), saved = built ? c->plain_scene_ns : c->plain_geometry_ns;
+        const double cost = !built ? build_ns(c) : moved ? 1.0e5 + 100.0 * objects : 2.0e5 + 1500.0 * objects;
         if (saved < cost) return X;
         // A build allocates and synchronises, which a stream that is being
         // captured does not allow.

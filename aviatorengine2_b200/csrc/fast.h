@@ -9,7 +9,9 @@ int prepare_fast(Ctx *c);
 int build_mesh_structures(Ctx *c, FastScene &F);
 int prepare_precision(Ctx *c);
 struct ExactView;
-ExactView exact_view(Ctx *c, uint64_t rays);
+enum PlainForm { kPlainCompute, kPlainHybrid, kPlainAnyHit };
+// `rays`: the starting rays (paths) of the call; 0 for a call that traces none.
+ExactView exact_view(Ctx *c, PlainForm form, uint64_t rays);
 void destroy_fast(Ctx *c);
 cudaError_t launch_closest_fast(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, bool quant, cudaStream_t st);
 cudaError_t launch_closest_walk(Ctx *c, const ae_ray *rays, uint32_t n, ae_hit *hits, cudaStream_t st);

@@ -603,8 +603,9 @@ int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uint32_t n);
  * and deferred resolve, any hit.  The answers are the same bit for bit; what
  * differs is time, memory and what a call may do.
  *   AE_PLAIN_WALK_AUTO (a new context's): on the optimised structures where
- *     they are current, and a call builds them once the rays traced without
- *     them would have paid for it.  That call allocates and waits for the
+ *     they are current (any hit and the hybrid passes: unless the scene is a
+ *     handful of objects), and a call builds them once they would have saved
+ *     the calls before what they cost.  That call allocates and waits for the
  *     context's stream; no call builds while that stream is being captured.
  *   AE_PLAIN_WALK_PREPARED: on the structures where they are current
  *     (ae_prepare_fast, or an optimised form's call, after the last upload or

@@ -7,8 +7,7 @@ reference walk's answers."""
 import numpy as np
 import pytest
 
-from aviatorengine2_b200 import _lib, scenes
-from test_gpu_exact import both_any_hits
+from aviatorengine2_b200 import Context, _lib, scenes
 
 pytestmark = pytest.mark.gpu
 L = _lib
@@ -34,6 +33,17 @@ def finish(ents, lib, name):
 
 def small_mesh(lib, half=0.001, at=(0.0, 0.0, 0.0)):
     return scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, at, mesh=lib.add(*scenes.box_mesh((half,) * 3)))
+
+
+def both_any_hits(s, rays, tmax):
+    """(on the structures, by the reference walk)"""
+    out = []
+    for mode in (L.PLAIN_WALK_PREPARED, L.PLAIN_WALK_REFERENCE):
+        with scenes_context(s) as ctx:
+            ctx.prepare_fast()
+            ctx.set_plain_walk(mode)
+            out.append(ctx.any_hit(rays, tmax))
+    return out
 
 
 def agree(s, rays, tmax):
@@ -102,9 +112,9 @@ def test_refit_that_grows_the_scene():
 
 
 def scenes_context(s):
-    from aviatorengine2_b200 import Context
     ctx = Context(96, 64)
     ctx.upload(s)
+    ctx.set_plain_walk(L.PLAIN_WALK_PREPARED)
     return ctx
 
 

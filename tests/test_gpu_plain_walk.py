@@ -81,12 +81,12 @@ def test_scenes_for_the_reference_walk(scene):
     assert same(got, want)
 
 
-@pytest.mark.parametrize("scene", [field, boxes])
-def test_build_in_mid_sequence(scene):
+@pytest.mark.parametrize("scene,width,height,samples", [(field, 160, 120, 2), (boxes, 320, 240, 16)])
+def test_build_in_mid_sequence(scene, width, height, samples):
     """Frames before and after the call that builds."""
     s = scene()
-    want, _ = frames(s, 24, L.PLAIN_WALK_REFERENCE, width=320, height=240, samples=2, depth=5)
-    got, used = frames(s, 24, L.PLAIN_WALK_AUTO, width=320, height=240, samples=2, depth=5)
+    want, _ = frames(s, 6, L.PLAIN_WALK_REFERENCE, width=width, height=height, samples=samples, depth=5)
+    got, used = frames(s, 6, L.PLAIN_WALK_AUTO, width=width, height=height, samples=samples, depth=5)
     assert not used[0] and used[-1] and used == sorted(used)
     assert same(got, want)
 
@@ -171,3 +171,52 @@ def test_display_only_frames_trace_nothing():
         rays["dx"], rays["tnear"] = 1.0, 0.001
         ctx.any_hit(rays, np.ones(64, np.float32))
         assert not ctx.plain_walk_used()
+
+
+def test_small_scenes_stay_on_the_reference_walk():
+    """Any hit and the hybrid passes of a handful of objects, prepared or not;
+    PREPARED still takes the structures there."""
+    s = scenes.cornell_box()
+    rng = np.random.default_rng(3)
+    rays = np.zeros(300_000, L.RAY)
+    for x in "xyz":
+        rays["o" + x], rays["d" + x] = rng.uniform(1, 9, len(rays)), rng.normal(size=len(rays))
+    rays["tnear"] = 0.001
+    tmax = np.full(len(rays), 3.0, np.float32)
+    got = {}
+    for mode in (L.PLAIN_WALK_AUTO, L.PLAIN_WALK_PREPARED, L.PLAIN_WALK_REFERENCE):
+        with Context(96, 64, hybrid=True) as ctx:
+            ctx.upload(s)
+            ctx.prepare_fast()
+            ctx.set_plain_walk(mode)
+            got[mode] = ctx.any_hit(rays, tmax)
+            used = [ctx.plain_walk_used()]
+            ctx.build_gbuffer()
+            used.append(ctx.plain_walk_used())
+            ctx.render_frame(L.MODE_DEFERRED)
+            used.append(ctx.plain_walk_used())
+            assert used == [mode == L.PLAIN_WALK_PREPARED] * 3
+    assert all(np.array_equal(g, got[L.PLAIN_WALK_REFERENCE]) for g in got.values())
+
+
+def test_builds_when_it_pays():
+    """The first calls on new scenes: a large scene's compute-only frames build
+    at once or nearly, a small one's only after a score of frames, a few any-hit
+    rays never."""
+    big = scenes.wavefront_scene(seed=3, width=480, height=270, depth=8, n_meshes=8, n_instances=64, n_lights=4,
+                                 target_tris=60_000)
+    for s, w, h, first, last in ((big, 480, 270, 0, 1), (scenes.cornell_box(), 320, 240, 12, 40)):
+        with Context(w, h) as ctx:
+            ctx.upload(s)
+            used = []
+            for _ in range(last + 1):
+                ctx.render_frame(L.MODE_COMPUTE_ONLY)
+                used.append(ctx.plain_walk_used())
+            assert True in used and first <= used.index(True)
+    with Context(64, 48) as ctx:
+        ctx.upload(big)
+        rays = np.zeros(10_000, L.RAY)
+        rays["dx"], rays["tnear"] = 1.0, 0.001
+        for _ in range(5):
+            ctx.any_hit(rays, np.ones(len(rays), np.float32))
+            assert not ctx.plain_walk_used()
