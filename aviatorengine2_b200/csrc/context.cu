@@ -201,7 +201,7 @@ namespace {
 
 template <class T> int upload(Ctx *c, DevBuf<T> &buf, const T *src, size_t n, const char *what) {
     if (n == 0) return AE_OK;
-    int rc = buf.reserve(n);
+    int rc = reserve_or_spare(c, [&] { return buf.reserve(n); });
     if (rc != AE_OK) return c->fail(rc, "cudaMalloc(%s, %zu elements) failed", what, n);
     return c->cuda(cudaMemcpyAsync(buf.ptr, src, n * sizeof(T), cudaMemcpyHostToDevice, c->stream), what);
 }
@@ -655,7 +655,7 @@ int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, in
     const uint32_t chunk = *std::max_element(plan.begin(), plan.end());
     if (plan.size() > 1 && (rc = ensure_side_streams(c))) return rc;
     for (size_t k = 0; k < std::min<size_t>(Ctx::kIoSlots, plan.size()); k++)
-        if (c->io_rays[k].reserve(chunk) || c->io_hits[k].reserve(chunk))
+        if (reserve_or_spare(c, [&] { return c->io_rays[k].reserve(chunk) || c->io_hits[k].reserve(chunk) ? AE_ERR_OOM : AE_OK; }))
             return c->fail(AE_ERR_OOM, "staging allocation failed");
     cudaStream_t st[Ctx::kIoSlots] = {c->stream, c->side_stream, c->side_stream2};
     uint32_t off = 0;

@@ -142,6 +142,17 @@ struct Ctx {
     int timed_end();
 };
 
+// Memory that a context holds for speed alone and can do without: the second
+// set of light samples of the wavefront form.  Waits for the context's stream.
+// False when there is nothing to give back.
+bool release_spare(Ctx *c);
+// An allocation that may have that memory: reserve() once, and again after
+// giving it back if it failed with AE_ERR_OOM.
+template <class Reserve> int reserve_or_spare(Ctx *c, Reserve reserve) {
+    const int rc = reserve();
+    return rc == AE_ERR_OOM && release_spare(c) ? reserve() : rc;
+}
+
 // Implemented by the optimised-kernel translation units.
 std::vector<uint32_t> host_chunks(uint32_t n);
 bool unit_rotations(const ae_instance *inst, uint32_t n);

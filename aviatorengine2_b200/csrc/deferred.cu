@@ -912,8 +912,13 @@ static int ensure(Ctx *c) {
     if (!D) return c->fail(AE_ERR_OOM, "deferred state");
     const size_t px = size_t(c->settings.width) * c->settings.height;
     if (D->gpos.cap < px) {
-        if (D->gpos.reserve(px) || D->gnrm.reserve(px) || D->galb.reserve(px) || D->gdepth.reserve(px) ||
-            D->accum[0].reserve(px) || D->accum[1].reserve(px) || D->geom[0].reserve(px) || D->geom[1].reserve(px))
+        if (reserve_or_spare(c, [&] {
+                return D->gpos.reserve(px) || D->gnrm.reserve(px) || D->galb.reserve(px) || D->gdepth.reserve(px) ||
+                               D->accum[0].reserve(px) || D->accum[1].reserve(px) || D->geom[0].reserve(px) ||
+                               D->geom[1].reserve(px)
+                           ? AE_ERR_OOM
+                           : AE_OK;
+            }))
             return c->fail(AE_ERR_OOM, "deferred images");
         cudaMemsetAsync(D->gnrm.ptr, 0, px * sizeof(float4), c->stream);
         cudaMemsetAsync(D->gpos.ptr, 0, px * sizeof(float4), c->stream);
@@ -974,7 +979,7 @@ int render_deferred(Ctx *c, const ae_gbuffer *gb) {
     if (!D.have_gbuffer) return c->fail(AE_ERR_STATE, "deferred resolve without a G-buffer (ae_build_gbuffer)");
     if (P.reduced) {
         const size_t rn = size_t(P.ext_w) * P.ext_h;
-        if (D.reduced.reserve(rn)) return c->fail(AE_ERR_OOM, "reduced grid");
+        if (reserve_or_spare(c, [&] { return D.reduced.reserve(rn); })) return c->fail(AE_ERR_OOM, "reduced grid");
         D.red_w = P.ext_w;
         D.red_h = P.ext_h;
     }
@@ -1100,7 +1105,11 @@ extern "C" int ae_any_hit(ae_ctx *ctx, const ae_ray *rays, const float *tmax, ui
     const std::vector<uint32_t> plan = host_chunks(n);
     const uint32_t chunk = *std::max_element(plan.begin(), plan.end());
     for (size_t k = 0; k < std::min<size_t>(Ctx::kIoSlots, plan.size()); k++)
-        if (c->io_rays[k].reserve(chunk) || c->io_bound[k].reserve(chunk) || c->io_blocked[k].reserve(chunk))
+        if (reserve_or_spare(c, [&] {
+                return c->io_rays[k].reserve(chunk) || c->io_bound[k].reserve(chunk) || c->io_blocked[k].reserve(chunk)
+                           ? AE_ERR_OOM
+                           : AE_OK;
+            }))
             return c->fail(AE_ERR_OOM, "any-hit buffers");
     const ExactView X = exact_view(c, kPlainAnyHit, n);
     int rc;

@@ -33,7 +33,7 @@ int prepare_variant(Ctx *c, int variant) {
         return AE_OK;
     case AE_VARIANT_FAST:
     case AE_VARIANT_QUANT:
-    case AE_VARIANT_FAST_WALK: return prepare_fast(c);
+    case AE_VARIANT_FAST_WALK: return reserve_or_spare(c, [&] { return prepare_fast(c); });
     default: return c->fail(AE_ERR_INVALID, "unknown kernel variant %d", variant);
     }
 }
@@ -136,5 +136,5 @@ extern "C" int ae_path_counters(ae_ctx *ctx, uint64_t *counters) {
 extern "C" int ae_prepare_fast(ae_ctx *ctx) {
     ae::Ctx *c = reinterpret_cast<ae::Ctx *>(ctx);
     if (!c) return AE_ERR_INVALID;
-    return ae::prepare_fast(c);
+    return ae::reserve_or_spare(c, [&] { return ae::prepare_fast(c); });
 }

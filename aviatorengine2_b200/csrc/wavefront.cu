@@ -589,8 +589,37 @@ static WfView view_of(Ctx *c, uint32_t bounce = 0) {
     return W;
 }
 
+// Everything that has a copy for each set.
+static void release_sets(Wavefront &Wf) {
+    for (auto *x : {&Wf.pend, &Wf.sh_o, &Wf.sh_d, &Wf.sh_lp, &Wf.sh_c}) x->release();
+    for (auto *x : {&Wf.nee, &Wf.sh_valid, &Wf.sh_occ}) x->release();
+    for (auto *x : {&Wf.qpid, &Wf.sq}) x->release();
+}
+static int reserve_sets(Wavefront &Wf, size_t k, size_t n, size_t ne) {
+    return Wf.qpid.reserve((k + 1) * n) || Wf.pend.reserve(k * n) || Wf.nee.reserve(k * n) || Wf.sh_o.reserve(k * ne) ||
+                   Wf.sh_d.reserve(k * ne) || Wf.sh_lp.reserve(k * ne) || Wf.sh_c.reserve(k * ne) ||
+                   Wf.sh_valid.reserve(k * ne) || Wf.sh_occ.reserve(k * ne) || Wf.sq.reserve(k * ne)
+               ? AE_ERR_OOM
+               : AE_OK;
+}
+
+bool release_spare(Ctx *c) {
+    Wavefront *Wf = c->wave;
+    if (!Wf || !Wf->cap || Wf->sets == 1) return false;
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return false;
+    if (Wf->graph) {
+        cudaGraphExecDestroy(Wf->graph);
+        Wf->graph = nullptr;
+    }
+    release_sets(*Wf);
+    Wf->sets = 1;
+    // One set fits where two were; if not, the next frame allocates it.
+    if (reserve_sets(*Wf, 1, Wf->cap, size_t(Wf->cap) * Wf->n_lights)) Wf->cap = 0;
+    return true;
+}
+
 static int ensure_wavefront(Ctx *c) {
-    int rc = prepare_fast(c);
+    int rc = reserve_or_spare(c, [&] { return prepare_fast(c); });
     if (rc) return rc;
     if (!c->wave) c->wave = new (std::nothrow) Wavefront();
     if (!c->wave) return c->fail(AE_ERR_OOM, "wavefront state");
@@ -602,20 +631,15 @@ static int ensure_wavefront(Ctx *c) {
     if (Wf.cap < n || Wf.n_lights < std::max(nl, 1u)) {
         const size_t ne = size_t(n) * std::max(nl, 1u);
         auto reserve = [&](size_t k) {
-            return Wf.qray[0].reserve(n) || Wf.qray[1].reserve(n) || Wf.qpid.reserve((k + 1) * n) || Wf.qhit.reserve(n) ||
-                   Wf.thr.reserve(n) || Wf.acc.reserve(n) || Wf.end.reserve(n) || Wf.col.reserve(n) ||
-                   Wf.pend.reserve(k * n) || Wf.seed.reserve(n) || Wf.nee.reserve(k * n) || Wf.sh_o.reserve(k * ne) ||
-                   Wf.sh_d.reserve(k * ne) || Wf.sh_lp.reserve(k * ne) || Wf.sh_c.reserve(k * ne) ||
-                   Wf.sh_valid.reserve(k * ne) || Wf.sh_occ.reserve(k * ne) || Wf.sq.reserve(k * ne) ||
-                   Wf.cnt.reserve(C_COUNT) || Wf.params.reserve(1);
+            return Wf.qray[0].reserve(n) || Wf.qray[1].reserve(n) || Wf.qhit.reserve(n) || Wf.thr.reserve(n) ||
+                   Wf.acc.reserve(n) || Wf.end.reserve(n) || Wf.col.reserve(n) || Wf.seed.reserve(n) ||
+                   reserve_sets(Wf, k, n, ne) || Wf.cnt.reserve(C_COUNT) || Wf.params.reserve(1);
         };
         // Short of memory, one set does: the shadow stages then follow one another.
         Wf.sets = kShadowSets;
         bool failed = reserve(Wf.sets);
         if (failed) {
-            for (auto *x : {&Wf.pend, &Wf.sh_o, &Wf.sh_d, &Wf.sh_lp, &Wf.sh_c}) x->release();
-            for (auto *x : {&Wf.nee, &Wf.sh_valid, &Wf.sh_occ}) x->release();
-            for (auto *x : {&Wf.qpid, &Wf.sq}) x->release();
+            release_sets(Wf);
             Wf.sets = 1;
             failed = reserve(1);
         }
@@ -861,9 +885,11 @@ int render_wavefront(Ctx *c, bool prec) {
     Wavefront &Wf = *c->wave;
     const uint32_t n_px = c->settings.width * c->settings.height;
     if (prec) {
-        if ((rc = prepare_precision(c))) return rc;
-        if (Wf.ksum.reserve(n_px) || Wf.kcomp.reserve(n_px))
+        if ((rc = reserve_or_spare(c, [&] { return prepare_precision(c); }))) return rc;
+        if (reserve_or_spare(c, [&] { return Wf.ksum.reserve(n_px) || Wf.kcomp.reserve(n_px) ? AE_ERR_OOM : AE_OK; }))
             return c->fail(AE_ERR_OOM, "compensated accumulation (%u pixels)", n_px);
+        // Given back by these, the queues may be gone.
+        if (!Wf.cap && (rc = ensure_wavefront(c))) return rc;
     }
     WfParams hp;
     std::memset(&hp, 0, sizeof(hp));
