@@ -911,7 +911,7 @@ static int ensure(Ctx *c) {
     Deferred *D = c->deferred;
     if (!D) return c->fail(AE_ERR_OOM, "deferred state");
     const size_t px = size_t(c->settings.width) * c->settings.height;
-    if (D->gpos.cap < px) {
+    if (D->geom[1].cap < px) {  // the last of them: all or none are there
         if (reserve_or_spare(c, [&] {
                 return D->gpos.reserve(px) || D->gnrm.reserve(px) || D->galb.reserve(px) || D->gdepth.reserve(px) ||
                                D->accum[0].reserve(px) || D->accum[1].reserve(px) || D->geom[0].reserve(px) ||

@@ -69,3 +69,28 @@ def test_allocation_after_the_queues(call):
         got = run(k)
         assert np.array_equal(got[0].view(np.uint8), want[0].view(np.uint8)), k
         assert np.array_equal(got[1].view(np.uint8), want[1].view(np.uint8)), k
+
+
+def test_hybrid_images_after_a_failed_allocation():
+    """A failed allocation of the hybrid images is an error of that call; the
+    next one allocates what is missing."""
+    s = scenes.hybrid_box(width=131, height=77, depth=3)
+
+    def frame(ctx):
+        ctx.build_gbuffer()
+        ctx.render_frame(L.MODE_DEFERRED)
+        return ctx.read_deferred_accum()
+
+    with Context(131, 77, hybrid=True) as ctx:
+        ctx.upload(s)
+        want = frame(ctx)
+    for k in range(8):
+        with Context(131, 77, hybrid=True) as ctx:
+            ctx.upload(s)
+            L.lib().ae_debug_fail_alloc_after(k)
+            try:
+                with pytest.raises(L.AeError):
+                    frame(ctx)
+            finally:
+                L.lib().ae_debug_fail_alloc_after(-1)
+            assert np.array_equal(frame(ctx), want), k
