@@ -236,20 +236,8 @@ std::string check_tree(const ae_bvh_node *nodes, uint64_t base, uint64_t limit_n
     return "";
 }
 
-int validate_scene(Ctx *c, const ae_object *objects, uint32_t n_objects, const ae_bvh_node *tlas, uint32_t n_nodes,
-                   const uint32_t *lights, uint32_t n_lights, const ae_instance *inst, uint32_t n_inst) {
-    if (n_nodes) {
-        const std::string e = check_tree(tlas, 0, n_nodes, n_objects, ae::kTlasStack);
-        if (!e.empty()) return c->fail(AE_ERR_LAYOUT, "TLAS: %s", e.c_str());
-    }
-    for (uint32_t i = 0; i < n_lights; i++)
-        if (lights[i] >= n_objects) return c->fail(AE_ERR_LAYOUT, "light %u -> object %u of %u", i, lights[i], n_objects);
-    for (uint32_t i = 0; i < n_objects; i++) {
-        const ae_object &o = objects[i];
-        if (o.shapeType > AE_SHAPE_MESH) return c->fail(AE_ERR_LAYOUT, "object %u has shape %u", i, o.shapeType);
-        if (o.shapeType == AE_SHAPE_MESH && o.instanceIndex >= n_inst)
-            return c->fail(AE_ERR_LAYOUT, "object %u -> instance %u of %u", i, o.instanceIndex, n_inst);
-    }
+// The instances' meshes against the uploaded geometry.
+int check_meshes(Ctx *c, const ae_instance *inst, uint32_t n_inst) {
     for (uint32_t i = 0; i < n_inst; i++) {
         const ae_instance &m = inst[i];
         const auto key = std::make_tuple(m.vertexBase, m.indexBase, m.triangleCount, m.blasBase);
@@ -270,7 +258,33 @@ int validate_scene(Ctx *c, const ae_object *objects, uint32_t n_objects, const a
     return AE_OK;
 }
 
+int validate_scene(Ctx *c, const ae_object *objects, uint32_t n_objects, const ae_bvh_node *tlas, uint32_t n_nodes,
+                   const uint32_t *lights, uint32_t n_lights, const ae_instance *inst, uint32_t n_inst) {
+    if (n_nodes) {
+        const std::string e = check_tree(tlas, 0, n_nodes, n_objects, ae::kTlasStack);
+        if (!e.empty()) return c->fail(AE_ERR_LAYOUT, "TLAS: %s", e.c_str());
+    }
+    for (uint32_t i = 0; i < n_lights; i++)
+        if (lights[i] >= n_objects) return c->fail(AE_ERR_LAYOUT, "light %u -> object %u of %u", i, lights[i], n_objects);
+    for (uint32_t i = 0; i < n_objects; i++) {
+        const ae_object &o = objects[i];
+        if (o.shapeType > AE_SHAPE_MESH) return c->fail(AE_ERR_LAYOUT, "object %u has shape %u", i, o.shapeType);
+        if (o.shapeType == AE_SHAPE_MESH && o.instanceIndex >= n_inst)
+            return c->fail(AE_ERR_LAYOUT, "object %u -> instance %u of %u", i, o.instanceIndex, n_inst);
+    }
+    return check_meshes(c, inst, n_inst);
+}
+
 }  // namespace
+
+namespace ae {
+int check_scene_meshes(Ctx *c) {
+    if (c->scene_geometry == c->geometry_version) return AE_OK;
+    const int rc = check_meshes(c, c->host_instances.data(), c->n_instances);
+    if (!rc) c->scene_geometry = c->geometry_version;
+    return rc;
+}
+}  // namespace ae
 
 extern "C" {
 
@@ -452,6 +466,7 @@ int ae_upload_scene(ae_ctx *ctx, const ae_object *objects, uint32_t n_objects, c
         if (o.shapeType == AE_SHAPE_SPHERE && !(o.x == o.x2 && o.y == o.y2 && o.z == o.z2)) c->scene_has_moving_spheres = true;
     }
     c->scene_rigid = unit_rotations(instances, n_instances);
+    c->scene_geometry = c->geometry_version;
     c->scene_uploaded = true;
     c->scene_version++;
     c->scene_version_layout++;

@@ -96,6 +96,7 @@ struct Ctx {
     DevBuf<uint32_t> check_word;      // AE_CHECK_* bits of the debug walk (ae_debug_flags)
     uint64_t scene_version = 0;         // bumps on every change of scene content
     uint64_t geometry_version = 0;      // bumps on every ae_upload_geometry
+    uint64_t scene_geometry = ~0ull;    // the one that the scene's meshes were checked against
     uint64_t scene_version_layout = 0;  // bumps when arrays are re-uploaded (topology may change)
     DevBuf<float> obj_box;              // world box per object (refit)
 
@@ -155,6 +156,9 @@ template <class Reserve> int reserve_or_spare(Ctx *c, Reserve reserve) {
 
 // Implemented by the optimised-kernel translation units.
 std::vector<uint32_t> host_chunks(uint32_t n);
+// The current scene's meshes against geometry uploaded after it: AE_ERR_LAYOUT
+// where they reach out of it.
+int check_scene_meshes(Ctx *c);
 bool unit_rotations(const ae_instance *inst, uint32_t n);
 int ensure_side_streams(Ctx *c);
 int ensure_chunk_events(Ctx *c, size_t chunks);

@@ -730,6 +730,9 @@ int prepare_fast(Ctx *c) {
     if (!c->fast) return c->fail(AE_ERR_OOM, "fast scene");
     FastScene &F = *c->fast;
     if (F.geometry_key != c->geometry_version) {
+        // The host's and the device's builders follow the instances' ranges and
+        // trees, which a geometry upload after the scene's may have changed.
+        if (const int bad = check_scene_meshes(c)) return bad;
         // New geometry arrays: every mesh is converted again (the device
         // buffers are reused).
         F.mesh_roots.clear();
