@@ -921,12 +921,12 @@ ExactView exact_view(Ctx *c, PlainForm form, uint64_t rays) {
     std::memset(&X, 0, sizeof(X));
     c->plain_exact = false;
     if (rays == 0 || c->plain_walk == AE_PLAIN_WALK_REFERENCE) return X;
-    if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0 || c->exact_refused == c->scene_version) return X;
+    if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0) return X;
     const bool small = c->n_objects < 16 && c->scene_triangles < 128;
     if (small && form != kPlainCompute && c->plain_walk == AE_PLAIN_WALK_AUTO) return X;
     const bool built = c->fast && c->fast->geometry_key == c->geometry_version && !c->fast->geometry_dirty;
     if (!built || c->fast->scene_key != c->scene_version) {
-        if (c->plain_walk != AE_PLAIN_WALK_AUTO) return X;
+        if (c->plain_walk != AE_PLAIN_WALK_AUTO || c->exact_refused == c->scene_version) return X;
         if (c->plain_scene != c->scene_version) c->plain_scene_ns = 0.0;
         if (c->plain_geometry != c->geometry_version) c->plain_geometry_ns = 0.0;
         c->plain_scene = c->scene_version;
@@ -960,7 +960,7 @@ ExactView exact_view(Ctx *c, PlainForm form, uint64_t rays) {
     c->fast_accepted = accepted;
     c->err.swap(err);
     if (rc) {
-        c->exact_refused = c->scene_version;  // until the scene changes
+        c->exact_refused = c->scene_version;  // not tried again until the scene changes or the caller prepares it
         return X;
     }
     const FastScene &F = *c->fast;

@@ -114,6 +114,37 @@ def test_prepared_mode_builds_nothing():
             ctx.set_plain_walk(3)
 
 
+def test_prepared_after_a_failed_build():
+    """A build that fails leaves its call to the reference walk and is not tried
+    again by itself; structures that the caller then prepares are used."""
+    s = field()
+    want, _ = frames(s, 3, L.PLAIN_WALK_REFERENCE, width=160, height=120, samples=2, depth=5)
+    with Context(160, 120, samples=2) as ctx:
+        ctx.upload(s)
+        cfg = ctx.get_config().copy()
+        cfg["samples"], cfg["depth"] = 2, 5
+        got, used = [], []
+        ctx.set_config(cfg)
+        ctx.render_frame(L.MODE_COMPUTE_ONLY)
+        # Pending until a call allocates, which is the one that builds.
+        L.lib().ae_debug_fail_alloc_after(0)
+        try:
+            for _ in range(30):
+                ctx.render_frame(L.MODE_COMPUTE_ONLY)
+                assert not ctx.plain_walk_used()
+        finally:
+            L.lib().ae_debug_fail_alloc_after(-1)
+        ctx.prepare_fast()
+        for k in range(3):
+            cfg["batch"] = k
+            ctx.set_config(cfg)
+            ctx.render_frame(L.MODE_COMPUTE_ONLY)
+            used.append(ctx.plain_walk_used())
+            got.append((ctx.read_image(L.IMAGE_ACCUM).view(np.uint8), ctx.read_image(L.IMAGE_DISPLAY)))
+    assert all(used)
+    assert same(got, want)
+
+
 def test_capture():
     """A compute-only frame recorded into a caller's graph on the context's
     stream, at the call that would build: it is recorded on the reference walk
