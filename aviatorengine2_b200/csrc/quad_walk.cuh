@@ -82,7 +82,10 @@ AE_DEV bool walk_quad(const DevScene &S, const FastView &V, f3 o, f3 d, float tn
                 have = false;
                 break;
             }
-            if (sp + hits - 1 > kQuadStack) return false;
+            if (sp + hits - 1 > kQuadStack) {
+                __syncwarp(quad);  // the lanes' pushes before the caller's walk takes the entries over
+                return false;
+            }
             if (t != none && rank > 0) stk[sp + hits - 1 - rank] = make_uint2(child, __float_as_uint(t));
             sp += hits - 1;
             const uint32_t first = __ballot_sync(quad, rank == 0) & quad;
