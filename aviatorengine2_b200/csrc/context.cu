@@ -639,7 +639,7 @@ int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, in
     }
     // A few rays from ordinary memory: through a small page-locked buffer that
     // the kernel reads and writes itself, one launch and no device copies (a
-    // 1,000-ray call: 44 -> 32 us).  Up to 4,096 rays the two host copies stay
+    // 1,000-ray call: 43-44 -> 32 us).  Up to 4,096 rays the two host copies stay
     // below what the driver's staged copies cost.
     if (n <= Ctx::kSmallRays && (variant == AE_VARIANT_FAST || variant == AE_VARIANT_QUANT || variant == AE_VARIANT_FAST_WALK)) {
         if (!c->small_io && cudaHostAlloc(&c->small_io, Ctx::kSmallRays * (sizeof(ae_ray) + sizeof(ae_hit)),
