@@ -169,12 +169,20 @@ int ensure_chunk_events(Ctx *c, size_t chunks) {
     return AE_OK;
 }
 
-// Whether every instance's quaternion has length 1 to 2^-18 in the square (a
-// normalised binary32 one is within 2^-21).  Then its conjugate, by which the
-// walks take a ray to the mesh, inverts the rotation by which the instance's
-// box was made to 2^-16 of the mesh's size, a quarter of the boxes' margin.
-bool unit_rotations(const ae_instance *inst, uint32_t n) {
+// Whether the exact walks may count on every instance's box.  Its quaternion
+// has length 1 to 2^-18 in the square (a normalised binary32 one is within
+// 2^-21); then its conjugate, by which the walks take a ray to the mesh, inverts
+// the rotation by which the box was made to 2^-16 of the mesh's size, a quarter
+// of the boxes' margin.  And its place and scale are numbers that the box and
+// the ray in the mesh's space can be computed from: one instance at infinity
+// takes the margin of all boxes with it, and a NaN passes the reference walk's
+// slab tests.
+bool plain_transforms(const ae_instance *inst, uint32_t n) {
     for (uint32_t i = 0; i < n; i++) {
+        const ae_instance &m = inst[i];
+        const float s = std::fabs(m.scale);
+        if (!(std::fabs(m.px) < kPlainReach && std::fabs(m.py) < kPlainReach && std::fabs(m.pz) < kPlainReach)) return false;
+        if (!(s == 0.0f || (s < kPlainReach && s > 1.0f / kPlainReach))) return false;
         const double x = inst[i].qx, y = inst[i].qy, z = inst[i].qz, w = inst[i].qw;
         if (!(std::fabs(x * x + y * y + z * z + w * w - 1.0) <= std::ldexp(1.0, -18))) return false;
     }
@@ -465,7 +473,7 @@ int ae_upload_scene(ae_ctx *ctx, const ae_object *objects, uint32_t n_objects, c
         if (o.colorType == AE_MAT_ISOTROPIC) c->scene_has_media = true;
         if (o.shapeType == AE_SHAPE_SPHERE && !(o.x == o.x2 && o.y == o.y2 && o.z == o.z2)) c->scene_has_moving_spheres = true;
     }
-    c->scene_rigid = unit_rotations(instances, n_instances);
+    c->scene_plain = plain_transforms(instances, n_instances);
     c->scene_geometry = c->geometry_version;
     c->scene_uploaded = true;
     c->scene_version++;

@@ -89,7 +89,7 @@ struct Ctx {
     bool scene_uploaded = false;
     uint64_t scene_triangles = 0;  // over all instances
     bool scene_has_media = false, scene_has_moving_spheres = false;
-    bool scene_rigid = true;  // unit_rotations of the current instances
+    bool scene_plain = true;  // plain_transforms of the current instances
     bool scene_has_ggx = false;  // an object uses AE_MAT_GGX_METAL (not shaded by the hybrid passes)
     uint32_t fault_tile_wait = 0;  // ae_debug_inject(AE_FAULT_TILE_WAIT)
     uint32_t fault_check_limits = 0;  // ae_debug_inject(AE_FAULT_CHECK_LIMITS)
@@ -159,7 +159,8 @@ std::vector<uint32_t> host_chunks(uint32_t n);
 // The current scene's meshes against geometry uploaded after it: AE_ERR_LAYOUT
 // where they reach out of it.
 int check_scene_meshes(Ctx *c);
-bool unit_rotations(const ae_instance *inst, uint32_t n);
+constexpr float kPlainReach = 1e15f;  // coordinates beyond this may overflow in the walks
+bool plain_transforms(const ae_instance *inst, uint32_t n);
 int ensure_side_streams(Ctx *c);
 int ensure_chunk_events(Ctx *c, size_t chunks);
 int prepare_variant(Ctx *c, int variant);

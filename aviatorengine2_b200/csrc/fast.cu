@@ -64,6 +64,12 @@ struct Box {
 };
 static_assert(sizeof(Box) == 24, "the device's boxes");
 Box node_box(const ae_bvh_node &n) { return Box{{n.min_x, n.min_y, n.min_z}, {n.max_x, n.max_y, n.max_z}}; }
+// Not inside out, and no coordinate beyond `reach`, infinite or NaN.
+bool box_within(const Box &b, float reach) {
+    for (int a = 0; a < 3; a++)
+        if (!(b.lo[a] <= b.hi[a] && b.lo[a] > -reach && b.hi[a] < reach)) return false;
+    return true;
+}
 float half_area(const Box &b) {
     const float dx = b.hi[0] - b.lo[0], dy = b.hi[1] - b.lo[1], dz = b.hi[2] - b.lo[2];
     return dx * dy + dy * dz + dz * dx;
@@ -523,8 +529,10 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
             const ae_aabb b = analytic_box(o);
             boxes[s] = Box{{b.min_x, b.min_y, b.min_z}, {b.max_x, b.max_y, b.max_z}};
             std::memcpy(&stat[6 * size_t(s)], &b, 24);
+            // One object at infinity would take the margin of all boxes with it.
             for (int a = 0; a < 3; a++)
-                F.static_range = std::max(F.static_range, std::max(std::fabs(boxes[s].lo[a]), std::fabs(boxes[s].hi[a])));
+                for (const float x : {std::fabs(boxes[s].lo[a]), std::fabs(boxes[s].hi[a])})
+                    if (std::isfinite(x)) F.static_range = std::max(F.static_range, x);
         }
     }
     // For the exact walks' widening: the spheres (a radius that is no positive
@@ -532,8 +540,18 @@ static int build_instance_tree(Ctx *c, FastScene &F) {
     // that the reference test can accept.
     for (double &x : F.sphere) x = 0.0;
     F.planar_factor = 1.0f;
+    F.odd_boxes = false;
     for (uint32_t s = 0; s < n; s++) {
         const ae_object &o = c->host_objects[s];
+        // The reference walk hits a box of negative half extents, and objects
+        // whose NaN passes its slab tests; neither has a box in the tree.  The
+        // walks reduce a yaw in binary32, to 2^-24 of the angle: up to 100
+        // radians a tenth of the boxes' margin.  (Meshes: plain_transforms.)
+        if (o.shapeType != AE_SHAPE_MESH && !box_within(boxes[s], kPlainReach)) F.odd_boxes = true;
+        // The object tree's buckets and the collapse need numbers; where such an
+        // object lies in the tree does not matter.
+        if (!box_within(boxes[s], 1e30f)) boxes[s] = Box{};
+        if (o.shapeType == AE_SHAPE_BOX && !(std::fabs(o.rotation) < 100.0f)) F.odd_boxes = true;
         if (o.shapeType == AE_SHAPE_SPHERE) {
             const double r = o.radius > 0.0f ? double(o.radius) : 0.0;
             const double q = std::sqrt(double(o.x) * o.x + double(o.y) * o.y + double(o.z) * o.z) + r;
@@ -622,7 +640,7 @@ static int refresh_instance_tree(Ctx *c, FastScene &F) {
             const float sc = (m.scale != 0.0f && m.scale != 1.0f) ? std::fabs(m.scale) : 1.0f;
             const float r = std::max(std::fabs(m.px), std::max(std::fabs(m.py), std::fabs(m.pz))) +
                             1.75f * sc * F.inst_radius[o.instanceIndex];
-            range = std::max(range, r);
+            if (std::isfinite(r)) range = std::max(range, r);
         }
     }
     range = std::max(range, F.static_range);
@@ -880,9 +898,10 @@ int prepare_fast(Ctx *c) {
 // grades its image again) and where the plain walks have to answer: participating
 // media (they draw random numbers in visit order), spheres that move within a
 // frame (their boxes hold one position), rotations that are not of unit length
-// (unit_rotations), triangles so thin that the widening would swallow the
-// scene, uploaded trees whose boxes do not hold their triangles, or structures
-// that cannot be built.
+// and transforms that are no plain numbers (plain_transforms), objects without
+// a box that holds them (odd_boxes), triangles so thin that the widening would
+// swallow the scene, uploaded trees whose boxes do not hold their triangles, or
+// structures that cannot be built.
 //
 // Structures that are not current are brought up to date once they would have
 // saved the calls made without them (this one included) what they cost, so a
@@ -921,7 +940,7 @@ ExactView exact_view(Ctx *c, PlainForm form, uint64_t rays) {
     std::memset(&X, 0, sizeof(X));
     c->plain_exact = false;
     if (rays == 0 || c->plain_walk == AE_PLAIN_WALK_REFERENCE) return X;
-    if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_rigid || c->n_nodes == 0) return X;
+    if (c->scene_has_media || c->scene_has_moving_spheres || !c->scene_plain || c->n_nodes == 0) return X;
     const bool small = c->n_objects < 16 && c->scene_triangles < 128;
     if (small && form != kPlainCompute && c->plain_walk == AE_PLAIN_WALK_AUTO) return X;
     const bool built = c->fast && c->fast->geometry_key == c->geometry_version && !c->fast->geometry_dirty;
@@ -965,7 +984,7 @@ ExactView exact_view(Ctx *c, PlainForm form, uint64_t rays) {
     }
     const FastScene &F = *c->fast;
     const float factor = std::max(F.tri_factor, F.planar_factor);
-    if (!(factor <= 4096.0f) || F.loose_trees) return X;
+    if (!(factor <= 4096.0f) || F.loose_trees || F.odd_boxes || !(F.mesh_range < kPlainReach)) return X;
     X.V = fast_view(F);
     X.chain = F.obj_chain.ptr;
     X.k = std::ldexp(factor, -17);

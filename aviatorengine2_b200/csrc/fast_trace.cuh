@@ -127,6 +127,7 @@ struct FastScene {
     // intersection of the reference TLAS boxes above it.
     float tri_factor = 1.0f, planar_factor = 1.0f, mesh_range = 0.0f, range = 1.0f;
     bool loose_trees = false;  // a triangle reaches out of a box above it in its tree
+    bool odd_boxes = false;    // an object has no box that is sure to hold it (build_instance_tree)
     double sphere[3] = {};     // largest 1/r, q/r and q^2/r over the spheres, q = |centre| + r
     uint2 nan_ref = {0xffffffffu, 0xffffffffu}, nan_wt = {0xffffffffu, 0xffffffffu};
     DevBuf<float4> obj_chain;

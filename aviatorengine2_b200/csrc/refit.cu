@@ -265,7 +265,7 @@ extern "C" int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uin
     if ((rc = c->timed_end())) return rc;
     // The optimised walk's instance records follow the new transforms.
     std::memcpy(c->host_instances.data(), instances, size_t(n) * sizeof(ae_instance));
-    c->scene_rigid = unit_rotations(instances, n);
+    c->scene_plain = plain_transforms(instances, n);
     c->scene_version++;
     return AE_OK;
 }

@@ -613,8 +613,9 @@ int ae_refit_instances(ae_ctx *ctx, const ae_instance *instances, uint32_t n);
  *     neither allocate nor wait.
  *   AE_PLAIN_WALK_REFERENCE: always the reference walk.
  * Participating media, spheres that move within a frame, rotations off unit
- * length and trees whose boxes do not hold their triangles take the reference
- * walk in every mode.  No counterpart in the reference. */
+ * length, transforms and objects that are infinite, NaN or inside out, and
+ * trees whose boxes do not hold their triangles take the reference walk in
+ * every mode.  No counterpart in the reference. */
 enum { AE_PLAIN_WALK_AUTO = 0, AE_PLAIN_WALK_PREPARED = 1, AE_PLAIN_WALK_REFERENCE = 2 };
 int ae_set_plain_walk(ae_ctx *ctx, int mode);
 /* 1 when the context's last plain-form call traced on the optimised

@@ -189,6 +189,69 @@ def test_quaternions_off_unit_length(norm):
     agree(s, rays, (dist * 2.0).astype(np.float32))
 
 
+@pytest.mark.parametrize("what", ["far", "nan place", "nan scale", "tiny scale", "quad", "nan quad", "box", "angle"])
+def test_transforms_that_are_no_plain_numbers(what):
+    """One instance or object at infinity, NaN, inside out or turned by many
+    radians: the reference walk goes on with the others, and hits the odd one
+    where its arithmetic says so."""
+    rng = np.random.default_rng(11)
+    lib = scenes.MeshLibrary()
+    ents = [scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (0, 0, 0), mesh=lib.add(*scenes.box_mesh((3, 3, 3)))),
+            scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (7, 0, 0), mesh=lib.add(*scenes.box_mesh((1, 2, 1)))),
+            scenes.entity(L.SHAPE_QUAD, L.MAT_LAMBERTIAN, (-8, -8, -8), u=(6.0, 0, 0), v=(0, 6.0, 0)),
+            scenes.entity(L.SHAPE_BOX, L.MAT_LAMBERTIAN, (0, 8, 0), half_extent=(1, 2, 3))]
+    s = finish(ents, lib, "odd")
+    odd = np.argmax(s.instances["px"])
+    quad, box = (np.flatnonzero(s.objects["shapeType"] == k)[0] for k in (L.SHAPE_QUAD, L.SHAPE_BOX))
+    if what == "far":
+        s.instances["px"][odd] = np.inf
+    elif what == "nan place":
+        s.instances["py"][odd] = np.nan
+    elif what == "nan scale":
+        s.instances["scale"][odd] = np.nan
+    elif what == "tiny scale":
+        s.instances["scale"][odd] = 1e-30
+    elif what == "quad":
+        s.objects["x"][quad] = np.inf
+    elif what == "nan quad":
+        s.objects["y"][quad] = np.nan
+    elif what == "box":
+        s.objects["half_y"][box] *= -1
+    else:
+        s.objects["rotation"][box] = 1e7
+    p = rng.uniform(-9, 9, (60_000, 3))
+    rays, dist = rays_to(p + 15.0 * rng.normal(size=p.shape), p, rng)
+    agree(s, rays, (dist * 2.0).astype(np.float32))
+
+
+def test_refit_to_infinity_and_back():
+    """An instance hidden by moving it to infinity, and shown again."""
+    rng = np.random.default_rng(12)
+    lib = scenes.MeshLibrary()
+    ents = [scenes.entity(L.SHAPE_MESH, L.MAT_LAMBERTIAN, (x, 0, 0), mesh=lib.add(*scenes.box_mesh((2, 2, 2))))
+            for x in (-4, 4)]
+    s = finish(ents, lib, "hidden")
+    hidden = s.instances.copy()
+    hidden["px"][1] = np.inf
+    p = rng.uniform(-7, 7, (40_000, 3))
+    rays, dist = rays_to(p + 12.0 * rng.normal(size=p.shape), p, rng)
+    tmax = (dist * 2.0).astype(np.float32)
+    answers = []
+    for mode in (L.PLAIN_WALK_PREPARED, L.PLAIN_WALK_REFERENCE):
+        with scenes_context(s) as ctx:
+            ctx.set_plain_walk(mode)
+            for pose in (hidden, s.instances, hidden):
+                ctx.refit_instances(pose)
+                ctx.prepare_fast()
+                answers.append(ctx.any_hit(rays, tmax))
+            ctx.refit_instances(s.instances)
+            ctx.prepare_fast()
+            answers.append(ctx.any_hit(rays, tmax))
+            assert ctx.plain_walk_used() == (mode == L.PLAIN_WALK_PREPARED)
+    for a, b in zip(answers[:4], answers[4:]):
+        assert 0 < b.mean() < 1 and np.array_equal(a, b)
+
+
 def test_refit_to_quaternions_off_unit_length():
     """The same by a refit, and back."""
     rng = np.random.default_rng(9)
