@@ -631,12 +631,15 @@ int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, in
     // staged pipeline: its lanes take new rays all through the launch, and
     // each such read waiting on the bus cost more than the copies (1.3M
     // bounce rays: 2.25 -> 4.45 ms).
-    if (variant == AE_VARIANT_FAST || variant == AE_VARIANT_QUANT) {
+    bool in_device_memory = false;  // taken by the copies below, but not by the host
+    if (variant == AE_VARIANT_FAST || variant == AE_VARIANT_QUANT || (variant == AE_VARIANT_FAST_WALK && n <= Ctx::kSmallRays)) {
         cudaPointerAttributes ar{}, ah{};
-        const bool mapped = cudaPointerGetAttributes(&ar, rays) == cudaSuccess &&
-                            cudaPointerGetAttributes(&ah, hits) == cudaSuccess && ar.type == cudaMemoryTypeHost &&
+        const bool known = cudaPointerGetAttributes(&ar, rays) == cudaSuccess &&
+                           cudaPointerGetAttributes(&ah, hits) == cudaSuccess;
+        const bool mapped = known && variant != AE_VARIANT_FAST_WALK && ar.type == cudaMemoryTypeHost &&
                             ah.type == cudaMemoryTypeHost && ar.devicePointer && ah.devicePointer &&
                             (reinterpret_cast<uintptr_t>(ar.devicePointer) & 15u) == 0;
+        in_device_memory = ar.type == cudaMemoryTypeDevice || ah.type == cudaMemoryTypeDevice;
         cudaGetLastError();  // pageable memory is not an error here
         if (mapped) {
             if ((rc = closest_hit_dispatch(c, static_cast<const ae_ray *>(ar.devicePointer), n,
@@ -649,7 +652,8 @@ int ae_closest_hit(ae_ctx *ctx, const ae_ray *rays, uint32_t n, ae_hit *hits, in
     // the kernel reads and writes itself, one launch and no device copies (a
     // 1,000-ray call: 43-44 -> 32 us).  Up to 4,096 rays the two host copies stay
     // below what the driver's staged copies cost.
-    if (n <= Ctx::kSmallRays && (variant == AE_VARIANT_FAST || variant == AE_VARIANT_QUANT || variant == AE_VARIANT_FAST_WALK)) {
+    if (n <= Ctx::kSmallRays && !in_device_memory &&
+        (variant == AE_VARIANT_FAST || variant == AE_VARIANT_QUANT || variant == AE_VARIANT_FAST_WALK)) {
         if (!c->small_io && cudaHostAlloc(&c->small_io, Ctx::kSmallRays * (sizeof(ae_ray) + sizeof(ae_hit)),
                                           cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
